@@ -182,6 +182,47 @@ __global__ void node_tables_kernel(int64_t nn, const NodeTables* rec, int32_t* r
     }
 }
 
+// A warp per row: sums over the row's live entries of h(u, v) - h(v, u) for
+// two mixing functions h.  Over a symmetric adjacency the terms cancel; over
+// another one both sums vanish with probability 2^-128.
+__device__ __forceinline__ unsigned long long mix64(unsigned long long x, unsigned long long m) {
+    x ^= x >> 31;
+    x *= m;
+    x ^= x >> 29;
+    x *= 0x9E3779B97F4A7C15ull;
+    return x ^ (x >> 32);
+}
+
+__global__ void symmetry_kernel(DevGraph g, unsigned long long* out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    unsigned long long s0 = 0, s1 = 0;
+    for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < g.n; u += nw) {
+        const int64_t rp = g.row_ptr[u];
+        const int len = g.row_len[u];
+        for (int j = lane; j < len; j += 32) {
+            const unsigned long long v = (unsigned)g.col[rp + j], uu = (unsigned long long)u;
+            const unsigned long long a = (uu << 32) | v, b = (v << 32) | uu;
+            s0 += mix64(a, 0xD6E8FEB86659FD93ull) - mix64(b, 0xD6E8FEB86659FD93ull);
+            s1 += mix64(a, 0xC2B2AE3D27D4EB4Full) - mix64(b, 0xC2B2AE3D27D4EB4Full);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    if (lane == 0 && (s0 | s1)) {
+        atomicAdd(out, s0);
+        atomicAdd(out + 1, s1);
+    }
+}
+
+__global__ void reciprocal_kernel(const double* in, double* out, int64_t n) {
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        out[i] = 1.0 / in[i];
+}
+
 __global__ void apply_entries_kernel(int32_t* col, const int64_t* pos, const int32_t* val, int64_t k) {
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < k; i += (int64_t)gridDim.x * blockDim.x)
         col[pos[i]] = val[i];
@@ -267,6 +308,19 @@ cudaError_t node_tables(int64_t nn, const NodeTables* rec, int32_t* row_len, dou
     if (nn == 0) return cudaSuccess;
     const int blocks = (int)std::min<int64_t>((nn + 255) / 256, 4096);
     node_tables_kernel<<<blocks, 256, 0, st>>>(nn, rec, row_len, degd, degf, nfac, tfac, tfac_f);
+    return cudaGetLastError();
+}
+
+cudaError_t reciprocals(const double* in, double* out, int64_t n, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    reciprocal_kernel<<<(int)std::min<int64_t>((n + 255) / 256, 4096), 256, 0, st>>>(in, out, n);
+    return cudaGetLastError();
+}
+
+cudaError_t symmetry_sums(const DevGraph& g, unsigned long long* out, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(out, 0, 16, st);
+    if (e != cudaSuccess) return e;
+    symmetry_kernel<<<(int)std::min<int64_t>((g.n * 32 + 255) / 256, 4096), 256, 0, st>>>(g, out);
     return cudaGetLastError();
 }
 

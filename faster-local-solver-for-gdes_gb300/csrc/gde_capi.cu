@@ -135,6 +135,15 @@ int katz_compute_prec(gde_ctx* ctx, gde_graph* G, const gde_params* p) {
     return (p->alpha * G->lam_max_est >= kKatzFp64Ratio) ? GDE_FP64 : p->prec;
 }
 
+// When a round pulls (PushArgs::pull_div): its frontier's volume against the
+// graph's.  A pull reads every entry of the graph, about an eighth of the
+// price of pushing along it in a W > 1 tile (1/2 to 1/32 measured: InstantGNN
+// push and update 272 / 85 ms at 1/2, 245 / 70 at 1/8, 245 / 70 at 1/32;
+// global GD and Chebyshev flat).  In a one-column tile each row costs about
+// as much as 16 entries, and 1/6 of that total measured best.
+constexpr int kPullDiv = 8, kPullDivServed = 6;
+constexpr double kPullRowW1 = 16.0;
+
 bool valid_w(int W) { return W == 1 || W == 2 || W == 4 || W == 8 || W == 16 || W == 32; }
 
 // Workspace for `ntiles` tiles of width W over n nodes.
@@ -226,9 +235,125 @@ int alloc_large(gde_ctx* ctx, gde_graph* G, int ntiles, TileWs& tw) {
     return GDE_OK;
 }
 
+// Pull plan of the graph's row capacities: static rows are already in
+// descending order of length; padded rows get an order by capacity (a row's
+// capacity bounds its length through every edit until a repad).
+int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
+    const int64_t n = G->g.n;
+    std::vector<int32_t> ord;
+    std::vector<int2> chunks;
+    auto capacity = [&](int64_t u) { return G->h_indptr[u + 1] - G->h_indptr[u]; };
+    if (!G->relabeled) {
+        int64_t most = 0;
+        for (int64_t u = 0; u < n; u++) most = std::max(most, capacity(u));
+        std::vector<int64_t> at(most + 2, 0);
+        for (int64_t u = 0; u < n; u++) at[most - capacity(u) + 1]++;
+        for (int64_t c = 0; c <= most; c++) at[c + 1] += at[c];
+        ord.resize(n);
+        for (int64_t u = 0; u < n; u++) ord[at[most - capacity(u)]++] = (int32_t)u;
+    }
+    int64_t i = 0;
+    for (; i < n; i++) {
+        const int32_t u = G->relabeled ? (int32_t)i : ord[i];
+        const int64_t c = capacity(u);
+        if (c <= kPullLong) break;
+        for (int64_t b = 0; b < c; b += kPullChunk) chunks.push_back(make_int2(u, (int)b));
+    }
+    G->g.pull_long = (int)i;
+    while (i < n && capacity(G->relabeled ? i : ord[i]) > kPullMid) i++;
+    G->g.pull_mid = (int)i;
+    G->g.npchunk = (int)chunks.size();
+    cudaFree(G->pord);
+    cudaFree(G->pchunk);
+    G->pord = nullptr;
+    G->pchunk = nullptr;
+    G->g.pord = nullptr;
+    G->g.pchunk = nullptr;
+    if (cudaMalloc(&G->pchunk, std::max<size_t>(chunks.size(), 1) * sizeof(int2)) != cudaSuccess ||
+        (!G->relabeled && cudaMalloc(&G->pord, n * sizeof(int32_t)) != cudaSuccess)) {
+        cudaGetLastError();
+        return fail(ctx, GDE_ENOMEM, "device memory exhausted (pull plan)");
+    }
+    CK(cudaMemcpyAsync(G->pchunk, chunks.data(), chunks.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
+    if (G->pord) CK(cudaMemcpyAsync(G->pord, ord.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    G->g.pord = G->pord;
+    G->g.pchunk = G->pchunk;
+    G->pull_plan = true;
+    return GDE_OK;
+}
+
+// Lets this launch's tiles pull in rounds whose frontier holds more than
+// 1/div of the graph's volume.  Needs a symmetric adjacency (checked on the
+// device, once per graph and edit) and room for the frontier bitmaps; without
+// either the launch pushes in every round.
+int enable_pull(gde_ctx* ctx, gde_graph* G, PushArgs& a, int W, int div) {
+    a.pull_div = 0;
+    const double row_cost = W == 1 ? kPullRowW1 * (double)G->g.n : 0.0;
+    if (2.0 * (G->g.vol + row_cost) > div * G->g.vol) return GDE_OK;  // not even half the volume would pull
+    if (!G->pull_plan) {
+        const int rc = build_pull_plan(ctx, G);
+        if (rc == GDE_ENOMEM) { ctx->err.clear(); return GDE_OK; }
+        if (rc != GDE_OK) return rc;
+    }
+    if (G->symmetric < 0) {
+        unsigned long long* sums = (unsigned long long*)wsget(ctx, "sym_sums", 16);
+        if (!sums) return GDE_OK;
+        unsigned long long h[2];
+        CK(symmetry_sums(G->g, sums, ctx->stream));
+        CK(cudaMemcpyAsync(h, sums, 16, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        G->symmetric = (h[0] | h[1]) == 0 ? 1 : 0;
+    }
+    if (!G->symmetric) return GDE_OK;
+    const int64_t words = (G->g.n + 31) / 32 + 1;
+    a.bits = (uint32_t*)wsget(ctx, "bits", (size_t)a.ntiles * 2 * words * 4);
+    if (!a.bits) return GDE_OK;
+    a.bit_words = words;
+    a.g.pord = G->g.pord;
+    a.g.pchunk = G->g.pchunk;
+    a.g.npchunk = G->g.npchunk;
+    a.g.pull_long = G->g.pull_long;
+    a.g.pull_mid = G->g.pull_mid;
+    a.pull_div = div;
+    a.pull_vol = G->g.vol + row_cost;
+    return GDE_OK;
+}
+
+// Reciprocal tables of an FP64 launch of `kind`, filled on the device when
+// they are stale; without memory for them the kernel divides.
+int enable_reciprocals(gde_ctx* ctx, gde_graph* G, PushArgs& a, int kind) {
+    const int64_t n = G->g.n;
+    auto table = [&](double*& t) {
+        if (!t && cudaMalloc(&t, n * 8) != cudaSuccess) {
+            cudaGetLastError();
+            t = nullptr;
+        }
+        return t != nullptr;
+    };
+    if (kind == KIND_IGN) {
+        if (!table(G->rnf) || !table(G->rtf)) return GDE_OK;
+        if (!G->rign_ok) {
+            CK(reciprocals(G->nfac, G->rnf, n, ctx->stream));
+            CK(reciprocals(G->tfac, G->rtf, n, ctx->stream));
+            G->rign_ok = true;
+        }
+        a.g.rnf = G->rnf;
+        a.g.rtf = G->rtf;
+    } else if (kind != KIND_KATZ) {
+        if (!table(G->rdeg)) return GDE_OK;
+        if (!G->rdeg_ok) {
+            CK(reciprocals(G->degd, G->rdeg, n, ctx->stream));
+            G->rdeg_ok = true;
+        }
+        a.g.rdeg = G->rdeg;
+    }
+    return GDE_OK;
+}
+
 // Run the persistent engine until every tile is done (or max_rounds).
 int run_engine(gde_ctx* ctx, PushArgs& a, int prec64, int W, gde_stats* st, double* kernel_ms) {
-    int grid = engine_max_grid(prec64, W, ctx->sms);
+    int grid = engine_max_grid(prec64, W, a.pull_div > 0, ctx->sms);
     if (grid <= 0) return fail(ctx, GDE_ECUDA, "push kernel does not fit on the device");
     if (a.serve && a.queue.sp_blocks > grid / 2) a.queue.sp_blocks = grid / 2;  // at least half the grid stays dense
     const int dense_grid = grid - (a.serve ? a.queue.sp_blocks : 0);
@@ -333,6 +458,7 @@ int upload_ign_tables(gde_ctx* ctx, gde_graph* G, double beta) {
     G->g.npush = G->nfac;
     G->g.tfac = G->tfac;
     G->g.tfac_f = G->tfac_f;
+    G->rign_ok = false;
     G->ign_beta = beta;
     return GDE_OK;
 }
@@ -471,6 +597,12 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
     a.groups = std::max(1, std::min(std::min(p->groups > 0 ? p->groups : g_default, S), kMaxGroups));
     rc = alloc_large(ctx, G, S, tw);
     if (rc != GDE_OK) return rc;
+    // the frontier bitmaps count against an HBM budget too
+    if (budget_bytes <= 0.0 || (double)S * ((double)served_slot_bytes(n, G->g.cap, prec64, any_hk, base, G->g.hub_cut) +
+                                            (double)(n / 4 + 16)) <= budget_bytes) {
+        rc = enable_pull(ctx, G, a, 1, kPullDivServed);
+        if (rc != GDE_OK) return rc;
+    }
     const size_t es = prec64 ? 8 : 4;
     const size_t slab = (size_t)S * n * es;
     // Interleaved FP32 solution slabs: when every query's {x, c} slab fits
@@ -1120,6 +1252,8 @@ int gde_graph_free(gde_graph* G) {
     cudaFree(G->row_ptr); cudaFree(G->col); cudaFree(G->row_len); cudaFree(G->degf); cudaFree(G->degd);
     cudaFree(G->nfac); cudaFree(G->tfac); cudaFree(G->tfac_f); cudaFree(G->perm_d); cudaFree(G->iperm_d);
     cudaFree(G->col_deg); cudaFree(G->rec);
+    cudaFree(G->pord); cudaFree(G->pchunk);
+    cudaFree(G->rdeg); cudaFree(G->rnf); cudaFree(G->rtf);
     cudaFree(G->pw1); cudaFree(G->pwb);
     delete G;
     return GDE_OK;
@@ -1251,6 +1385,9 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         a.small_max = base.small_max; a.med_max = base.med_max; a.chunk = base.chunk;
         a.dense_div = base.dense_div; a.max_rounds = base.max_rounds; a.allow_dense = base.allow_dense;
         rc = alloc_large(ctx, G, nt, tw);
+        if (rc != GDE_OK) return rc;
+        rc = enable_pull(ctx, G, a, W, kPullDiv);
+        if (rc == GDE_OK && prec64) rc = enable_reciprocals(ctx, G, a, kind);
         if (rc != GDE_OK) return rc;
         const size_t slab = (size_t)nt * n * W * es;
         CK(cudaMemsetAsync(a.R, 0, slab, ctx->stream));
@@ -1478,6 +1615,12 @@ static int feature_push_impl(gde_ctx* ctx, gde_graph* G, const gde_params* p, in
         a.allow_dense = cand ? 0 : 1;
         rc = alloc_large(ctx, G, nt, tw);
         if (rc != GDE_OK) return rc;
+        rc = enable_pull(ctx, G, a, W, kPullDiv);
+        if (rc == GDE_OK && prec64) rc = enable_reciprocals(ctx, G, a, kind);
+        if (rc != GDE_OK) return rc;
+        // the scan of every node starts as a pull round
+        const bool pull0 = !cand && a.pull_div > 0;
+        if (pull0) CK(cudaMemsetAsync(a.bits, 0, (size_t)nt * 2 * a.bit_words * 4, ctx->stream));
         const size_t es = prec64 ? 8 : 4;
         a.ld = (int)ld;
         a.tile_stride = W;
@@ -1502,6 +1645,7 @@ static int feature_push_impl(gde_ctx* ctx, gde_graph* G, const gde_params* p, in
             memset(&S, 0, sizeof(S));
             S.stamp = ctx->stamp[t];
             S.dense_next[0] = cand ? 0 : 1;
+            S.pull[0] = pull0 ? 1 : 0;
             S.cand_cnt[0] = cand ? (int)ncand : 0;
             for (int c = 0; c < W; c++) {
                 ColState& C = cs[(size_t)t * W + c];
@@ -1709,6 +1853,7 @@ void gde_internal_graph_relayout(gde_graph* G, int64_t* row_ptr, int32_t* col, i
     G->g.col = col;
     G->g.cap = cap;
     G->h_indptr.assign(h_indptr, h_indptr + G->g.n + 1);
+    G->pull_plan = false;  // the capacities changed
 }
 
 int gde_internal_graph_host(gde_graph* G, const int64_t** indptr, const int64_t** len, int64_t* n) {

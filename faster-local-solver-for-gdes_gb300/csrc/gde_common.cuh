@@ -64,6 +64,10 @@ struct DevGraph {
     const double* npush;      // [n] InstantGNN push divisor d^(1-beta)
     const double* tfac;       // [n] InstantGNN target divisor d^beta
     const float* tfac_f;      // [n] same, FP32
+    // reciprocals 1/degd, 1/npush and 1/tfac for FP64 tiles (nullptr: divide)
+    const double* rdeg;       // [n]
+    const double* rnf;        // [n]
+    const double* rtf;        // [n]
     double vol;               // sum of degrees (m)
     int degf_exact;           // 1 when every degree is an integer < 2^24 (degf == degd exactly)
     const int32_t* perm;      // caller id -> internal id (nullptr: identity)
@@ -75,7 +79,21 @@ struct DevGraph {
     int idx_bits;
     uint32_t deg_esc;
     const NodeRec* rec;       // [n] (nullptr: not built)
+    // Pull plan (pull rounds, symmetric graphs only; PushArgs::pull_div > 0):
+    // node ids by descending row capacity, the first pull_long of them cut
+    // into the chunks of pchunk, the next ones up to pull_mid shared by
+    // several lane groups per row, the rest one lane group per row.
+    const int32_t* pord;      // [n] (nullptr: the ids themselves are in that order)
+    const int2* pchunk;       // [npchunk] {node, first edge within the row}
+    int npchunk;
+    int pull_long, pull_mid;
 };
+
+// Rows longer than kPullLong are pulled by whole warps, kPullChunk edges at a
+// time; rows longer than kPullMid by a few lane groups each.
+constexpr int kPullLong = 64;
+constexpr int kPullMid = 16;
+constexpr int kPullChunk = 256;
 
 // ---------------------------------------------------------------------------
 // Per-tile state
@@ -158,11 +176,13 @@ struct OnlineSlot {           // the query a slot holds (copied out of the ring 
     OnlineReq mail;           // written by the ring reader, read by the slot's own group at admission
 };
 
-struct TileState {            // device-updated
+// (each tile's counters on lines of their own: slots of different groups update theirs at the same time)
+struct alignas(128) TileState {  // device-updated
     int cand_cnt[3];          // candidate list sizes (by level mod 3)
     int front_cnt[2];         // frontier sizes (by parity)
     int small_cnt[2], med_cnt[2], large_cnt[2];
     int dense_next[2];        // 1: the PREP of that parity scans all nodes
+    int pull[2];              // 1: the round of that parity pulls (push values by node, rows gather them)
     int t0;                   // launch iteration at which the tile's level 0 ran
     int done;                 // SlotState
     int stamp;                // touch-stamp base (marks start at -1; stamps only grow)
@@ -240,7 +260,7 @@ struct ServeQueue {
     double alpha0;                //                     and alpha
 };
 
-struct ColState {             // one per column slot
+struct ColState {            // one per column slot
     double theta;             // threshold scale (eps*alpha, eps, e^tau*eps, eps ...)
     double oper;              // operation count (sum of degrees of pushed nodes)
     int64_t fsum;             // sum over rounds of frontier size
@@ -343,6 +363,13 @@ struct PushArgs {
     // about 2 theta d of l1.  nullptr: every residual entry is in R.
     double* RH;
     int rh_cut;
+    // Pull rounds: a round whose predecessor's frontier held more than
+    // 1/pull_div of the graph's volume lets every row gather its neighbours'
+    // push values instead of pushing them with atomics (0: never).
+    int pull_div;
+    double pull_vol;           // the graph's volume, plus the cost of a pull's rows
+    uint32_t* bits;            // [ntiles][2][bit_words] frontier bitmap by round parity
+    int64_t bit_words;
 };
 
 constexpr int kMaxGroups = 512;  // at most one per slot (kMaxLaunchTiles)

@@ -7,7 +7,8 @@
 namespace gde {
 
 // Persistent push engine (push_engine.cu).
-int engine_max_grid(int prec64, int W, int sms);
+// (pull: the launch's a.pull_div > 0; max_grid and launch must agree on it.)
+int engine_max_grid(int prec64, int W, bool pull, int sms);
 cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st);
 
 // Column initialisation and result extraction (aux_kernels.cu).
@@ -71,6 +72,13 @@ struct NodeTables {
 // Write the tables of nn touched nodes (nfac null: degrees only).
 cudaError_t node_tables(int64_t nn, const NodeTables* rec, int32_t* row_len, double* degd, float* degf, double* nfac,
                         double* tfac, float* tfac_f, cudaStream_t st);
+
+// Is every live entry v of a row u matched by an entry u of row v (aux_kernels.cu)?  Adds two
+// hashes of every (u, v) minus those of (v, u) into out[0], out[1] (zeroed here): both end at zero.
+cudaError_t symmetry_sums(const DevGraph& g, unsigned long long* out, cudaStream_t st);
+
+// out[i] = 1 / in[i] (aux_kernels.cu).
+cudaError_t reciprocals(const double* in, double* out, int64_t n, cudaStream_t st);
 
 // Graph helpers (aux_kernels.cu).
 cudaError_t graph_apply_entries(int32_t* col, const int64_t* pos, const int32_t* val, int64_t k, cudaStream_t st);

@@ -82,5 +82,16 @@ struct gde_graph {
     double lam_max_est = NAN;    // adjacency spectral radius from gde_katz_spectral_bounds (NaN: none)
     uint32_t* col_deg = nullptr;
     gde::NodeRec* rec = nullptr;
+    // pull plan of the row capacities (DevGraph::pord, pchunk), built on first
+    // use, and whether the live rows are symmetric (-1: not checked since the last edit)
+    int32_t* pord = nullptr;
+    int2* pchunk = nullptr;
+    bool pull_plan = false;
+    int symmetric = -1;
+    // reciprocals of degd (rdeg) and of nfac, tfac (rnf, rtf); rebuilt on use after an edit
+    double* rdeg = nullptr;
+    double* rnf = nullptr;
+    double* rtf = nullptr;
+    bool rdeg_ok = false, rign_ok = false;
     int32_t node_in(int64_t u) const { return relabeled ? h_perm[u] : (int32_t)u; }
 };

@@ -1087,6 +1087,8 @@ static int feature_update_impl(gde_ctx* ctx, gde_graph* G, int32_t* h_indices, i
         G->ncolors = 0;  // the edges change: the SOR colouring is rebuilt on its next use,
         G->dmax = -1.0;  // the degree bound recomputed and the spectral estimate dropped
         G->lam_max_est = NAN;
+        G->symmetric = -1;       // (a self-loop may leave a row that no longer matches its neighbours')
+        G->rdeg_ok = G->rign_ok = false;
     }
     // ---- the edit, the repair keys and the push, all on the device ----
     if (k >= ((int64_t)1 << 30)) return gde_internal_fail(ctx, GDE_EINVAL, "edge batch too large (2^30 edges at most)");

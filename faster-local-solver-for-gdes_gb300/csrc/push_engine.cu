@@ -14,7 +14,9 @@
 //           chunks, medium rows one warp per row, short rows one lane group
 //           per row; W columns move per edge with one vector atomic; touched
 //           nodes are appended (deduplicated by a round stamp) as the next
-//           round's candidates unless the next round scans densely.
+//           round's candidates unless the next round scans densely.  A round
+//           with a large frontier pulls instead: PREP writes push rows by
+//           node, and every row gathers its neighbours' (see PULL).
 //
 // Semantics follow the reference's synchronous round of ppr_gd local
 // (ppr_solver.py:246-288): the frontier of round t+1 is exactly the set of
@@ -86,6 +88,30 @@ __device__ __forceinline__ bool ge_band(float r, float t32, F thr64) {
     if (r >= t32 * (1.f + 0x1p-20f)) return true;
     if (r < t32 * (1.f - 0x1p-20f)) return false;
     return (double)r >= thr64();
+}
+
+// FP64 comparisons |r| >= thr and r >= thr of a threshold thr >= 0, on the
+// bit patterns (the order of non-negative doubles is that of their bits; a
+// NaN compares false, as in FP64).  GB300 runs one FP64 instruction per SM
+// and warp in 16 cycles, an integer one in one: the FP64 tiles' tests, like
+// their divisions (DevGraph::rdeg), stay off that pipe where they can.
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+__device__ __forceinline__ bool ge_bits(long long r, long long thr) { return r >= thr && r <= kInfBits; }
+__device__ __forceinline__ bool ge_abs64(double r, double thr) {
+    return ge_bits(__double_as_longlong(r) & 0x7fffffffffffffffll, __double_as_longlong(thr));
+}
+__device__ __forceinline__ bool crossed64(double old, double s, double thr) {
+    const long long t = __double_as_longlong(thr);
+    return __double_as_longlong(old) < t && ge_bits(__double_as_longlong(s), t);
+}
+// |r| >= thr64() where approx is within 2^-48 (relative) of thr64(): decided
+// by the approximation outside a band of 64 ulps.
+template <typename F>
+__device__ __forceinline__ bool ge_band64(double r, double approx, F thr64) {
+    const long long b = __double_as_longlong(r) & 0x7fffffffffffffffll, t = __double_as_longlong(approx);
+    if (b >= t + 64) return b <= kInfBits;
+    if (b < t - 64) return false;
+    return fabs(r) >= thr64();
 }
 
 // ---------------------------------------------------------------------------
@@ -191,7 +217,7 @@ __device__ __forceinline__ double* rh_ptr(const PushArgs& a, int t) {
 struct TileSh {
     TileParams tp;
     int cand_cnt, front_cnt, small_cnt, med_cnt, large_cnt;
-    int dense, parity, level, stamp, m3;
+    int dense, pull, parity, level, stamp, m3;
     double psi;             // HK: psi[level]
     double coef1, coef2;    // Chebyshev coefficients of this round
     int final_level;        // HK: pushes of this level go into X
@@ -240,6 +266,7 @@ __device__ void load_tile(const PushArgs& a, int t, int it, TileSh& sh) {
         sh.med_cnt = ts.med_cnt[par];
         sh.large_cnt = ts.large_cnt[par];
         sh.dense = ts.dense_next[par];
+        sh.pull = ts.pull[par];
         sh.stamp = ts.stamp + sh.level + 1;
         int m = sh.tp.method;
         sh.psi = 1.0;
@@ -407,15 +434,21 @@ struct RoundSh {
     int any_idle;                               // served solves: some slot awaits a query
     int tiles[kMaxLaunchTiles];                 // live tile ids (ascending)
     unsigned char idle[kMaxLaunchTiles];        // 1: slot idle at the round start; 2: draining (online)
-    short drain[kMaxLaunchTiles];               // online slots to clear this round (SLOT_DRAIN)
+    union {
+        short drain[kMaxLaunchTiles];           // online slots to clear this round (SLOT_DRAIN)
+        short pull[kMaxLaunchTiles];            // other launches: live tiles whose round pulls
+    };
     int ndrain;
+    int npull;
     long long off[4][kMaxLaunchTiles + 1];      // exclusive prefix sums of the current phase's spaces
     int level[kMaxLaunchTiles];                 // per live tile: rounds since its start
     unsigned char flags[kMaxLaunchTiles];       // per live tile scatter flags (SF_*)
     long long scan_tmp[kWarps];
 };
 
-enum : unsigned char { SF_FINAL = 1, SF_TRACK = 2, SF_NOPUSH = 4, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32 };
+enum : unsigned char {
+    SF_FINAL = 1, SF_TRACK = 2, SF_NOPUSH = 4, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32, SF_PULL = 64
+};
 
 // Local GD for PPR and Katz only ever adds non-negative values to
 // non-negative residuals, so a node enters the next frontier exactly when one
@@ -433,6 +466,17 @@ __device__ __forceinline__ bool dense_next_round(const PushArgs& a, const TilePa
     if (method_is_global(tp.method)) return true;
     if (tile_crosses(tp) || !a.allow_dense) return false;
     return ts.union_vol[par] * (double)a.dense_div > (double)a.g.n;
+}
+
+// Does tile t's next round pull?  Frontier volumes change smoothly from round
+// to round, so this round's decides (identical in every block).
+__device__ __forceinline__ bool pull_next_round(const PushArgs& a, const TileState& ts, int par) {
+    return a.pull_div > 0 && ts.union_vol[par] * (double)a.pull_div > a.pull_vol;
+}
+
+// Frontier bitmap of tile t's rounds of parity par (pull rounds).
+__device__ __forceinline__ uint32_t* tile_bits(const PushArgs& a, int t, int par) {
+    return a.bits + ((int64_t)t * 2 + par) * a.bit_words;
 }
 
 // Exclusive prefix over vals[0..m) (m <= 512) written to out[0..m]; block-wide.
@@ -582,7 +626,7 @@ __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, 
 #endif
 constexpr int kPrepILP = GDE_PREP_ILP;
 
-template <typename T>
+template <typename T, bool PULL>
 __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
                               double& my_oper, int& my_nodes, double& my_vol, int& my_cnt) {
     const DevGraph& g = a.g;
@@ -602,6 +646,7 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
     const int64_t ld = a.ld;
     double* RH = (sizeof(T) == 4) ? rh_ptr(a, t) : nullptr;  // hub prefix in FP64
     const int rh_cut = a.rh_cut;
+    uint32_t* bits = (PULL && sh.pull) ? tile_bits(a, t, par) : nullptr;
     long long ideg = 0;  // sum of (integer) degrees of the pushed nodes
     for (long long base = beg + (long long)warp * 32 * kPrepILP; base < end;
          base += (long long)kWarps * 32 * kPrepILP) {
@@ -685,15 +730,227 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
                     my_cnt += 1;
                 }
             }
-            emit_node_w1<T>(a, t, par, act, len[q], rp[q], push);
+            if (PULL && bits) {
+                if (act) {  // a pull round: the push value by node, and the node's frontier bit
+                    reinterpret_cast<T*>(a.P)[(int64_t)t * n + u[q]] = push;
+                    atomicOr(bits + (u[q] >> 5), 1u << (u[q] & 31));
+                }
+            } else {
+                emit_node_w1<T>(a, t, par, act, len[q], rp[q], push);
+            }
         }
     }
     my_oper += (double)ideg;
     my_vol += (double)ideg;
 }
 
+// PREP of a W > 1 tile whose round pulls (every method but Chebyshev and the
+// relaxed heat kernel): most visited nodes push, so every load of a node --
+// residual, solution, Kahan term, degree, divisor -- is issued before any is
+// used, for kPullPrep nodes per lane group at a time, and the push row goes to
+// P by node id with no work items.  The arithmetic is prep_nodes'.  PREP of
+// the 128-column FP64 push went from 90 to 64 ms with it; it is bound by the
+// latency of the node loads and by FP64 issue.
+constexpr int kPullPrep = 2;
+
 template <typename T, int W>
-__device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& ps, long long beg, long long end) {
+struct PrepSums {
+    static constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    double oper[VEC];
+    long long deg[VEC];  // the same sum while degrees are exact integers
+    int nodes[VEC];
+    double vol;
+    long long ivol;
+    int cnt;
+};
+
+template <typename T, int W>
+__device__ void prep_pull(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
+                          PrepSums<T, W>& sum) {
+    constexpr int VEC = PrepSums<T, W>::VEC;
+    constexpr int L = W / VEC;
+    constexpr int GPW = 32 / L;
+    constexpr int Q = kPullPrep;
+    const DevGraph& g = a.g;
+    const int64_t n = g.n;
+    const int par = sh.parity, kind = sh.tp.kind;
+    const bool global = method_is_global(sh.tp.method), hk = kind == KIND_HK, ign = kind == KIND_IGN;
+    const bool lone = ign || kind == KIND_UPPR;  // nodes without neighbours absorb their residual
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane_g = lane % L, grp_w = lane / L;
+    const int c0 = lane_g * VEC;
+    const int32_t* cand = a.cand + ((int64_t)t * 2 + par) * n;
+    uint32_t* bits = tile_bits(a, t, par);
+    T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W;
+    T* R = slab_ptr<T>((hk && (sh.level & 1)) ? a.R2 : a.R, a, t);
+    T* X = xslab_ptr<T>(a.X, a, t);
+    float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) : nullptr;
+    const int64_t xld = x_ld(a);
+    const double alpha = sh.tp.alpha;
+    const double* rdiv = (sizeof(T) == 8 && kind != KIND_KATZ) ? (ign ? g.rnf : g.rdeg) : nullptr;
+    const bool f32 = (sizeof(T) == 4) && g.degf_exact;
+    const bool dint = g.degf_exact != 0;
+    const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
+    const double hkc = hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.)) : 0.0;
+    const float hkc_f = (float)hkc, alpha_f = (float)alpha, omalpha_f = (float)(1. - alpha);
+    const double x_gain = ign ? sh.tp.x_gain : 1.0;
+    const float xgain_f = (float)x_gain;
+    double theta[VEC], scale0 = 0.0;
+    float thr_f[VEC];
+    bool live[VEC], same = true;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+        live[k] = sh.col_live[c0 + k] != 0;
+        theta[k] = sh.col_theta[c0 + k];
+        same &= theta[k] == theta[0];
+        thr_f[k] = (float)(hk ? theta[k] / hk_div : theta[k]);
+    }
+    scale0 = hk ? theta[0] / hk_div : theta[0];
+    for (long long base = beg + (long long)warp * GPW * Q; base < end; base += (long long)kWarps * GPW * Q) {
+        int u[Q], len[Q];
+        float df[Q];
+        double nf[Q], rd[Q], dd[Q];
+        Vec<T, VEC> r[Q], x[Q];
+        Vec<float, VEC> xc[Q];
+        bool valid[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const long long i = base + q * GPW + grp_w;
+            valid[q] = i < end;
+            u[q] = valid[q] ? (sh.dense ? (int)i : cand[i]) : 0;
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            if (!valid[q]) continue;
+            vload<T, VEC>(R + (int64_t)u[q] * a.ld + c0, r[q]);
+            vload<T, VEC>(X + (int64_t)u[q] * xld + c0, x[q]);
+            if (XC) vload<float, VEC>(XC + (int64_t)u[q] * xld + c0, xc[q]);
+            df[q] = g.degf[u[q]];
+            dd[q] = dint ? 0.0 : g.degd[u[q]];
+            nf[q] = ign ? g.nfac[u[q]] : 0.0;
+            rd[q] = rdiv ? rdiv[u[q]] : 0.0;
+            len[q] = lone ? g.row_len[u[q]] : 2;
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            bool any = false, absorb = false;
+            Vec<T, VEC> push;
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
+            const int di = valid[q] ? (int)df[q] : 0;
+            double du = 0.0;
+            if (valid[q]) {
+                du = dint ? (double)df[q] : dd[q];
+                const double thr_base = ign ? nf[q] : du;
+                const float base_f = ign ? (float)thr_base : df[q];
+                const double thr64 = f32 ? 0.0 : scale0 * thr_base;
+                bool act[VEC];
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) {
+                    act[k] = false;
+                    if (!live[k]) continue;
+                    auto hk_thr = [&] { return ((theta[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi; };
+                    if (global) act[k] = r[q].v[k] != T(0);
+                    else if (f32)
+                        act[k] = ge_band(fabsf((float)r[q].v[k]), thr_f[k] * base_f,
+                                         [&] { return hk ? hk_thr() : theta[k] * thr_base; });
+                    else if (hk)
+                        act[k] = ge_band64((double)r[q].v[k], same ? thr64 : (theta[k] / hk_div) * thr_base, hk_thr);
+                    else act[k] = ge_abs64((double)r[q].v[k], same ? thr64 : theta[k] * thr_base);
+                    any |= act[k];
+                }
+                if (any && lone) {
+                    absorb = len[q] == 0 || (len[q] == 1 && g.col[g.row_ptr[u[q]]] == u[q]);
+                    if (absorb) {
+                        // (a zero residual has nothing to absorb)
+                        any = false;
+#pragma unroll
+                        for (int k = 0; k < VEC; ++k) {
+                            act[k] = act[k] && r[q].v[k] != T(0);
+                            any |= act[k];
+                        }
+                    }
+                }
+                if (any) {
+                    const float div_f = (f32 && ign) ? (float)g.npush[u[q]] : df[q];
+                    const double gain = (hk ? hkc : 1. - alpha) * rd[q];  // the push per unit of residual
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) {
+                        if (!act[k]) continue;
+                        const T rk = r[q].v[k];
+                        T pv, xadd;
+                        if (f32) {
+                            const float rf = (float)rk;
+                            pv = (T)(kind == KIND_KATZ ? alpha_f * rf
+                                     : (hk ? (sh.final_level ? rf : hkc_f * rf) : omalpha_f * rf) / div_f);
+                            xadd = (ign && !absorb) ? (T)(xgain_f * rf) : rk;
+                        } else {
+                            const double rv = (double)rk;
+                            if (rdiv) pv = (T)(gain * rv);
+                            else if (kind == KIND_KATZ) pv = (T)(alpha * rv);
+                            else pv = (T)((hk ? (sh.final_level ? rv : hkc * rv) : (1. - alpha) * rv) /
+                                          (ign ? g.npush[u[q]] : du));
+                            xadd = (ign && !absorb) ? (T)(x_gain * rv) : rk;
+                        }
+                        push.v[k] = absorb ? T(0) : pv;
+                        r[q].v[k] = T(0);
+                        sum.nodes[k] += 1;
+                        if (absorb) {
+                            // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
+                            x[q].v[k] = xadd;
+                            if (XC) xc[q].v[k] = 0.f;
+                            continue;
+                        }
+                        if (dint) sum.deg[k] += di;
+                        else sum.oper[k] += du;
+                        if (XC) {
+                            // Kahan-compensated FP32 accumulation of the solution
+                            const float y = (float)xadd - xc[q].v[k];
+                            const float s = (float)x[q].v[k] + y;
+                            xc[q].v[k] = (s - (float)x[q].v[k]) - y;
+                            x[q].v[k] = (T)s;
+                        } else {
+                            x[q].v[k] = x[q].v[k] + xadd;
+                        }
+                    }
+                    vstore<T, VEC>(R + (int64_t)u[q] * a.ld + c0, r[q]);
+                    vstore<T, VEC>(X + (int64_t)u[q] * xld + c0, x[q]);
+                    if (XC) vstore<float, VEC>(XC + (int64_t)u[q] * xld + c0, xc[q]);
+                }
+            }
+            // the node pushes when any of its columns does (OR over the lane group)
+            const unsigned bal = __ballot_sync(kFull, any);
+            if (bal == 0) continue;  // warp-uniform
+            const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
+            const bool node_in = valid[q] && (bal & gmask) != 0 && !absorb;
+            if (node_in) vstore<T, VEC>(Pw + (int64_t)u[q] * W + c0, push);
+            const bool in = lane_g == 0 && node_in;
+            if (in) {
+                if (dint) sum.ivol += di;
+                else sum.vol += du;
+                sum.cnt += 1;
+            }
+            if (sh.dense) {
+                // consecutive nodes: their bits lie in two words at most
+                const int w0 = (int)((base + q * GPW) >> 5);
+                const uint32_t bit = in ? 1u << (u[q] & 31) : 0u;
+                const uint32_t b0 = __reduce_or_sync(kFull, (u[q] >> 5) == w0 ? bit : 0u);
+                const uint32_t b1 = __reduce_or_sync(kFull, (u[q] >> 5) == w0 ? 0u : bit);
+                if (lane == 0 && b0) atomicOr(bits + w0, b0);
+                if (lane == 0 && b1) atomicOr(bits + w0 + 1, b1);
+            } else if (in) {
+                atomicOr(bits + (u[q] >> 5), 1u << (u[q] & 31));
+            }
+        }
+    }
+}
+
+// PREP of any tile and round: tests each candidate per column, then compacts
+// the frontier.  (Out of line: its registers would cost the one-column
+// crossing tiles, which never come here.)
+template <typename T, int W, bool PULL>
+__device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
+                                        PrepSums<T, W>& total) {
     constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
     constexpr int L = W / VEC;          // lanes per node
     constexpr int GPW = 32 / L;         // nodes per warp iteration
@@ -711,6 +968,7 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
     const int32_t* cand = a.cand + ((int64_t)t * 2 + par) * n;
     int32_t* next = a.cand + ((int64_t)t * 2 + (par ^ 1)) * n;
     int32_t* mark = a.mark + (int64_t)t * n;
+    uint32_t* bits = (PULL && sh.pull) ? tile_bits(a, t, par) : nullptr;
     T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;       // short rows grow up from 0,
     PushItem* bmed_end = bsmall + (n - 1);               // medium rows down from n-1
@@ -724,12 +982,7 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
     const double alpha = sh.tp.alpha;
     int* next_cnt = &ts.cand_cnt[(sh.level + 1) % 3];
 
-    if (threadIdx.x < W) { ps.col_oper[threadIdx.x] = 0.0; ps.col_nodes[threadIdx.x] = 0; }
-    if (threadIdx.x == 0) { ps.vol = 0.0; ps.nodes = 0; }
-    __syncthreads();
-
-    double my_oper[VEC];
-    int my_nodes[VEC];
+    PrepSums<T, W> sum = total;
     double thr_scale[VEC];
     bool live[VEC];
     // FP32 tiles on integer degrees decide and push in FP32, as the W = 1
@@ -740,275 +993,340 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
     const bool f32 = (sizeof(T) == 4) && g.degf_exact && !cheby;
     float thr_f[VEC];
     const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
+    // FP64 tiles: one threshold per node when the columns share theta, and
+    // divisions by the node's divisor as products with its reciprocal
+    const double* rdiv = (sizeof(T) == 8 && kind != KIND_KATZ) ? (kind == KIND_IGN ? g.rnf : g.rdeg) : nullptr;
+    const bool dint = g.degf_exact != 0;
+    bool same = true;
 #pragma unroll
     for (int k = 0; k < VEC; ++k) {
-        my_oper[k] = 0.0;
-        my_nodes[k] = 0;
+        same &= sh.col_theta[c0 + k] == sh.col_theta[c0];
         live[k] = sh.col_live[c0 + k] != 0;
         thr_scale[k] = sh.col_theta[c0 + k];
         thr_f[k] = (float)(hk ? thr_scale[k] / hk_div : thr_scale[k]);
     }
     const float alpha_f = (float)alpha, omalpha_f = (float)(1. - alpha), xgain_f = (float)sh.tp.x_gain;
     const float hkc_f = hk ? (float)(sh.tp.tau / ((double)sh.level + 1.)) : 0.f;
-    double my_vol = 0.0;
-    int my_cnt = 0;
-
-    // A W = 1 crossing tile visits exactly the nodes that crossed their
-    // threshold last round: every candidate is active, so all its loads are
-    // issued at once (prep_w1_cross).
-    bool fast = false;
-    if constexpr (W == 1) fast = tile_crosses(sh.tp) && !sh.dense && live[0];
-    if (fast) {
-        if constexpr (W == 1) prep_w1_cross<T>(a, t, sh, beg, end, my_oper[0], my_nodes[0], my_vol, my_cnt);
-    } else {
-        for (long long base = beg + (long long)warp * GPW; base < end; base += (long long)kWarps * GPW) {
-            const long long i = base + grp_w;
-            const bool valid = i < end;
-            int u = 0;
-            bool act[VEC];
-            Vec<T, VEC> push;
-    #pragma unroll
-            for (int k = 0; k < VEC; ++k) { act[k] = false; push.v[k] = T(0); }
-            double du = 1.0;
-            bool absorb = false;
-            bool any = false;
-            Vec<T, VEC> r;
-            float df = 1.f;
-            if (valid) {
-                u = sh.dense ? (int)i : cand[i];
-                const int64_t off = (int64_t)u * a.ld + c0;
-                const int64_t xoff = (int64_t)u * xld + c0;
-                vload<T, VEC>(R + off, r);
-                // fast test first: most scanned nodes are below every threshold
-                df = g.degf[u];
-                du = g.degf_exact ? (double)df : g.degd[u];
-                const double thr_base = (kind == KIND_IGN) ? g.nfac[u] : du;
-                const float base_f = (kind == KIND_IGN) ? (float)thr_base : df;
-    #pragma unroll
+    const double hk_scale0 = hk ? thr_scale[0] / hk_div : 0.0;
+    const double hkc = hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.)) : 0.0;
+    for (long long base = beg + (long long)warp * GPW; base < end; base += (long long)kWarps * GPW) {
+        const long long i = base + grp_w;
+        const bool valid = i < end;
+        int u = 0;
+        bool act[VEC];
+        Vec<T, VEC> push;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) { act[k] = false; push.v[k] = T(0); }
+        double du = 1.0;
+        bool absorb = false;
+        bool any = false;
+        Vec<T, VEC> r;
+        float df = 1.f;
+        int di = 1;
+        if (valid) {
+            u = sh.dense ? (int)i : cand[i];
+            const int64_t off = (int64_t)u * a.ld + c0;
+            const int64_t xoff = (int64_t)u * xld + c0;
+            vload<T, VEC>(R + off, r);
+            // fast test first: most scanned nodes are below every threshold
+            df = g.degf[u];
+            du = g.degf_exact ? (double)df : g.degd[u];
+            di = (int)df;
+            const double thr_base = (kind == KIND_IGN) ? g.nfac[u] : du;
+            const float base_f = (kind == KIND_IGN) ? (float)thr_base : df;
+            double thr64 = 0.0;
+            if (!f32 && !global) thr64 = (hk ? hk_scale0 : thr_scale[0]) * thr_base;
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) {
+                if (!live[k]) continue;
+                bool a_k;
+                if (global) {
+                    a_k = (r.v[k] != T(0));
+                } else if (f32) {
+                    a_k = ge_band(fabsf((float)r.v[k]), thr_f[k] * base_f, [&] {
+                        return hk ? ((thr_scale[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi
+                                  : thr_scale[k] * thr_base;
+                    });
+                } else {
+                    const double rv = (double)r.v[k];
+                    if (hk)
+                        a_k = ge_band64(rv, same ? thr64 : (thr_scale[k] / hk_div) * thr_base, [&] {
+                            return ((thr_scale[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi;
+                        });
+                    else
+                        a_k = ge_abs64(rv, same ? thr64 : thr_scale[k] * thr_base);
+                }
+                act[k] = a_k;
+                any |= a_k;
+            }
+            if (cheby && global) {
+                // global Chebyshev updates every node whose three-term step is non-zero
+                Vec<T, VEC> dxv;
+                vload<T, VEC>(DX + off, dxv);
+#pragma unroll
                 for (int k = 0; k < VEC; ++k) {
                     if (!live[k]) continue;
-                    bool a_k;
-                    if (global) {
-                        a_k = (r.v[k] != T(0));
-                    } else if (f32) {
-                        a_k = ge_band(fabsf((float)r.v[k]), thr_f[k] * base_f, [&] {
-                            return hk ? ((thr_scale[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi
-                                      : thr_scale[k] * thr_base;
-                        });
+                    act[k] = (r.v[k] != T(0)) || (dxv.v[k] != T(0));
+                    any |= act[k];
+                }
+            }
+            if (any) {
+                absorb = ign && is_absorbing(g, u);
+                const float npush_f = (f32 && kind == KIND_IGN) ? (float)g.npush[u] : 1.f;
+                const double rd = rdiv ? rdiv[u] : 0.0;
+                const double gain = hk ? hkc * rd : (1. - alpha) * rd;  // the push per unit of residual
+                Vec<T, VEC> dxv;
+                if (cheby) vload<T, VEC>(DX + off, dxv);
+                Vec<T, VEC> xadd;
+                bool wrote = false;
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) {
+                    xadd.v[k] = T(0);
+                    if (!act[k]) continue;
+                    const double rv = (double)r.v[k];
+                    if (cheby) {
+                        // ppr_solver.py:642-646 / katz_solver.py:407-411
+                        double tmp;
+                        if (kind == KIND_KATZ) tmp = sh.coef1 * rv - sh.coef2 * (double)dxv.v[k];
+                        else tmp = sh.coef1 * rv + (sh.coef1 - 1.) * (double)dxv.v[k];
+                        if (global && tmp == 0.0) { act[k] = false; continue; }
+                        T tmpT = (T)tmp;
+                        xadd.v[k] = tmpT;
+                        dxv.v[k] = tmpT;
+                        r.v[k] = (T)(rv - (double)tmpT);  // rt[u] += -delta_xt[u] (:657)
+                        double pv;
+                        if (kind == KIND_KATZ) pv = alpha * (double)tmpT;
+                        else pv = rdiv ? gain * (double)tmpT : ((1. - alpha) * (double)tmpT) / du;
+                        push.v[k] = (T)pv;
                     } else {
-                        const double rv = (double)r.v[k];
-                        double thr;
-                        if (hk) thr = ((thr_scale[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi;
-                        else thr = thr_scale[k] * thr_base;
-                        a_k = fabs(rv) >= thr;
-                    }
-                    act[k] = a_k;
-                    any |= a_k;
-                }
-                if (cheby && global) {
-                    // global Chebyshev updates every node whose three-term step is non-zero
-                    Vec<T, VEC> dxv;
-                    vload<T, VEC>(DX + off, dxv);
-    #pragma unroll
-                    for (int k = 0; k < VEC; ++k) {
-                        if (!live[k]) continue;
-                        act[k] = ((double)r.v[k] != 0.0) || ((double)dxv.v[k] != 0.0);
-                        any |= act[k];
-                    }
-                }
-                if (any) {
-                    absorb = ign && is_absorbing(g, u);
-                    const float npush_f = (f32 && kind == KIND_IGN) ? (float)g.npush[u] : 1.f;
-                    Vec<T, VEC> dxv;
-                    if (cheby) vload<T, VEC>(DX + off, dxv);
-                    Vec<T, VEC> xadd;
-                    bool wrote = false;
-    #pragma unroll
-                    for (int k = 0; k < VEC; ++k) {
-                        xadd.v[k] = T(0);
-                        if (!act[k]) continue;
-                        const double rv = (double)r.v[k];
-                        if (cheby) {
-                            // ppr_solver.py:642-646 / katz_solver.py:407-411
-                            double tmp;
-                            if (kind == KIND_KATZ) tmp = sh.coef1 * rv - sh.coef2 * (double)dxv.v[k];
-                            else tmp = sh.coef1 * rv + (sh.coef1 - 1.) * (double)dxv.v[k];
-                            if (global && tmp == 0.0) { act[k] = false; continue; }
-                            T tmpT = (T)tmp;
-                            xadd.v[k] = tmpT;
-                            dxv.v[k] = tmpT;
-                            r.v[k] = (T)(rv - (double)tmpT);  // rt[u] += -delta_xt[u] (:657)
-                            double pv = (kind == KIND_KATZ) ? alpha * (double)tmpT : ((1. - alpha) * (double)tmpT) / du;
-                            push.v[k] = (T)pv;
-                        } else {
-                            // An absorbing node (threshold 0) is visited once by the
-                            // reference's initial scan and never re-enqueued; with a
-                            // zero residual it has nothing to absorb.
-                            if (absorb && r.v[k] == T(0)) { act[k] = false; continue; }
-                            if (f32) {
-                                const float rf = (float)r.v[k];
-                                float pvf;
-                                if (kind == KIND_PPR || kind == KIND_UPPR) pvf = (omalpha_f * rf) / df;
-                                else if (kind == KIND_KATZ) pvf = alpha_f * rf;
-                                else if (kind == KIND_HK) pvf = sh.final_level ? rf / df : (hkc_f * rf) / df;
-                                else pvf = (omalpha_f * rf) / npush_f;
-                                push.v[k] = absorb ? T(0) : (T)pvf;
-                                xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(xgain_f * rf) : r.v[k];
-                                r.v[k] = T(0);
-                                wrote = true;
-                                my_nodes[k] += 1;
-                                if (!absorb) my_oper[k] += du;
-                                continue;
-                            }
-                            double pv;
-                            if (kind == KIND_PPR || kind == KIND_UPPR) pv = ((1. - alpha) * rv) / du;
-                            else if (kind == KIND_KATZ) pv = alpha * rv;
-                            else if (kind == KIND_HK) {
-                                if (sh.final_level) pv = rv / du;  // hk_solver.py:254-256
-                                else pv = ((sh.tp.tau / ((double)sh.level + 1.)) * rv) / du;
-                            } else {
-                                pv = ((1. - alpha) * rv) / g.npush[u];  // InstantGNN.py:28
-                            }
-                            if (absorb) pv = 0.0;
-                            push.v[k] = (T)pv;
-                            xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(sh.tp.x_gain * rv) : r.v[k];
+                        // An absorbing node (threshold 0) is visited once by the
+                        // reference's initial scan and never re-enqueued; with a
+                        // zero residual it has nothing to absorb.
+                        if (absorb && r.v[k] == T(0)) { act[k] = false; continue; }
+                        if (f32) {
+                            const float rf = (float)r.v[k];
+                            float pvf;
+                            if (kind == KIND_PPR || kind == KIND_UPPR) pvf = (omalpha_f * rf) / df;
+                            else if (kind == KIND_KATZ) pvf = alpha_f * rf;
+                            else if (kind == KIND_HK) pvf = sh.final_level ? rf / df : (hkc_f * rf) / df;
+                            else pvf = (omalpha_f * rf) / npush_f;
+                            push.v[k] = absorb ? T(0) : (T)pvf;
+                            xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(xgain_f * rf) : r.v[k];
                             r.v[k] = T(0);
-                            if constexpr (sizeof(T) == 8) {  // HK relaxation runs in FP64 only (host-checked)
-                                if (kind == KIND_HK && hk_relaxed(sh.tp)) {
-                                    const double thr = ((thr_scale[k] * du) / (double)sh.tp.n_levels) / sh.psi;
-                                    int subs;
-                                    double left;
-                                    const double moved = hk_relax(rv, sh.tp.omega, thr,
-                                                                  global ? sh.col_sweeps[c0 + k] : 0, &subs, &left);
-                                    if (sh.final_level) push.v[k] = moved / du;
-                                    else push.v[k] = ((sh.tp.tau / ((double)sh.level + 1.)) * moved) / du;
-                                    xadd.v[k] = moved;
-                                    r.v[k] = left;
-                                    my_oper[k] += (double)(subs - 1) * du;  // the first sub-push is counted below
-                                }
+                            wrote = true;
+                            sum.nodes[k] += 1;
+                            if (!absorb) sum.deg[k] += di;
+                            continue;
+                        }
+                        double pv;
+                        if (rdiv) pv = gain * rv;
+                        else if (kind == KIND_PPR || kind == KIND_UPPR) pv = ((1. - alpha) * rv) / du;
+                        else if (kind == KIND_KATZ) pv = alpha * rv;
+                        else if (kind == KIND_HK) {
+                            if (sh.final_level) pv = rv / du;  // hk_solver.py:254-256
+                            else pv = ((sh.tp.tau / ((double)sh.level + 1.)) * rv) / du;
+                        } else {
+                            pv = ((1. - alpha) * rv) / g.npush[u];  // InstantGNN.py:28
+                        }
+                        if (absorb) pv = 0.0;
+                        push.v[k] = (T)pv;
+                        xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(sh.tp.x_gain * rv) : r.v[k];
+                        r.v[k] = T(0);
+                        if constexpr (sizeof(T) == 8) {  // HK relaxation runs in FP64 only (host-checked)
+                            if (kind == KIND_HK && hk_relaxed(sh.tp)) {
+                                const double thr = ((thr_scale[k] * du) / (double)sh.tp.n_levels) / sh.psi;
+                                int subs;
+                                double left;
+                                const double moved = hk_relax(rv, sh.tp.omega, thr,
+                                                              global ? sh.col_sweeps[c0 + k] : 0, &subs, &left);
+                                if (sh.final_level) push.v[k] = moved / du;
+                                else push.v[k] = ((sh.tp.tau / ((double)sh.level + 1.)) * moved) / du;
+                                xadd.v[k] = moved;
+                                r.v[k] = left;
+                                sum.oper[k] += (double)(subs - 1) * du;  // the first sub-push is counted below
                             }
                         }
-                        wrote = true;
-                        my_nodes[k] += 1;
-                        if (!absorb) my_oper[k] += du;
                     }
-                    if (wrote) {
-                        vstore<T, VEC>(R + off, r);
-                        if (cheby) vstore<T, VEC>(DX + off, dxv);
-                        Vec<T, VEC> xv;
-                        vload<T, VEC>(X + xoff, xv);
-                        if (absorb) {
-                            // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
-    #pragma unroll
-                            for (int k = 0; k < VEC; ++k)
-                                if (act[k]) {
-                                    xv.v[k] = xadd.v[k];
-                                    if (XC) XC[xoff + k] = 0.f;
-                                }
-                        } else if (XC) {
-                            // Kahan-compensated FP32 accumulation of the solution
-                            Vec<float, VEC> cc;
-                            vload<float, VEC>(XC + xoff, cc);
-    #pragma unroll
-                            for (int k = 0; k < VEC; ++k)
-                                if (act[k]) {
-                                    float y = (float)xadd.v[k] - cc.v[k];
-                                    float s = (float)xv.v[k] + y;
-                                    cc.v[k] = (s - (float)xv.v[k]) - y;
-                                    xv.v[k] = (T)s;
-                                }
-                            vstore<float, VEC>(XC + xoff, cc);
-                        } else {
-    #pragma unroll
-                            for (int k = 0; k < VEC; ++k)
-                                if (act[k]) xv.v[k] = xv.v[k] + xadd.v[k];
-                        }
-                        vstore<T, VEC>(X + xoff, xv);
-                    }
-                    any = false;
-    #pragma unroll
-                    for (int k = 0; k < VEC; ++k) any |= act[k];
-                }
-            }
-            // ---- node-level frontier decision (OR over the lane group) ----
-            const unsigned bal = __ballot_sync(kFull, any);
-            if (bal == 0) continue;  // warp-uniform: nothing active in this warp
-            const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
-            const bool node_act = valid && (bal & gmask) != 0;
-            const bool leader = (lane_g == 0);
-            // Chebyshev moves r[u] by -dx[u]: u itself is a candidate next round
-            if (cheby && !global) append_once(leader && node_act, u, mark, sh.stamp, next, next_cnt, kFull);
-            const bool node_in = node_act && !absorb;  // absorbed nodes do not push
-            int len = 0;
-            int nch = 0;
-            long long rp = 0;
-            int bucket = -1;  // 0 short, 1 medium, 2 long
-            if (node_in && leader) {
-                len = g.row_len[u];
-                rp = g.row_ptr[u];
-                if (len <= a.small_max) bucket = 0;
-                else if (len <= a.med_max) bucket = 1;
-                else { bucket = 2; nch = (len + a.chunk - 1) / a.chunk; }
-            }
-            const unsigned bf = __ballot_sync(kFull, leader && node_in);
-            if (bf == 0) continue;
-            const unsigned bs = __ballot_sync(kFull, bucket == 0);
-            const unsigned bm = __ballot_sync(kFull, bucket == 1);
-            int lch = (bucket == 2) ? nch : 0;
-            int sc = lch;  // inclusive warp scan of chunk counts
-    #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(kFull, sc, o);
-                if (lane >= o) sc += y;
-            }
-            const int wch = __shfl_sync(kFull, sc, 31);
-            int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-            if (lane == 0) {
-                b0 = atomicAdd(&ts.front_cnt[par], __popc(bf));
-                if (bs) b1 = atomicAdd(&ts.small_cnt[par], __popc(bs));
-                if (bm) b2 = atomicAdd(&ts.med_cnt[par], __popc(bm));
-                if (wch) b3 = atomicAdd(&ts.large_cnt[par], wch);
-            }
-            b0 = __shfl_sync(kFull, b0, 0);
-            b1 = __shfl_sync(kFull, b1, 0);
-            b2 = __shfl_sync(kFull, b2, 0);
-            b3 = __shfl_sync(kFull, b3, 0);
-            const unsigned below = (1u << lane) - 1u;
-            int fidx = 0;
-            if (leader && node_in) {
-                fidx = b0 + __popc(bf & below);
-                PushItem item;
-                item.rp = rp;
-                item.len = len;
-                item.fidx = fidx;
-                if (bucket == 0) bsmall[b1 + __popc(bs & below)] = item;
-                else if (bucket == 1) bmed_end[-(b2 + __popc(bm & below))] = item;
-                else {
-                    int lb = b3 + (sc - lch);
-                    for (int ch = 0; ch < nch; ++ch) {
-                        item.rp = rp + (long long)ch * a.chunk;
-                        item.len = min(a.chunk, len - ch * a.chunk);
-                        blarge[lb + ch] = item;
+                    wrote = true;
+                    sum.nodes[k] += 1;
+                    if (!absorb) {
+                        if (dint) sum.deg[k] += di;
+                        else sum.oper[k] += du;
                     }
                 }
-                my_vol += du;
-                my_cnt += 1;
+                if (wrote) {
+                    vstore<T, VEC>(R + off, r);
+                    if (cheby) vstore<T, VEC>(DX + off, dxv);
+                    Vec<T, VEC> xv;
+                    vload<T, VEC>(X + xoff, xv);
+                    if (absorb) {
+                        // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
+#pragma unroll
+                        for (int k = 0; k < VEC; ++k)
+                            if (act[k]) {
+                                xv.v[k] = xadd.v[k];
+                                if (XC) XC[xoff + k] = 0.f;
+                            }
+                    } else if (XC) {
+                        // Kahan-compensated FP32 accumulation of the solution
+                        Vec<float, VEC> cc;
+                        vload<float, VEC>(XC + xoff, cc);
+#pragma unroll
+                        for (int k = 0; k < VEC; ++k)
+                            if (act[k]) {
+                                float y = (float)xadd.v[k] - cc.v[k];
+                                float s = (float)xv.v[k] + y;
+                                cc.v[k] = (s - (float)xv.v[k]) - y;
+                                xv.v[k] = (T)s;
+                            }
+                        vstore<float, VEC>(XC + xoff, cc);
+                    } else {
+#pragma unroll
+                        for (int k = 0; k < VEC; ++k)
+                            if (act[k]) xv.v[k] = xv.v[k] + xadd.v[k];
+                    }
+                    vstore<T, VEC>(X + xoff, xv);
+                }
+                any = false;
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) any |= act[k];
             }
-            fidx = __shfl_sync(kFull, fidx, grp_w * L);
-            if (node_in) vstore<T, VEC>(Pw + (int64_t)fidx * W + c0, push);
         }
+        // ---- node-level frontier decision (OR over the lane group) ----
+        const unsigned bal = __ballot_sync(kFull, any);
+        if (bal == 0) continue;  // warp-uniform: nothing active in this warp
+        const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
+        const bool node_act = valid && (bal & gmask) != 0;
+        const bool leader = (lane_g == 0);
+        // Chebyshev moves r[u] by -dx[u]: u itself is a candidate next round
+        if (cheby && !global) append_once(leader && node_act, u, mark, sh.stamp, next, next_cnt, kFull);
+        const bool node_in = node_act && !absorb;  // absorbed nodes do not push
+        if (PULL && bits) {
+            // a pull round: the push row by node, and the node's frontier
+            // bit (a dense scan's nodes are consecutive: two words at most)
+            if (node_in) vstore<T, VEC>(Pw + (int64_t)u * W + c0, push);
+            const bool in = leader && node_in;
+            if (in) {
+                if (dint) sum.ivol += di;
+                else sum.vol += du;
+                sum.cnt += 1;
+            }
+            if (sh.dense) {
+                const int w0 = (int)(base >> 5);
+                const uint32_t bit = in ? 1u << (u & 31) : 0u;
+                const uint32_t b0 = __reduce_or_sync(kFull, (u >> 5) == w0 ? bit : 0u);
+                const uint32_t b1 = __reduce_or_sync(kFull, (u >> 5) == w0 ? 0u : bit);
+                if (lane == 0 && b0) atomicOr(bits + w0, b0);
+                if (lane == 0 && b1) atomicOr(bits + w0 + 1, b1);
+            } else if (in) {
+                atomicOr(bits + (u >> 5), 1u << (u & 31));
+            }
+            continue;
+        }
+        int len = 0;
+        int nch = 0;
+        long long rp = 0;
+        int bucket = -1;  // 0 short, 1 medium, 2 long
+        if (node_in && leader) {
+            len = g.row_len[u];
+            rp = g.row_ptr[u];
+            if (len <= a.small_max) bucket = 0;
+            else if (len <= a.med_max) bucket = 1;
+            else { bucket = 2; nch = (len + a.chunk - 1) / a.chunk; }
+        }
+        const unsigned bf = __ballot_sync(kFull, leader && node_in);
+        if (bf == 0) continue;
+        const unsigned bs = __ballot_sync(kFull, bucket == 0);
+        const unsigned bm = __ballot_sync(kFull, bucket == 1);
+        int lch = (bucket == 2) ? nch : 0;
+        int sc = lch;  // inclusive warp scan of chunk counts
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            int y = __shfl_up_sync(kFull, sc, o);
+            if (lane >= o) sc += y;
+        }
+        const int wch = __shfl_sync(kFull, sc, 31);
+        int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
+        if (lane == 0) {
+            b0 = atomicAdd(&ts.front_cnt[par], __popc(bf));
+            if (bs) b1 = atomicAdd(&ts.small_cnt[par], __popc(bs));
+            if (bm) b2 = atomicAdd(&ts.med_cnt[par], __popc(bm));
+            if (wch) b3 = atomicAdd(&ts.large_cnt[par], wch);
+        }
+        b0 = __shfl_sync(kFull, b0, 0);
+        b1 = __shfl_sync(kFull, b1, 0);
+        b2 = __shfl_sync(kFull, b2, 0);
+        b3 = __shfl_sync(kFull, b3, 0);
+        const unsigned below = (1u << lane) - 1u;
+        int fidx = 0;
+        if (leader && node_in) {
+            fidx = b0 + __popc(bf & below);
+            PushItem item;
+            item.rp = rp;
+            item.len = len;
+            item.fidx = fidx;
+            if (bucket == 0) bsmall[b1 + __popc(bs & below)] = item;
+            else if (bucket == 1) bmed_end[-(b2 + __popc(bm & below))] = item;
+            else {
+                int lb = b3 + (sc - lch);
+                for (int ch = 0; ch < nch; ++ch) {
+                    item.rp = rp + (long long)ch * a.chunk;
+                    item.len = min(a.chunk, len - ch * a.chunk);
+                    blarge[lb + ch] = item;
+                }
+            }
+            if (dint) sum.ivol += di;
+            else sum.vol += du;
+            sum.cnt += 1;
+        }
+        fidx = __shfl_sync(kFull, fidx, grp_w * L);
+        if (node_in) vstore<T, VEC>(Pw + (int64_t)fidx * W + c0, push);
+    }
+    total = sum;
+}
+
+// PREP over candidates [beg, end) of tile t, by the loop that fits the tile,
+// then this block's counts into the tile's.
+template <typename T, int W, bool PULL>
+__device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& ps, long long beg, long long end) {
+    constexpr int VEC = PrepSums<T, W>::VEC;
+    const int par = sh.parity;
+    const int c0 = ((threadIdx.x & 31) % (W / VEC)) * VEC;
+    TileState& ts = a.ts[t];
+    if (threadIdx.x < W) { ps.col_oper[threadIdx.x] = 0.0; ps.col_nodes[threadIdx.x] = 0; }
+    if (threadIdx.x == 0) { ps.vol = 0.0; ps.nodes = 0; }
+    __syncthreads();
+    PrepSums<T, W> sum;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) { sum.oper[k] = 0.0; sum.deg[k] = 0; sum.nodes[k] = 0; }
+    sum.vol = 0.0;
+    sum.ivol = 0;
+    sum.cnt = 0;
+    if constexpr (W == 1) {
+        // A W = 1 crossing tile visits exactly the nodes that crossed their
+        // threshold last round: every candidate is active, so all its loads are
+        // issued at once.
+        if (tile_crosses(sh.tp) && !sh.dense && sh.col_live[0])
+            prep_w1_cross<T, PULL>(a, t, sh, beg, end, sum.oper[0], sum.nodes[0], sum.vol, sum.cnt);
+        else
+            prep_nodes<T, W, PULL>(a, t, sh, beg, end, sum);
+    } else {
+        if (sh.pull && !method_is_cheby(sh.tp.method) && !(sh.tp.kind == KIND_HK && hk_relaxed(sh.tp)))
+            prep_pull<T, W>(a, t, sh, beg, end, sum);
+        else
+            prep_nodes<T, W, PULL>(a, t, sh, beg, end, sum);
     }
     // ---- flush per-column counters (one global atomic per column per block) ----
 #pragma unroll
     for (int k = 0; k < VEC; ++k) {
-        if (my_nodes[k]) {
-            atomicAdd(&ps.col_nodes[c0 + k], my_nodes[k]);
-            atomicAdd(&ps.col_oper[c0 + k], my_oper[k]);
+        if (sum.nodes[k]) {
+            atomicAdd(&ps.col_nodes[c0 + k], sum.nodes[k]);
+            atomicAdd(&ps.col_oper[c0 + k], sum.oper[k] + (double)sum.deg[k]);
         }
     }
-    if (my_cnt) {
-        atomicAdd(&ps.vol, my_vol);
-        atomicAdd(&ps.nodes, my_cnt);
+    if (sum.cnt) {
+        atomicAdd(&ps.vol, sum.vol + (double)sum.ivol);
+        atomicAdd(&ps.nodes, sum.cnt);
     }
     __syncthreads();
     if (threadIdx.x < W && ps.col_nodes[threadIdx.x]) {
@@ -1021,6 +1339,7 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
     }
     if (threadIdx.x == 0 && ps.nodes) {
         atomicAdd(&ts.union_vol[par], ps.vol);
+        if (PULL && sh.pull) atomicAdd(&ts.front_cnt[par], ps.nodes);  // push rounds count while they compact
         ps.acc_union_nodes += (unsigned long long)ps.nodes;
         ps.acc_union_vol += ps.vol;
     }
@@ -1120,8 +1439,7 @@ __device__ __forceinline__ bool crossed(const DevGraph& g, int v, T old, T s, do
             return !ge_threshold((float)old, t32, theta, (double)df) && ge_threshold((float)s, t32, theta, (double)df);
         }
     }
-    const double thr = theta * (g.degf_exact ? (double)g.degf[v] : g.degd[v]);
-    return ((double)old < thr) && ((double)s >= thr);
+    return crossed64((double)old, (double)s, theta * (g.degf_exact ? (double)g.degf[v] : g.degd[v]));
 }
 
 template <typename T, int VEC>
@@ -1205,9 +1523,15 @@ __device__ __forceinline__ void push_edge(const DevGraph& g, T* tgt, int64_t ld,
     Vec<T, VEC> q = p;
     if (tgt_scale) {
         // InstantGNN divides by d_v^beta at the target (InstantGNN.py:31)
-        T dv = (sizeof(T) == 4) ? (T)g.tfac_f[v] : (T)g.tfac[v];
+        if (sizeof(T) == 8 && g.rtf) {
+            const T rv = (T)g.rtf[v];
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) q.v[i] = q.v[i] / dv;
+            for (int i = 0; i < VEC; ++i) q.v[i] = q.v[i] * rv;
+        } else {
+            const T dv = (sizeof(T) == 4) ? (T)g.tfac_f[v] : (T)g.tfac[v];
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) q.v[i] = q.v[i] / dv;
+        }
     }
     vred<T, VEC>(tgt + (int64_t)v * ld + c0, q);
 }
@@ -1328,8 +1652,7 @@ __device__ __forceinline__ void edges_w1(const PushArgs& a, const ScatterCtx<T, 
                     }
                 }
                 const double dv = g.degf_exact ? (double)df[u] : g.degd[v[u]];
-                const double thr = theta * dv;
-                cr[u] = ((double)old[u] < thr) && ((double)s >= thr);
+                cr[u] = crossed64((double)old[u], (double)s, theta * dv);
             }
         }
         append_crossings(cr, v, c.next, c.next_cnt);
@@ -1625,6 +1948,240 @@ __device__ void scatter_small_flat(const PushArgs& a, int t, const ScatterCtx<T,
     }
 }
 
+// ---------------------------------------------------------------------------
+// PULL: a round whose frontier holds a good part of the graph's volume does
+// not push along its rows with atomics.  Every row gathers instead: node v
+// adds up its frontier neighbours' push rows (P by node id; the frontier
+// bitmap, small enough for the L1, tells which neighbours push), and one
+// plain read-modify-write updates its residual.  The adjacency is symmetric
+// (checked by the host), so v's row names exactly the nodes whose rows name v.
+// Touched nodes and threshold crossings are those of the push.
+//
+// Random atomics, FP64 ones above all, are the slow part of a push round
+// (22 to 30 G/s measured); a gather of the same edges reads L2 sectors without
+// them.  SCATTER's time with pull rounds, before -> after: 128 FP64 columns of
+// the 169k-node InstantGNN push 726 -> 79 ms, its 64-column update 211 -> 26,
+// 256 FP64 seeds in 8-column tiles on 87k nodes 128 -> 49, 8 FP32 columns of
+// global GD on 2.36M nodes 34 -> 11.  What is left is the latency of the chain
+// record -> columns -> bitmap and push rows, and FP64 additions.
+//
+// Rows come in the order of their capacity (a.g.pord), so the lane groups of
+// a warp work on rows of about the same length: long rows as chunks by whole
+// warps, middle rows by MS groups each, short rows by one group each.  Units
+// of work are dealt to warps round-robin, tile by tile: all blocks read one
+// tile's push rows at a time, which then stay in the L2.
+// ---------------------------------------------------------------------------
+template <typename T, int W, int SPLIT, typename A>
+__device__ __forceinline__ bool pull_edges(const DevGraph& g, const T* P, const uint32_t* bits,
+                                           long long rp, int beg, int end, int sub, int c0,
+                                           A (&acc)[(sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1)]) {
+    constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    constexpr int U = 4;  // neighbours in flight per lane group
+    bool any = false;
+    for (int j = beg + sub; j < end; j += SPLIT * U) {
+        int w[U];
+        bool on[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) w[i] = (j + i * SPLIT < end) ? g.col[rp + j + i * SPLIT] : -1;
+#pragma unroll
+        for (int i = 0; i < U; ++i) on[i] = w[i] >= 0 && ((bits[w[i] >> 5] >> (w[i] & 31)) & 1u);
+        Vec<T, VEC> p[U];
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) p[i].v[k] = T(0);
+            if (on[i]) vload<T, VEC>(P + (int64_t)w[i] * W + c0, p[i]);
+        }
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            any |= on[i];
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) acc[k] += (A)p[i].v[k];
+        }
+    }
+    return any;
+}
+
+// The gathered sum of node v into its residual: plainly, or (shared: a chunk
+// of a row that other warps work on too) with an atomic; then the append of v
+// on a crossing or, for tracking tiles, on a touch.  Every lane of the warp
+// calls it; ok holds for the lanes of one group per row.
+template <typename T, int W, typename A>
+__device__ __forceinline__ void pull_flush(const PushArgs& a, const ScatterCtx<T, W>& c, bool ok, bool shared_row,
+                                           int v, int c0, int lane_g, int grp_w,
+                                           const A (&acc)[(sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1)],
+                                           const double (&theta)[(sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1)],
+                                           const float (&theta_f)[(sizeof(T) == 4) ? (W >= 4 ? 4 : W)
+                                                                                   : (W >= 2 ? 2 : 1)]) {
+    constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    constexpr int L = W / VEC;
+    const DevGraph& g = a.g;
+    bool cr = false;
+    if (ok) {
+        if (W == 1 && sizeof(T) == 4 && c.rh && v < c.rh_cut) {
+            // FP64 hub prefix: the sum, the residual and the crossing test in FP64
+            const double add = (double)acc[0];
+            double old;
+            if (shared_row) {
+                old = atomicAdd(c.rh + v, add);
+            } else {
+                old = c.rh[v];
+                c.rh[v] = old + add;
+            }
+            const double thr = theta[0] * (g.degf_exact ? (double)g.degf[v] : g.degd[v]);
+            cr = (old < thr) && (old + add >= thr);
+        } else {
+            Vec<T, VEC> q, old;
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) q.v[k] = (T)acc[k];
+            if (c.tgt_scale) {
+                // InstantGNN divides by d_v^beta at the target (InstantGNN.py:31)
+                if (sizeof(T) == 8 && g.rtf) {
+                    const T rv = (T)g.rtf[v];
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) q.v[k] = q.v[k] * rv;
+                } else {
+                    const T dv = (sizeof(T) == 4) ? (T)g.tfac_f[v] : (T)g.tfac[v];
+#pragma unroll
+                    for (int k = 0; k < VEC; ++k) q.v[k] = q.v[k] / dv;
+                }
+            }
+            T* r = c.tgt + (int64_t)v * c.tld + c0;
+            if (shared_row) {
+                if (c.cross) vatomic_ret<T, VEC>(r, q, old);
+                else vred<T, VEC>(r, q);
+            } else {
+                Vec<T, VEC> s;
+                vload<T, VEC>(r, old);
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) s.v[k] = old.v[k] + q.v[k];
+                vstore<T, VEC>(r, s);
+            }
+            if (c.cross) {
+#pragma unroll
+                for (int k = 0; k < VEC; ++k)
+                    if (q.v[k] != T(0)) cr |= crossed<T>(g, v, old.v[k], (T)(old.v[k] + q.v[k]), theta[k], theta_f[k]);
+            }
+        }
+    }
+    if (c.cross) {
+        const unsigned b = __ballot_sync(kFull, cr);
+        const unsigned gm = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
+        append_once(ok && lane_g == 0 && (b & gm) != 0, v, c.mark, c.stamp, c.next, c.next_cnt, kFull);
+    } else if (c.track) {
+        append_once(ok && lane_g == 0, v, c.mark, c.stamp, c.next, c.next_cnt, kFull);
+    }
+}
+
+// One unit: the rows [pos, pos + GPW / SPLIT) of the order (rows below `last`), SPLIT lane groups per row.
+template <typename T, int W, int SPLIT>
+__device__ __forceinline__ void pull_rows(const PushArgs& a, const ScatterCtx<T, W>& c, const uint32_t* bits,
+                                          long long pos, long long last) {
+    constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    constexpr int L = W / VEC;
+    const DevGraph& g = a.g;
+    const int lane = threadIdx.x & 31;
+    const int lane_g = lane % L, grp_w = lane / L;
+    const int c0 = lane_g * VEC;
+    const int sub = grp_w % SPLIT;
+    const long long i = pos + grp_w / SPLIT;
+    int v = 0, len = 0;
+    long long rp = 0;
+    if (i < last) {
+        v = g.pord ? g.pord[i] : (int)i;
+        if (g.rec) {
+            const NodeRec nr = g.rec[v];
+            rp = nr.rp;
+            len = nr.len;
+        } else {
+            rp = g.row_ptr[v];
+            len = g.row_len[v];
+        }
+    }
+    T acc[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = T(0);
+    bool any = pull_edges<T, W, SPLIT, T>(g, c.Pw, bits, rp, 0, len, sub, c0, acc);
+    __syncwarp();
+#pragma unroll
+    for (int o = 1; o < SPLIT; o <<= 1) {
+        any |= __shfl_xor_sync(kFull, (int)any, o * L) != 0;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) acc[k] += __shfl_xor_sync(kFull, acc[k], o * L);
+    }
+    if (__ballot_sync(kFull, any) == 0) return;
+    double theta[VEC];
+    float theta_f[VEC];
+    load_thetas<T, VEC>(c.cs, c0, c.cross, theta, theta_f);
+    pull_flush<T, W, T>(a, c, any && sub == 0, false, v, c0, lane_g, grp_w, acc, theta, theta_f);
+}
+
+// One unit: a chunk of a long row, the whole warp on it.  A sum into an FP64
+// hub residual is formed in FP64, as the pushes into it are.
+template <typename T, int W, typename A>
+__device__ __forceinline__ void pull_chunk(const PushArgs& a, const ScatterCtx<T, W>& c, const uint32_t* bits, int v,
+                                           long long rp, int beg, int len) {
+    constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    constexpr int L = W / VEC;
+    constexpr int GPW = 32 / L;
+    const int lane = threadIdx.x & 31;
+    const int lane_g = lane % L, grp_w = lane / L;
+    const int c0 = lane_g * VEC;
+    A acc[VEC];
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) acc[k] = A(0);
+    bool any = pull_edges<T, W, GPW, A>(a.g, c.Pw, bits, rp, beg, min(beg + kPullChunk, len), grp_w, c0, acc);
+    any = __any_sync(kFull, any);
+    if (!any) return;
+#pragma unroll
+    for (int o = L; o < 32; o <<= 1)
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) acc[k] += __shfl_xor_sync(kFull, acc[k], o);
+    double theta[VEC];
+    float theta_f[VEC];
+    load_thetas<T, VEC>(c.cs, c0, c.cross, theta, theta_f);
+    pull_flush<T, W, A>(a, c, grp_w == 0, len > kPullChunk, v, c0, lane_g, grp_w, acc, theta, theta_f);
+}
+
+// Every row of the npull live tiles in `list` (indices into rs.tiles).
+template <typename T, int W>
+__device__ __noinline__ void pull_phase(const PushArgs& a, const RoundSh& rs, const short* list, int npull,
+                                        const GroupInfo& gi) {
+    constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
+    constexpr int GPW = 32 / (W / VEC);
+    constexpr int MS = GPW >= 4 ? GPW / 4 : 1;  // lane groups per middle row
+    constexpr int MR = GPW / MS;
+    const DevGraph& g = a.g;
+    const unsigned u_long = (unsigned)g.npchunk;
+    const unsigned u_mid = u_long + (unsigned)((g.pull_mid - g.pull_long + MR - 1) / MR);
+    const unsigned units = u_mid + (unsigned)((g.n - g.pull_mid + GPW - 1) / GPW);
+    const unsigned nw = (unsigned)gi.dim * kWarps;
+    unsigned u = (unsigned)gi.blk * kWarps + (threadIdx.x >> 5);
+    for (int p = 0; p < npull; ++p) {
+        const int k = list[p];
+        const int t = rs.tiles[k];
+        const uint32_t* bits = tile_bits(a, t, rs.level[k] & 1);
+        const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, rs.level[k], rs.flags[k]);
+        for (; u < units; u += nw) {
+            if (u < u_long) {
+                const int2 ch = g.pchunk[u];
+                const int len = g.row_len[ch.x];
+                if (ch.y >= len && ch.y > 0) continue;
+                const long long rp = g.row_ptr[ch.x];
+                if (W == 1 && sizeof(T) == 4 && c.rh && ch.x < c.rh_cut)
+                    pull_chunk<T, W, double>(a, c, bits, ch.x, rp, ch.y, len);
+                else
+                    pull_chunk<T, W, T>(a, c, bits, ch.x, rp, ch.y, len);
+            } else if (u < u_mid) {
+                pull_rows<T, W, MS>(a, c, bits, g.pull_long + (long long)(u - u_long) * MR, g.pull_mid);
+            } else {
+                pull_rows<T, W, 1>(a, c, bits, g.pull_mid + (long long)(u - u_mid) * GPW, g.n);
+            }
+        }
+        u -= units;  // the next tile's units follow round-robin
+    }
+}
+
 // HK: drop this level's sub-threshold residuals (hk_solver.py:284); the
 // frontier's own entries were already moved into x.
 template <typename T, int W>
@@ -1688,6 +2245,7 @@ __device__ void finish_round(const PushArgs& a, int t, int level, bool dense_nex
     {
         TileState& ts = a.ts[t];
         ts.dense_next[par ^ 1] = dense_next ? 1 : 0;
+        ts.pull[par ^ 1] = pull_next_round(a, ts, par) ? 1 : 0;
         // a served heat-kernel slot ends one (empty) round after its last
         // level: that level pushes into x during SCATTER, so x is read out by
         // the next round's retire
@@ -1793,7 +2351,7 @@ __device__ void admit_query(const PushArgs& a, int t, int it) {
     for (int i = 0; i < 3; ++i) ts.cand_cnt[i] = 0;
     for (int i = 0; i < 2; ++i) {
         ts.front_cnt[i] = ts.small_cnt[i] = ts.med_cnt[i] = ts.large_cnt[i] = 0;
-        ts.dense_next[i] = 0;
+        ts.dense_next[i] = ts.pull[i] = 0;
         ts.union_vol[i] = 0.0;
     }
     a.cand[((int64_t)t * 2 + 0) * n] = seed;  // level-0 candidates: the seed
@@ -1990,7 +2548,7 @@ __device__ bool admit_online(const PushArgs& a, int t, int it) {
     for (int i = 0; i < 3; ++i) ts.cand_cnt[i] = 0;
     for (int i = 0; i < 2; ++i) {
         ts.front_cnt[i] = ts.small_cnt[i] = ts.med_cnt[i] = ts.large_cnt[i] = 0;
-        ts.dense_next[i] = 0;
+        ts.dense_next[i] = ts.pull[i] = 0;
         ts.union_vol[i] = 0.0;
     }
     const int64_t n = a.g.n;
@@ -2358,7 +2916,10 @@ __device__ __forceinline__ void trace_point(const PushArgs& a, int it, int k) {
         a.trace[((size_t)it * gridDim.x + blockIdx.x) * kTracePoints + k] = globaltimer_ns();
 }
 
-template <typename T, int W>
+// PULL: the launch may pull (a.pull_div > 0).  One-column launches that never
+// do run an instantiation without that code: its registers cost the served
+// FP32 slots 4%.
+template <typename T, int W, bool PULL>
 __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_MIN_BLOCKS_W1
                                            : (W <= 8 && sizeof(T) == 4) ? GDE_MIN_BLOCKS_F32
                                                                         : GDE_MIN_BLOCKS)
@@ -2466,7 +3027,7 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
                     const long long e = min(hi, rs.off[0][k + 1]) - rs.off[0][k];
                     if (b >= e) continue;
                     load_tile<W>(a, rs.tiles[k], it, sh);
-                    prep_range<T, W>(a, rs.tiles[k], sh, ps, b, e);
+                    prep_range<T, W, PULL>(a, rs.tiles[k], sh, ps, b, e);
                 }
             }
         }
@@ -2497,6 +3058,7 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             if (tp.kind == KIND_IGN) f |= SF_TGTSCALE;
             if (tile_crosses(tp)) f |= SF_CROSS;
             else if (!dnext && !fin && !last_taylor) f |= SF_TRACK;
+            if (ts.pull[par] && ts.front_cnt[par] > 0 && !last_taylor) f |= SF_PULL;
             rs.flags[k] = f;
             const bool has = ts.front_cnt[par] > 0 && !last_taylor;
             s_vals[k] = has ? ts.small_cnt[par] : 0;
@@ -2570,6 +3132,33 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
                     else if (sp == 1) scatter_warp_items<T, W>(a, a.bsmall + (int64_t)t * n + (n - 1), -1, c, b, e);
                     else scatter_small_flat<T, W>(a, t, c, b, e);
                 }
+            }
+        }
+        // tiles whose round pulls have no work items above
+        if (PULL && a.pull_div > 0) {
+            if (threadIdx.x < 32) {
+                int np = 0;
+                for (int k0 = 0; k0 < ntl; k0 += 32) {
+                    const int k = k0 + threadIdx.x;
+                    const bool p = k < ntl && (rs.flags[k] & SF_PULL);
+                    const unsigned b = __ballot_sync(kFull, p);
+                    if (p) rs.pull[np + __popc(b & ((1u << threadIdx.x) - 1u))] = (short)k;
+                    np += __popc(b);
+                }
+                if (threadIdx.x == 0) rs.npull = np;
+            }
+            __syncthreads();
+            if constexpr (PULL)
+                if (rs.npull > 0) pull_phase<T, W>(a, rs, rs.pull, rs.npull, gi);
+            // a clear bitmap for each tile whose next round pulls
+            for (int k = 0; k < ntl; ++k) {
+                const int t = rs.tiles[k];
+                const int par = rs.level[k] & 1;
+                if (!pull_next_round(a, a.ts[t], par)) continue;
+                uint32_t* b = tile_bits(a, t, par ^ 1);
+                for (int64_t w = (int64_t)gi.blk * kThreads + threadIdx.x; w < a.bit_words;
+                     w += (int64_t)gi.dim * kThreads)
+                    b[w] = 0u;
             }
         }
         trace_point(a, it, TP_SCAT_DONE);
@@ -2656,65 +3245,53 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
 
 }  // namespace
 
-// Host-side launcher: picks the instantiation for (T, W) and launches it
-// cooperatively with the largest co-resident grid.
-template <typename T, int W>
-static cudaError_t launch_t(const PushArgs& a, int grid, cudaStream_t st) {
-    void* args[] = {const_cast<PushArgs*>(&a)};
-    return cudaLaunchCooperativeKernel((void*)push_kernel<T, W>, dim3(grid), dim3(kThreads), args, 0, st);
-}
-
-template <typename T, int W>
+// Host-side launcher: picks the instantiation for (T, W, PULL) and launches
+// it cooperatively with the largest co-resident grid.
+template <typename T, int W, bool PULL>
 static int max_grid_t(int sms) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, push_kernel<T, W>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, push_kernel<T, W, PULL>, kThreads, 0);
     return per_sm * sms;
 }
 
-int engine_max_grid(int prec64, int W, int sms) {
-    if (prec64) {
-        switch (W) {
-            case 1: return max_grid_t<double, 1>(sms);
-            case 2: return max_grid_t<double, 2>(sms);
-            case 4: return max_grid_t<double, 4>(sms);
-            case 8: return max_grid_t<double, 8>(sms);
-            case 16: return max_grid_t<double, 16>(sms);
-            case 32: return max_grid_t<double, 32>(sms);
-        }
-    } else {
-        switch (W) {
-            case 1: return max_grid_t<float, 1>(sms);
-            case 2: return max_grid_t<float, 2>(sms);
-            case 4: return max_grid_t<float, 4>(sms);
-            case 8: return max_grid_t<float, 8>(sms);
-            case 16: return max_grid_t<float, 16>(sms);
-            case 32: return max_grid_t<float, 32>(sms);
-        }
+template <typename T, int W, bool PULL>
+static cudaError_t launch_t(const PushArgs& a, int grid, cudaStream_t st) {
+    void* args[] = {const_cast<PushArgs*>(&a)};
+    return cudaLaunchCooperativeKernel((void*)push_kernel<T, W, PULL>, dim3(grid), dim3(kThreads), args, 0, st);
+}
+
+template <typename T>
+static int max_grid_w(int W, bool pull, int sms) {
+    switch (W) {
+        case 1: return pull ? max_grid_t<T, 1, true>(sms) : max_grid_t<T, 1, false>(sms);
+        case 2: return max_grid_t<T, 2, true>(sms);
+        case 4: return max_grid_t<T, 4, true>(sms);
+        case 8: return max_grid_t<T, 8, true>(sms);
+        case 16: return max_grid_t<T, 16, true>(sms);
+        case 32: return max_grid_t<T, 32, true>(sms);
     }
     return 0;
 }
 
-cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st) {
-    if (prec64) {
-        switch (W) {
-            case 1: return launch_t<double, 1>(a, grid, st);
-            case 2: return launch_t<double, 2>(a, grid, st);
-            case 4: return launch_t<double, 4>(a, grid, st);
-            case 8: return launch_t<double, 8>(a, grid, st);
-            case 16: return launch_t<double, 16>(a, grid, st);
-            case 32: return launch_t<double, 32>(a, grid, st);
-        }
-    } else {
-        switch (W) {
-            case 1: return launch_t<float, 1>(a, grid, st);
-            case 2: return launch_t<float, 2>(a, grid, st);
-            case 4: return launch_t<float, 4>(a, grid, st);
-            case 8: return launch_t<float, 8>(a, grid, st);
-            case 16: return launch_t<float, 16>(a, grid, st);
-            case 32: return launch_t<float, 32>(a, grid, st);
-        }
+template <typename T>
+static cudaError_t launch_w(const PushArgs& a, int W, int grid, cudaStream_t st) {
+    switch (W) {
+        case 1: return a.pull_div > 0 ? launch_t<T, 1, true>(a, grid, st) : launch_t<T, 1, false>(a, grid, st);
+        case 2: return launch_t<T, 2, true>(a, grid, st);
+        case 4: return launch_t<T, 4, true>(a, grid, st);
+        case 8: return launch_t<T, 8, true>(a, grid, st);
+        case 16: return launch_t<T, 16, true>(a, grid, st);
+        case 32: return launch_t<T, 32, true>(a, grid, st);
     }
     return cudaErrorInvalidValue;
+}
+
+int engine_max_grid(int prec64, int W, bool pull, int sms) {
+    return prec64 ? max_grid_w<double>(W, pull, sms) : max_grid_w<float>(W, pull, sms);
+}
+
+cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st) {
+    return prec64 ? launch_w<double>(a, W, grid, st) : launch_w<float>(a, W, grid, st);
 }
 
 }  // namespace gde

@@ -276,7 +276,7 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
     CK_S(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    s->grid = engine_max_grid(s->prec64, 1, sms);
+    s->grid = engine_max_grid(s->prec64, 1, false, sms);
     if (s->grid <= 0) {
         int rc = s->fail(GDE_ECUDA, "push kernel does not fit on the device");
         s->free_all();
