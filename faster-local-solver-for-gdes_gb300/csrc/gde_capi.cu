@@ -353,11 +353,14 @@ int enable_reciprocals(gde_ctx* ctx, gde_graph* G, PushArgs& a, int kind) {
 
 // Run the persistent engine until every tile is done (or max_rounds).
 int run_engine(gde_ctx* ctx, PushArgs& a, int prec64, int W, gde_stats* st, double* kernel_ms) {
-    int grid = engine_max_grid(prec64, W, a.pull_div > 0, ctx->sms);
+    int grid = engine_max_grid(a, prec64, W, ctx->sms);
     if (grid <= 0) return fail(ctx, GDE_ECUDA, "push kernel does not fit on the device");
     if (a.serve && a.queue.sp_blocks > grid / 2) a.queue.sp_blocks = grid / 2;  // at least half the grid stays dense
     const int dense_grid = grid - (a.serve ? a.queue.sp_blocks : 0);
-    if (a.groups > dense_grid) a.groups = dense_grid;  // every group holds at least one block
+    if (a.groups > dense_grid) {  // every group holds at least one block
+        a.groups = dense_grid;
+        grid = std::min(grid, engine_max_grid(a, prec64, W, ctx->sms));
+    }
     CK(cudaMemsetAsync(ctx->bar, 0, kMaxGroups * sizeof(GridBarrier), ctx->stream));
     CK(cudaMemsetAsync(ctx->derr, 0, sizeof(int), ctx->stream));
     CK(cudaMemsetAsync(ctx->dstats, 0, sizeof(LaunchStats), ctx->stream));

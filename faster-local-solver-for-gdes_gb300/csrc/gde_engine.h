@@ -7,8 +7,8 @@
 namespace gde {
 
 // Persistent push engine (push_engine.cu).
-// (pull: the launch's a.pull_div > 0; max_grid and launch must agree on it.)
-int engine_max_grid(int prec64, int W, bool pull, int sms);
+// (max_grid goes by the launch's ntiles, groups and pull_div: they are set before it)
+int engine_max_grid(const PushArgs& a, int prec64, int W, int sms);
 cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st);
 
 // Column initialisation and result extraction (aux_kernels.cu).

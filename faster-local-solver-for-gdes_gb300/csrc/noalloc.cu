@@ -225,7 +225,7 @@ extern "C" int gde_solve_noalloc(gde_ctx* ctx, gde_graph* G, const gde_params* p
 
     // ---- seed, push to completion, extract ----
     NA_CK(init_columns(a, prec64, 1, d_ic, 1, st));
-    const int grid = engine_max_grid(prec64, 1, false, gde_internal_sms(ctx));
+    const int grid = engine_max_grid(a, prec64, 1, gde_internal_sms(ctx));
     if (grid <= 0) return gde_internal_fail(ctx, GDE_ECUDA, "push kernel does not fit on the device");
     NA_CK(engine_launch(a, prec64, 1, grid, st));
     if (x_out || r_out) NA_CK(extract_columns(a, prec64, 1, d_ec, 1, x_out, r_out, out64, n, n, 0, st));

@@ -426,28 +426,36 @@ __device__ void check_phase(const PushArgs& a, int t, int it, int* s_cnt) {
 // matter how it is spread over tiles, and a block touches only the one or
 // two tiles its share overlaps.
 // ---------------------------------------------------------------------------
-constexpr int kMaxLaunchTiles = 512;
-
-struct RoundSh {
-    int ntl;                                    // live tiles this round
-    int any_check;                              // some live tile needs a CHECK phase
-    int any_idle;                               // served solves: some slot awaits a query
-    int tiles[kMaxLaunchTiles];                 // live tile ids (ascending)
-    unsigned char idle[kMaxLaunchTiles];        // 1: slot idle at the round start; 2: draining (online)
-    union {
-        short drain[kMaxLaunchTiles];           // online slots to clear this round (SLOT_DRAIN)
-        short pull[kMaxLaunchTiles];            // other launches: live tiles whose round pulls
-    };
-    int ndrain;
-    int npull;
-    long long off[4][kMaxLaunchTiles + 1];      // exclusive prefix sums of the current phase's spaces
-    int level[kMaxLaunchTiles];                 // per live tile: rounds since its start
-    unsigned char flags[kMaxLaunchTiles];       // per live tile scatter flags (SF_*)
-    long long scan_tmp[kWarps];
+// One entry per tile of the block's group (and one more: the prefix sums'
+// ends), in dynamic shared memory sized by the launch: a served launch with a
+// group per slot needs two entries, and what 512 would take goes to the L1
+// (five blocks of 32 KB per SM: 100 bytes instead of 28 KB of it each).  One
+// warp fills it with no block-wide scans.  A single FP32 query on 2.36M nodes
+// took 2.31 -> 2.17 ms with both, and the kernel's parameters in constant
+// memory instead of a stack copy for the out-of-line calls.
+struct TileSlot {
+    long long off[4];     // by live tile: exclusive prefix sums of the current phase's spaces
+    int tile;             // by live tile: its id (ascending)
+    int level;            //               rounds since its start
+    short drain;          // online: the k-th slot to clear this round (SLOT_DRAIN)
+    short pull;           // the k-th live tile whose round pulls
+    unsigned char flags;  // by live tile: scatter flags (SF_*)
+    unsigned char idle;   // by the group's j-th slot: 1 if it was idle at the round start
 };
 
+struct RoundSh {
+    int ntl;              // live tiles this round
+    int any_check;        // some live tile needs a CHECK phase
+    int any_idle;         // served solves: some slot awaits a query
+    int ndrain;           // online: slots to clear
+    int npull;            // live tiles whose round pulls
+};
+
+extern __shared__ __align__(16) unsigned char dyn_smem[];
+__device__ __forceinline__ TileSlot* tile_slots() { return reinterpret_cast<TileSlot*>(dyn_smem); }
+
 enum : unsigned char {
-    SF_FINAL = 1, SF_TRACK = 2, SF_NOPUSH = 4, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32, SF_PULL = 64
+    SF_FINAL = 1, SF_TRACK = 2, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32
 };
 
 // Local GD for PPR and Katz only ever adds non-negative values to
@@ -479,47 +487,38 @@ __device__ __forceinline__ uint32_t* tile_bits(const PushArgs& a, int t, int par
     return a.bits + ((int64_t)t * 2 + par) * a.bit_words;
 }
 
-// Exclusive prefix over vals[0..m) (m <= 512) written to out[0..m]; block-wide.
-__device__ void block_exclusive_scan(const long long* vals, int m, long long* out, long long* tmp) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    long long v0 = (2 * tid < m) ? vals[2 * tid] : 0;
-    long long v1 = (2 * tid + 1 < m) ? vals[2 * tid + 1] : 0;
-    long long s = v0 + v1;
-    long long inc = s;
+// Exclusive prefix sums of val(0..m-1) into tile_slots()[0..m].off[w], by one warp.
+template <typename F>
+__device__ __forceinline__ void warp_offsets(int w, int m, F val) {
+    const int lane = threadIdx.x & 31;
+    TileSlot* sl = tile_slots();
+    long long carry = 0;
+    for (int k0 = 0; k0 < m; k0 += 32) {
+        const int k = k0 + lane;
+        const long long v = k < m ? val(k) : 0;
+        long long inc = v;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        long long y = __shfl_up_sync(kFull, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) tmp[warp] = inc;
-    __syncthreads();
-    if (tid == 0) {
-        long long acc = 0;
-        for (int w = 0; w < kWarps; ++w) {
-            long long c = tmp[w];
-            tmp[w] = acc;
-            acc += c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long y = __shfl_up_sync(kFull, inc, o);
+            if (lane >= o) inc += y;
         }
-        out[m] = acc;
+        if (k < m) sl[k].off[w] = carry + inc - v;
+        carry += __shfl_sync(kFull, inc, 31);
     }
-    __syncthreads();
-    long long excl = tmp[warp] + inc - s;
-    if (2 * tid < m) out[2 * tid] = excl;
-    if (2 * tid + 1 < m) out[2 * tid + 1] = excl + v0;
-    __syncthreads();
+    if (lane == 0) sl[m].off[w] = carry;
 }
 
 // First live-tile index k with off[k+1] > x (off ascending, off[0] = 0).
-__device__ __forceinline__ int find_tile(const long long* off, int ntl, long long x) {
+__device__ __forceinline__ int find_tile(int w, int ntl, long long x) {
+    const TileSlot* sl = tile_slots();
     int lo = 0, hi = ntl - 1;
     while (lo < hi) {
         int mid = (lo + hi) >> 1;
-        if (off[mid + 1] > x) hi = mid;
+        if (sl[mid + 1].off[w] > x) hi = mid;
         else lo = mid + 1;
     }
     return lo;
 }
-
 
 // The block group this block belongs to (served launches with a.groups > 1
 // split the grid; every other launch is one group): group g holds blocks
@@ -2143,10 +2142,9 @@ __device__ __forceinline__ void pull_chunk(const PushArgs& a, const ScatterCtx<T
     pull_flush<T, W, A>(a, c, grp_w == 0, len > kPullChunk, v, c0, lane_g, grp_w, acc, theta, theta_f);
 }
 
-// Every row of the npull live tiles in `list` (indices into rs.tiles).
+// Every row of the npull live tiles named by tile_slots()[0..npull).pull.
 template <typename T, int W>
-__device__ __noinline__ void pull_phase(const PushArgs& a, const RoundSh& rs, const short* list, int npull,
-                                        const GroupInfo& gi) {
+__device__ __noinline__ void pull_phase(const PushArgs& a, int npull, const GroupInfo& gi) {
     constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
     constexpr int GPW = 32 / (W / VEC);
     constexpr int MS = GPW >= 4 ? GPW / 4 : 1;  // lane groups per middle row
@@ -2158,10 +2156,10 @@ __device__ __noinline__ void pull_phase(const PushArgs& a, const RoundSh& rs, co
     const unsigned nw = (unsigned)gi.dim * kWarps;
     unsigned u = (unsigned)gi.blk * kWarps + (threadIdx.x >> 5);
     for (int p = 0; p < npull; ++p) {
-        const int k = list[p];
-        const int t = rs.tiles[k];
-        const uint32_t* bits = tile_bits(a, t, rs.level[k] & 1);
-        const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, rs.level[k], rs.flags[k]);
+        const TileSlot& s = tile_slots()[tile_slots()[p].pull];
+        const int t = s.tile;
+        const uint32_t* bits = tile_bits(a, t, s.level & 1);
+        const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, s.level, s.flags);
         for (; u < units; u += nw) {
             if (u < u_long) {
                 const int2 ch = g.pchunk[u];
@@ -2213,11 +2211,11 @@ __device__ __forceinline__ bool hk_end_level(const TileParams& tp, int level) {
 
 // Column part of the bookkeeping: one thread per (live tile, column).
 template <int W>
-__device__ void finish_columns_all(const PushArgs& a, const RoundSh& rs, int ntl) {
+__device__ void finish_columns_all(const PushArgs& a, int ntl) {
     for (int idx = threadIdx.x; idx < ntl * W; idx += kThreads) {
         const int k = idx / W, c = idx % W;
-        const int t = rs.tiles[k];
-        const int level = rs.level[k];
+        const int t = tile_slots()[k].tile;
+        const int level = tile_slots()[k].level;
         const TileParams& tp = a.tp[t];
         if (c >= tp.ncols) continue;
         const int m = tp.method;
@@ -2923,13 +2921,14 @@ template <typename T, int W, bool PULL>
 __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_MIN_BLOCKS_W1
                                            : (W <= 8 && sizeof(T) == 4) ? GDE_MIN_BLOCKS_F32
                                                                         : GDE_MIN_BLOCKS)
-    push_kernel(PushArgs a) {
+    push_kernel(const __grid_constant__ PushArgs a) {
     __shared__ TileSh sh;
     __shared__ PrepSh ps;
     __shared__ RoundSh rs;
     __shared__ int s_cnt[kMaxW];
-    __shared__ long long s_vals[kMaxLaunchTiles];
+    TileSlot* const sl = tile_slots();
     const int64_t n = a.g.n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (blockIdx.x == 0 && threadIdx.x == 0) a.stats->start_ns = globaltimer_ns();
     if (threadIdx.x == 0) {
         ps.acc_col_nodes = 0; ps.acc_union_nodes = 0;
@@ -2944,46 +2943,54 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
     const bool online = a.serve && a.queue.online;
     const GroupInfo gi = group_of(a);
     const int G = a.groups > 1 ? a.groups : 1;
+    const int own = (a.ntiles - gi.id + G - 1) / G;  // this group's tiles
     if (online && blockIdx.x == 0 && threadIdx.x == 0) *a.queue.last_ns = globaltimer_ns();
     for (; it < a.round_budget; ++it) {
         // online server: group 0 decided to stop (stop flag, or idle), and this
         // group took its copy of the decision before last round's barrier
         if (online && ld_volatile_i(a.queue.gquit + gi.id) != 0) break;
         trace_point(a, it, TP_ITER);
-        // ---- live tiles of this round (identical in every block) ----
-        if (threadIdx.x == 0) { rs.any_check = 0; rs.any_idle = 0; rs.ndrain = 0; }
-        __syncthreads();
-        for (int t = threadIdx.x; t < a.ntiles; t += kThreads) {
-            const TileState& ts = a.ts[t];
-            const bool mine = (t % G) == gi.id;  // this group's slots
-            const bool live = mine && ts.done == SLOT_LIVE && it >= ts.t0 && (it - ts.t0) < a.max_rounds;
-            s_vals[t] = live ? 1 : 0;
-            rs.idle[t] = !mine ? 0 : (ts.done == SLOT_IDLE) ? 1 : (ts.done == SLOT_DRAIN ? 2 : 0);
-            if (mine && ts.done == SLOT_IDLE) rs.any_idle = 1;
-        }
-        if (online) {
-            // drained slots in ascending order: the same list in every block
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int nd = 0;
-                for (int t = 0; t < a.ntiles; ++t)
-                    if (rs.idle[t] == 2) rs.drain[nd++] = (short)t;
+        // ---- live tiles of this round, and PREP's spaces (identical in every
+        // block): the first warp reads the group's tiles t = id + j G ----
+        if (warp == 0) {
+            int nl = 0, nd = 0;
+            bool check = false, idle = false;
+            for (int j0 = 0; j0 < own; j0 += 32) {
+                const int j = j0 + lane, t = gi.id + j * G;
+                const bool in = j < own;
+                const int done = in ? a.ts[t].done : SLOT_EMPTY;
+                const int lv = in ? it - a.ts[t].t0 : 0;
+                const bool live = in && done == SLOT_LIVE && lv >= 0 && lv < a.max_rounds;
+                const unsigned bl = __ballot_sync(kFull, live), below = (1u << lane) - 1u;
+                if (live) {
+                    TileSlot& s = sl[nl + __popc(bl & below)];
+                    s.tile = t;
+                    s.level = lv;
+                    const int m = a.tp[t].method;
+                    check |= m == M_GLOBAL_GD || m == M_GLOBAL_CHEBY || (m == M_HK_GLOBAL && hk_relaxed(a.tp[t]));
+                }
+                nl += __popc(bl);
+                if (in) sl[j].idle = done == SLOT_IDLE;
+                idle |= in && done == SLOT_IDLE;
+                const bool dr = online && in && done == SLOT_DRAIN;
+                const unsigned bd = __ballot_sync(kFull, dr);
+                if (dr) sl[nd + __popc(bd & below)].drain = (short)t;
+                nd += __popc(bd);
+            }
+            check = __any_sync(kFull, check);
+            idle = __any_sync(kFull, idle);
+            __syncwarp();
+            warp_offsets(0, nl, [&](int k) -> long long {
+                const TileState& ts = a.ts[sl[k].tile];
+                return ts.dense_next[sl[k].level & 1] ? n : ts.cand_cnt[sl[k].level % 3];
+            });
+            if (lane == 0) {
+                rs.ntl = nl;
                 rs.ndrain = nd;
+                rs.any_check = check;
+                rs.any_idle = idle;
             }
         }
-        __syncthreads();
-        block_exclusive_scan(s_vals, a.ntiles, rs.off[0], rs.scan_tmp);
-        for (int t = threadIdx.x; t < a.ntiles; t += kThreads) {
-            if (rs.off[0][t + 1] != rs.off[0][t]) {
-                const int k = (int)rs.off[0][t];
-                rs.tiles[k] = t;
-                rs.level[k] = it - a.ts[t].t0;
-                const int m = a.tp[t].method;
-                if (m == M_GLOBAL_GD || m == M_GLOBAL_CHEBY || (m == M_HK_GLOBAL && hk_relaxed(a.tp[t])))
-                    rs.any_check = 1;
-            }
-        }
-        if (threadIdx.x == 0) rs.ntl = (int)rs.off[0][a.ntiles];
         __syncthreads();
         const int ntl = rs.ntl;
         if (ntl == 0 && !rs.any_idle && rs.ndrain == 0) break;
@@ -2992,7 +2999,7 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         // ---- CHECK (global GD / Chebyshev tiles) ----
         if (rs.any_check) {
             for (int k = 0; k < ntl; ++k) {
-                const int t = rs.tiles[k];
+                const int t = sl[k].tile;
                 const int m = a.tp[t].method;
                 if constexpr (sizeof(T) == 8)
                     if (m == M_HK_GLOBAL && hk_relaxed(a.tp[t])) hk_sweeps_phase<T, W>(a, t, it);
@@ -3008,26 +3015,19 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         }
         // ---- PREP: flattened candidates of all live tiles ----
         if (gi.blk == 0) {
-            for (int k = 0; k < ntl; ++k) zero_next_counters<W>(a, rs.tiles[k], rs.level[k]);
+            for (int k = 0; k < ntl; ++k) zero_next_counters<W>(a, sl[k].tile, sl[k].level);
         }
-        for (int k = threadIdx.x; k < ntl; k += kThreads) {
-            const TileState& ts = a.ts[rs.tiles[k]];
-            const int lv = rs.level[k];
-            s_vals[k] = ts.dense_next[lv & 1] ? n : ts.cand_cnt[lv % 3];
-        }
-        __syncthreads();
-        block_exclusive_scan(s_vals, ntl, rs.off[0], rs.scan_tmp);
         trace_point(a, it, TP_PREP_WORK);
         {
             long long lo, hi;
-            block_share(rs.off[0][ntl], lo, hi, gi);
+            block_share(sl[ntl].off[0], lo, hi, gi);
             if (lo < hi) {
-                for (int k = find_tile(rs.off[0], ntl, lo); k < ntl && rs.off[0][k] < hi; ++k) {
-                    const long long b = max(lo, rs.off[0][k]) - rs.off[0][k];
-                    const long long e = min(hi, rs.off[0][k + 1]) - rs.off[0][k];
+                for (int k = find_tile(0, ntl, lo); k < ntl && sl[k].off[0] < hi; ++k) {
+                    const long long b = max(lo, sl[k].off[0]) - sl[k].off[0];
+                    const long long e = min(hi, sl[k + 1].off[0]) - sl[k].off[0];
                     if (b >= e) continue;
-                    load_tile<W>(a, rs.tiles[k], it, sh);
-                    prep_range<T, W, PULL>(a, rs.tiles[k], sh, ps, b, e);
+                    load_tile<W>(a, sl[k].tile, it, sh);
+                    prep_range<T, W, PULL>(a, sl[k].tile, sh, ps, b, e);
                 }
             }
         }
@@ -3040,63 +3040,72 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             t0 = t1;
         }
         // ---- SCATTER: flattened short rows / medium rows / long-row chunks ----
-        for (int k = threadIdx.x; k < ntl; k += kThreads) {
-            const int t = rs.tiles[k];
-            const TileState& ts = a.ts[t];
-            const TileParams& tp = a.tp[t];
-            const int lv = rs.level[k];
-            const int par = lv & 1;
-            const int m = tp.method;
-            const bool hk = method_is_hk(m);
-            const bool fin = hk && (m != M_HK_TAYLOR) && (lv + 1 == tp.n_levels);
-            const bool last_taylor = (m == M_HK_TAYLOR) && (lv >= tp.n_levels);
-            const bool dnext = dense_next_round(a, tp, ts, par);
-            unsigned char f = 0;
-            if (hk) f |= SF_HK;
-            if (fin) f |= SF_FINAL;
-            if (last_taylor) f |= SF_NOPUSH;
-            if (tp.kind == KIND_IGN) f |= SF_TGTSCALE;
-            if (tile_crosses(tp)) f |= SF_CROSS;
-            else if (!dnext && !fin && !last_taylor) f |= SF_TRACK;
-            if (ts.pull[par] && ts.front_cnt[par] > 0 && !last_taylor) f |= SF_PULL;
-            rs.flags[k] = f;
-            const bool has = ts.front_cnt[par] > 0 && !last_taylor;
-            s_vals[k] = has ? ts.small_cnt[par] : 0;
+        // a warp per space: short rows, medium rows, long-row chunks, retiring
+        // slots' nodes; another one the flags and the tiles that pull
+        {
+            auto pushes = [&](int k) {
+                const int t = sl[k].tile, lv = sl[k].level;
+                return a.ts[t].front_cnt[lv & 1] > 0 &&
+                       !(a.tp[t].method == M_HK_TAYLOR && lv >= a.tp[t].n_levels);
+            };
+            if (warp == 0)
+                warp_offsets(0, ntl, [&](int k) -> long long {
+                    return pushes(k) ? a.ts[sl[k].tile].small_cnt[sl[k].level & 1] : 0;
+                });
+            else if (warp == 1)
+                warp_offsets(1, ntl, [&](int k) -> long long {
+                    return pushes(k) ? a.ts[sl[k].tile].med_cnt[sl[k].level & 1] : 0;
+                });
+            else if (warp == 2)
+                warp_offsets(2, ntl, [&](int k) -> long long {
+                    return pushes(k) ? a.ts[sl[k].tile].large_cnt[sl[k].level & 1] : 0;
+                });
+            else if (warp == 3 && a.serve)
+                warp_offsets(3, ntl, [&](int k) -> long long {
+                    return a.ts[sl[k].tile].front_cnt[sl[k].level & 1] == 0 ? n : 0;
+                });
+            else if (warp == 4) {
+                int np = 0;
+                for (int k0 = 0; k0 < ntl; k0 += 32) {
+                    const int k = k0 + lane;
+                    bool pull = false;
+                    if (k < ntl) {
+                        const int t = sl[k].tile, lv = sl[k].level, par = lv & 1;
+                        const TileState& ts = a.ts[t];
+                        const TileParams& tp = a.tp[t];
+                        const int m = tp.method;
+                        const bool hk = method_is_hk(m);
+                        const bool fin = hk && (m != M_HK_TAYLOR) && (lv + 1 == tp.n_levels);
+                        const bool last_taylor = (m == M_HK_TAYLOR) && (lv >= tp.n_levels);
+                        unsigned char f = 0;
+                        if (hk) f |= SF_HK;
+                        if (fin) f |= SF_FINAL;
+                        if (tp.kind == KIND_IGN) f |= SF_TGTSCALE;
+                        if (tile_crosses(tp)) f |= SF_CROSS;
+                        else if (!dense_next_round(a, tp, ts, par) && !fin && !last_taylor) f |= SF_TRACK;
+                        sl[k].flags = f;
+                        pull = PULL && ts.pull[par] && ts.front_cnt[par] > 0 && !last_taylor;
+                    }
+                    const unsigned b = __ballot_sync(kFull, pull);
+                    if (pull) sl[np + __popc(b & ((1u << lane) - 1u))].pull = (short)k;
+                    np += __popc(b);
+                }
+                if (lane == 0) rs.npull = np;
+            }
         }
         __syncthreads();
-        block_exclusive_scan(s_vals, ntl, rs.off[0], rs.scan_tmp);
-        for (int k = threadIdx.x; k < ntl; k += kThreads) {
-            const TileState& ts = a.ts[rs.tiles[k]];
-            const int par = rs.level[k] & 1;
-            s_vals[k] = (ts.front_cnt[par] > 0 && !(rs.flags[k] & SF_NOPUSH)) ? ts.med_cnt[par] : 0;
-        }
-        __syncthreads();
-        block_exclusive_scan(s_vals, ntl, rs.off[1], rs.scan_tmp);
-        for (int k = threadIdx.x; k < ntl; k += kThreads) {
-            const TileState& ts = a.ts[rs.tiles[k]];
-            const int par = rs.level[k] & 1;
-            s_vals[k] = (ts.front_cnt[par] > 0 && !(rs.flags[k] & SF_NOPUSH)) ? ts.large_cnt[par] : 0;
-        }
-        __syncthreads();
-        block_exclusive_scan(s_vals, ntl, rs.off[2], rs.scan_tmp);
         if (a.serve) {
             // slots whose query finished this round: extract + clear, every
             // block an equal share of the retiring slots' nodes
-            for (int k = threadIdx.x; k < ntl; k += kThreads) {
-                const TileState& ts = a.ts[rs.tiles[k]];
-                s_vals[k] = (ts.front_cnt[rs.level[k] & 1] == 0) ? n : 0;
-            }
-            __syncthreads();
-            block_exclusive_scan(s_vals, ntl, rs.off[3], rs.scan_tmp);
             long long lo, hi;
-            block_share(rs.off[3][ntl], lo, hi, gi);
+            block_share(sl[ntl].off[3], lo, hi, gi);
             if (lo < hi) {
-                for (int k = find_tile(rs.off[3], ntl, lo); k < ntl && rs.off[3][k] < hi; ++k) {
-                    const long long b = max(lo, rs.off[3][k]) - rs.off[3][k];
-                    const long long e = min(hi, rs.off[3][k + 1]) - rs.off[3][k];
+                for (int k = find_tile(3, ntl, lo); k < ntl && sl[k].off[3] < hi; ++k) {
+                    const long long b = max(lo, sl[k].off[3]) - sl[k].off[3];
+                    const long long e = min(hi, sl[k + 1].off[3]) - sl[k].off[3];
                     if (b >= e) continue;
-                    if (online) gather_online_range<T, W>(a, rs.tiles[k], b, e);
-                    else retire_range<T, W>(a, rs.tiles[k], b, e);
+                    if (online) gather_online_range<T, W>(a, sl[k].tile, b, e);
+                    else retire_range<T, W>(a, sl[k].tile, b, e);
                 }
             }
             // online slots drained last round: every block of the group an equal share of their nodes
@@ -3105,7 +3114,7 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
                 for (long long x = lo; x < hi;) {
                     const long long k = x / n;
                     const long long e = min(hi, (k + 1) * n);
-                    clear_slot_range<T, W>(a, rs.drain[k], x - k * n, e - k * n);
+                    clear_slot_range<T, W>(a, sl[k].drain, x - k * n, e - k * n);
                     x = e;
                 }
             }
@@ -3113,16 +3122,15 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         trace_point(a, it, TP_SCAT_WORK);
         // long-row chunks first (largest pieces), then medium, then short rows
         for (int sp = 2; sp >= 0; --sp) {
-            const long long* off = rs.off[sp];
             long long lo, hi;
-            block_share(off[ntl], lo, hi, gi);
+            block_share(sl[ntl].off[sp], lo, hi, gi);
             if (lo >= hi) continue;
-            for (int k = find_tile(off, ntl, lo); k < ntl && off[k] < hi; ++k) {
-                const long long b = max(lo, off[k]) - off[k];
-                const long long e = min(hi, off[k + 1]) - off[k];
+            for (int k = find_tile(sp, ntl, lo); k < ntl && sl[k].off[sp] < hi; ++k) {
+                const long long b = max(lo, sl[k].off[sp]) - sl[k].off[sp];
+                const long long e = min(hi, sl[k + 1].off[sp]) - sl[k].off[sp];
                 if (b >= e) continue;
-                const int t = rs.tiles[k];
-                const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, rs.level[k], rs.flags[k]);
+                const int t = sl[k].tile;
+                const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, sl[k].level, sl[k].flags);
                 if constexpr (W == 1) {
                     if (sp == 2) scatter_warp_items_w1<T>(a, a.blarge + (int64_t)t * a.large_cap, 1, c, b, e);
                     else if (sp == 1) scatter_warp_items_w1<T>(a, a.bsmall + (int64_t)t * n + (n - 1), -1, c, b, e);
@@ -3136,24 +3144,12 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         }
         // tiles whose round pulls have no work items above
         if (PULL && a.pull_div > 0) {
-            if (threadIdx.x < 32) {
-                int np = 0;
-                for (int k0 = 0; k0 < ntl; k0 += 32) {
-                    const int k = k0 + threadIdx.x;
-                    const bool p = k < ntl && (rs.flags[k] & SF_PULL);
-                    const unsigned b = __ballot_sync(kFull, p);
-                    if (p) rs.pull[np + __popc(b & ((1u << threadIdx.x) - 1u))] = (short)k;
-                    np += __popc(b);
-                }
-                if (threadIdx.x == 0) rs.npull = np;
-            }
-            __syncthreads();
             if constexpr (PULL)
-                if (rs.npull > 0) pull_phase<T, W>(a, rs, rs.pull, rs.npull, gi);
+                if (rs.npull > 0) pull_phase<T, W>(a, rs.npull, gi);
             // a clear bitmap for each tile whose next round pulls
             for (int k = 0; k < ntl; ++k) {
-                const int t = rs.tiles[k];
-                const int par = rs.level[k] & 1;
+                const int t = sl[k].tile;
+                const int par = sl[k].level & 1;
                 if (!pull_next_round(a, a.ts[t], par)) continue;
                 uint32_t* b = tile_bits(a, t, par ^ 1);
                 for (int64_t w = (int64_t)gi.blk * kThreads + threadIdx.x; w < a.bit_words;
@@ -3164,9 +3160,9 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         trace_point(a, it, TP_SCAT_DONE);
         // HK level drop (touches the current level's slab only)
         for (int k = 0; k < ntl; ++k) {
-            if (!(rs.flags[k] & SF_HK)) continue;
-            const int t = rs.tiles[k];
-            const int lv = rs.level[k];
+            if (!(sl[k].flags & SF_HK)) continue;
+            const int t = sl[k].tile;
+            const int lv = sl[k].level;
             const TileState& ts = a.ts[t];
             if (ts.front_cnt[lv & 1] == 0) continue;
             hk_drop<T, W>(a, t, lv, ts.dense_next[lv & 1] != 0, ts.cand_cnt[lv % 3], gi);
@@ -3175,31 +3171,31 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
         if (gi.blk == 0 && online) {
             if (threadIdx.x == 0) {
                 for (int k = 0; k < rs.ndrain; ++k) {
-                    publish_online(a, rs.drain[k]);
-                    a.ts[rs.drain[k]].done = SLOT_IDLE;  // admitted from the next round on
+                    publish_online(a, sl[k].drain);
+                    a.ts[sl[k].drain].done = SLOT_IDLE;  // admitted from the next round on
                 }
                 if (gi.id == 0 && route_online(a)) admitted = true;
                 if (rs.any_idle)
-                    for (int t = 0; t < a.ntiles; ++t)
-                        if (rs.idle[t] == 1 && admit_online<T, W>(a, t, it)) admitted = true;
+                    for (int j = 0; j < own; ++j)
+                        if (sl[j].idle && admit_online<T, W>(a, gi.id + j * G, it)) admitted = true;
             }
         } else if (gi.blk == 0 && a.serve && rs.any_idle) {
-            for (int t = 0; t < a.ntiles; ++t)
-                if (rs.idle[t] == 1) admit_query<T, W>(a, t, it);
+            for (int j = 0; j < own; ++j)
+                if (sl[j].idle) admit_query<T, W>(a, gi.id + j * G, it);
         }
         if (gi.blk == 0) {
-            finish_columns_all<W>(a, rs, ntl);
+            finish_columns_all<W>(a, ntl);
             __syncthreads();
             for (int k = threadIdx.x; k < ntl; k += kThreads) {
-                const int t = rs.tiles[k];
-                const int lv = rs.level[k];
+                const int t = sl[k].tile;
+                const int lv = sl[k].level;
                 const bool dnext = dense_next_round(a, a.tp[t], a.ts[t], lv & 1);
                 finish_round<W>(a, t, lv, dnext);
             }
             if (online && threadIdx.x == 0) {
                 // a slot that reaches max_rounds ends with GDE_EITERCAP (its row is not written)
                 for (int k = 0; k < ntl; ++k) {
-                    const int t = rs.tiles[k];
+                    const int t = sl[k].tile;
                     TileState& ts = a.ts[t];
                     if (ts.done == SLOT_LIVE && it + 1 - ts.t0 >= a.max_rounds) {
                         OnlineSlot& os = a.queue.slot[t];
@@ -3247,28 +3243,34 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
 
 // Host-side launcher: picks the instantiation for (T, W, PULL) and launches
 // it cooperatively with the largest co-resident grid.
+static size_t tiles_smem(int ntiles, int groups) {
+    const int G = groups > 1 ? groups : 1;
+    return (size_t)((ntiles + G - 1) / G + 1) * sizeof(TileSlot);
+}
+
 template <typename T, int W, bool PULL>
-static int max_grid_t(int sms) {
+static int max_grid_t(int sms, size_t smem) {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, push_kernel<T, W, PULL>, kThreads, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, push_kernel<T, W, PULL>, kThreads, smem);
     return per_sm * sms;
 }
 
 template <typename T, int W, bool PULL>
 static cudaError_t launch_t(const PushArgs& a, int grid, cudaStream_t st) {
     void* args[] = {const_cast<PushArgs*>(&a)};
-    return cudaLaunchCooperativeKernel((void*)push_kernel<T, W, PULL>, dim3(grid), dim3(kThreads), args, 0, st);
+    return cudaLaunchCooperativeKernel((void*)push_kernel<T, W, PULL>, dim3(grid), dim3(kThreads), args,
+                                       tiles_smem(a.ntiles, a.groups), st);
 }
 
 template <typename T>
-static int max_grid_w(int W, bool pull, int sms) {
+static int max_grid_w(int W, bool pull, int sms, size_t smem) {
     switch (W) {
-        case 1: return pull ? max_grid_t<T, 1, true>(sms) : max_grid_t<T, 1, false>(sms);
-        case 2: return max_grid_t<T, 2, true>(sms);
-        case 4: return max_grid_t<T, 4, true>(sms);
-        case 8: return max_grid_t<T, 8, true>(sms);
-        case 16: return max_grid_t<T, 16, true>(sms);
-        case 32: return max_grid_t<T, 32, true>(sms);
+        case 1: return pull ? max_grid_t<T, 1, true>(sms, smem) : max_grid_t<T, 1, false>(sms, smem);
+        case 2: return max_grid_t<T, 2, true>(sms, smem);
+        case 4: return max_grid_t<T, 4, true>(sms, smem);
+        case 8: return max_grid_t<T, 8, true>(sms, smem);
+        case 16: return max_grid_t<T, 16, true>(sms, smem);
+        case 32: return max_grid_t<T, 32, true>(sms, smem);
     }
     return 0;
 }
@@ -3286,8 +3288,9 @@ static cudaError_t launch_w(const PushArgs& a, int W, int grid, cudaStream_t st)
     return cudaErrorInvalidValue;
 }
 
-int engine_max_grid(int prec64, int W, bool pull, int sms) {
-    return prec64 ? max_grid_w<double>(W, pull, sms) : max_grid_w<float>(W, pull, sms);
+int engine_max_grid(const PushArgs& a, int prec64, int W, int sms) {
+    const size_t smem = tiles_smem(a.ntiles, a.groups);
+    return prec64 ? max_grid_w<double>(W, a.pull_div > 0, sms, smem) : max_grid_w<float>(W, a.pull_div > 0, sms, smem);
 }
 
 cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st) {

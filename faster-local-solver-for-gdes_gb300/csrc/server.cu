@@ -276,13 +276,6 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
     CK_S(cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking));
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device);
-    s->grid = engine_max_grid(s->prec64, 1, false, sms);
-    if (s->grid <= 0) {
-        int rc = s->fail(GDE_ECUDA, "push kernel does not fit on the device");
-        s->free_all();
-        delete s;
-        return rc;
-    }
     // ---- device workspace: S one-column slots ----
     PushArgs& a = s->a;
     a = base;
@@ -313,8 +306,18 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
     // every group.
     {
         const int g_default = s->hk ? std::max(1, S / 8) : S;
-        a.groups = std::max(1, std::min(std::min(p->groups > 0 ? p->groups : g_default, S),
-                                        std::min(kMaxGroups, s->grid)));
+        a.groups = std::max(1, std::min(std::min(p->groups > 0 ? p->groups : g_default, S), kMaxGroups));
+        s->grid = engine_max_grid(a, s->prec64, 1, sms);
+        if (a.groups > s->grid && s->grid > 0) {
+            a.groups = s->grid;
+            s->grid = std::min(s->grid, engine_max_grid(a, s->prec64, 1, sms));
+        }
+        if (s->grid <= 0) {
+            int rc = s->fail(GDE_ECUDA, "push kernel does not fit on the device");
+            s->free_all();
+            delete s;
+            return rc;
+        }
     }
     a.bar = (GridBarrier*)s->dalloc((size_t)a.groups * sizeof(GridBarrier));
     a.err = (int*)s->dalloc(sizeof(int));
