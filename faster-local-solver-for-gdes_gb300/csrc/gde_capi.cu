@@ -105,6 +105,8 @@ void fill_tuning(const gde_params* p, PushArgs& a) {
     a.med_max = p->med_max > 0 ? p->med_max : d.med_max;
     if (a.med_max < a.small_max) a.med_max = a.small_max;
     a.chunk = p->chunk > 0 ? p->chunk : d.chunk;
+    // a one-column work item holds a length of up to 24 bits
+    for (int* m : {&a.small_max, &a.med_max, &a.chunk}) *m = std::min(*m, (1 << 24) - 1);
     a.dense_div = p->dense_div > 0 ? p->dense_div : d.dense_div;
     a.max_rounds = p->max_rounds > 0 ? p->max_rounds : kDefaultMaxRounds;
     a.allow_dense = 1;

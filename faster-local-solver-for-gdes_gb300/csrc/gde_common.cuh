@@ -292,18 +292,16 @@ struct LaunchStats {          // roofline counters summed over a launch
     unsigned long long sp_ovf;         // ... handed to the dense slots
 };
 
-// Arrival counter and generation word on separate 128-byte lines: waiting
-// blocks poll `gen` without slowing the arrivals on `count`.
+// Arrivals so far, on a 128-byte line of its own.
 struct GridBarrier {
-    unsigned int count;
-    unsigned int pad0[31];
-    unsigned int gen;
-    unsigned int pad1[31];
+    unsigned long long count;
+    unsigned long long pad[15];
 };
 
 // A piece of push work: `len` edges of one frontier row starting at col[rp]
 // (a whole short/medium row, or one chunk of a long row), and the row's
-// frontier index (its push values are P[fidx][0..W)).
+// frontier index (its push values are P[fidx][0..W)).  One-column tiles pack
+// start, length and push value into the same 16 bytes instead (pack_item).
 struct PushItem {
     long long rp;
     int len;

@@ -9,12 +9,11 @@ namespace gde {
 constexpr unsigned long long kSpinLimit = 1ull << 26;  // ~ seconds of polling
 
 // ---------------------------------------------------------------------------
-// Bounded grid barrier (sense by generation counter).  Co-residency of all
+// Bounded grid barrier (a counter of arrivals).  Co-residency of all
 // blocks is guaranteed by the cooperative launch; the spin limit only guards
 // against a bug turning into a hang: on expiry the block records GDE_EHANG
 // and every block leaves its loop at the next barrier.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned ld_volatile(const unsigned* p) { return *(volatile const unsigned*)p; }
 __device__ __forceinline__ int ld_volatile_i(const int* p) { return *(volatile const int*)p; }
 // A load that later loads of this thread cannot pass (device-scope acquire).
 __device__ __forceinline__ int ld_acquire_gpu_i(const int* p) {
@@ -23,8 +22,23 @@ __device__ __forceinline__ int ld_acquire_gpu_i(const int* p) {
     return v;
 }
 
+__device__ __forceinline__ unsigned long long ld_acquire_gpu_u64(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long add_release_gpu_u64(unsigned long long* p, unsigned long long x) {
+    unsigned long long v;
+    asm volatile("atom.add.release.gpu.u64 %0, [%1], %2;" : "=l"(v) : "l"(p), "l"(x) : "memory");
+    return v;
+}
+
 // `limit` polls (0: kSpinLimit) before a waiting block gives up; `members`
-// blocks meet at `bar` (0: the whole grid).
+// blocks meet at `bar` (0: the whole grid).  Arrivals only count up, so a
+// block knows from its own ticket the count that completes its phase and
+// polls for it: one release, one round trip for the ticket and one for the
+// last arrival, with no second word to reset and publish (2.8 us of a round's
+// ~23 on a small graph before, twice a round).
 __device__ __forceinline__ bool grid_barrier(GridBarrier* bar, int* err, unsigned long long limit = 0,
                                              unsigned members = 0) {
     if (limit == 0) limit = kSpinLimit;
@@ -33,29 +47,26 @@ __device__ __forceinline__ bool grid_barrier(GridBarrier* bar, int* err, unsigne
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
-        unsigned gen = ld_volatile(&bar->gen);
-        __threadfence();
-        unsigned arrived = atomicAdd(&bar->count, 1u);
-        if (arrived == members - 1) {
-            atomicExch(&bar->count, 0u);
-            __threadfence();
-            atomicAdd(&bar->gen, 1u);
-        } else {
-            unsigned long long spins = 0;
-            while (ld_volatile(&bar->gen) == gen) {
-                if (ld_volatile_i(err) != 0) { ok = 0; break; }
-                if (++spins > limit) { atomicCAS(err, 0, GDE_EHANG); ok = 0; break; }
-                __nanosleep(100);
+        const unsigned long long ticket = add_release_gpu_u64(&bar->count, 1ull);
+        const unsigned long long target = (ticket / members + 1) * members;
+        unsigned long long spins = 0;
+        for (;;) {
+            const int e = ld_volatile_i(err);  // in flight with the count
+            const bool all = ld_acquire_gpu_u64(&bar->count) >= target;
+            if (e != 0) ok = 0;
+            if (all || e != 0) break;
+            if (++spins > limit) {
+                atomicCAS(err, 0, GDE_EHANG);
+                ok = 0;
+                break;
             }
+            __nanosleep(32);
         }
-        __threadfence();
-        if (ld_volatile_i(err) != 0) ok = 0;
         s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;
 }
-
 
 // Device-wide nanosecond clock (PTX %globaltimer).
 __device__ __forceinline__ unsigned long long globaltimer_ns() {

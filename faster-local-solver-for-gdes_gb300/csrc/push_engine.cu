@@ -434,12 +434,13 @@ __device__ void check_phase(const PushArgs& a, int t, int it, int* s_cnt) {
 // took 2.31 -> 2.17 ms with both, and the kernel's parameters in constant
 // memory instead of a stack copy for the out-of-line calls.
 struct TileSlot {
-    long long off[4];     // by live tile: exclusive prefix sums of the current phase's spaces
+    long long off[2];     // by live tile: exclusive prefix sums of the current phase's spaces
     int tile;             // by live tile: its id (ascending)
     int level;            //               rounds since its start
     short drain;          // online: the k-th slot to clear this round (SLOT_DRAIN)
     short pull;           // the k-th live tile whose round pulls
     unsigned char flags;  // by live tile: scatter flags (SF_*)
+    unsigned char split;  //               1: its row items are cut into pieces (scatter_units)
     unsigned char idle;   // by the group's j-th slot: 1 if it was idle at the round start
 };
 
@@ -520,6 +521,19 @@ __device__ __forceinline__ int find_tile(int w, int ntl, long long x) {
     return lo;
 }
 
+// Short rows of one unit of scatter work: one per lane group of a warp.
+template <typename T, int W>
+constexpr int short_rows() {
+    return 32 / (W / ((sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1)));
+}
+
+// Edges of a piece of a chunk or medium row, when a round has fewer units of
+// scatter work than warps: a few iterations instead of a whole item's.
+template <typename T, int W>
+constexpr int piece_edges() {
+    return W == 1 ? 64 : 4 * short_rows<T, W>();
+}
+
 // The block group this block belongs to (served launches with a.groups > 1
 // split the grid; every other launch is one group): group g holds blocks
 // [ceil(g B / G), ceil((g+1) B / G)).
@@ -537,7 +551,14 @@ __device__ __forceinline__ GroupInfo group_of(const PushArgs& a) {
     return GroupInfo{g, (int)blockIdx.x - start, end - start};
 }
 
-// This block's share [lo, hi) of a flattened space of `total` items (its group's blocks split it).
+template <typename T, int W>
+__device__ __forceinline__ int pieces(int edges) {
+    return (edges + piece_edges<T, W>() - 1) / piece_edges<T, W>();
+}
+
+// This block's share [lo, hi) of a flattened space of `total` items (its
+// group's blocks split it evenly, however few there are: keeping 32 or 64
+// candidates together for one warp measured 10% slower on small frontiers).
 __device__ __forceinline__ void block_share(long long total, long long& lo, long long& hi, const GroupInfo& gi) {
     lo = total * (long long)gi.blk / gi.dim;
     hi = total * (long long)(gi.blk + 1) / gi.dim;
@@ -556,8 +577,32 @@ struct PrepSh {
     double acc_col_vol, acc_union_vol;
 };
 
-// Frontier compaction of one node per lane (W = 1): front index, degree
-// bucket, work items and the push row P[fidx].
+// A work item of a one-column tile holds its push value instead of the
+// frontier index of a push row: the edges are one load away from the item.
+// Row starts take 40 bits and lengths 24 (the host caps the row classes).
+template <typename T>
+__device__ __forceinline__ PushItem pack_item(long long rp, int len, T push) {
+    PushItem it;
+    it.rp = rp | ((long long)len << 40);
+    if constexpr (sizeof(T) == 8) {
+        it.len = __double2hiint(push);
+        it.fidx = __double2loint(push);
+    } else {
+        it.len = 0;
+        it.fidx = __float_as_int(push);
+    }
+    return it;
+}
+template <typename T>
+__device__ __forceinline__ T unpack_item(const PushItem& it, long long& rp, int& len) {
+    rp = it.rp & ((1ll << 40) - 1);
+    len = (int)((unsigned long long)it.rp >> 40);
+    if constexpr (sizeof(T) == 8) return __hiloint2double(it.len, it.fidx);
+    else return __int_as_float(it.fidx);
+}
+
+// Frontier compaction of one node per lane (W = 1): degree bucket and work
+// items, which carry the push value.
 template <typename T>
 __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, bool node_in, int len, long long rp,
                                              T push) {
@@ -581,39 +626,29 @@ __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, 
         if (lane >= o) sc += y;
     }
     const int wch = __shfl_sync(kFull, sc, 31);
-    int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
+    int b1 = 0, b2 = 0, b3 = 0;
     if (lane == 0) {
-        b0 = atomicAdd(&ts.front_cnt[par], __popc(bf));
+        atomicAdd(&ts.front_cnt[par], __popc(bf));
         if (bs) b1 = atomicAdd(&ts.small_cnt[par], __popc(bs));
         if (bm) b2 = atomicAdd(&ts.med_cnt[par], __popc(bm));
         if (wch) b3 = atomicAdd(&ts.large_cnt[par], wch);
     }
-    b0 = __shfl_sync(kFull, b0, 0);
     b1 = __shfl_sync(kFull, b1, 0);
     b2 = __shfl_sync(kFull, b2, 0);
     b3 = __shfl_sync(kFull, b3, 0);
     if (!node_in) return;
     const unsigned below = (1u << lane) - 1u;
-    const int fidx = b0 + __popc(bf & below);
-    PushItem item;
-    item.rp = rp;
-    item.len = len;
-    item.fidx = fidx;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;
     if (bucket == 0) {
-        bsmall[b1 + __popc(bs & below)] = item;
+        bsmall[b1 + __popc(bs & below)] = pack_item<T>(rp, len, push);
     } else if (bucket == 1) {
-        bsmall[(n - 1) - (b2 + __popc(bm & below))] = item;
+        bsmall[(n - 1) - (b2 + __popc(bm & below))] = pack_item<T>(rp, len, push);
     } else {
         PushItem* blarge = a.blarge + (int64_t)t * a.large_cap;
         const int lb = b3 + (sc - nch);
-        for (int ch = 0; ch < nch; ++ch) {
-            item.rp = rp + (long long)ch * a.chunk;
-            item.len = min(a.chunk, len - ch * a.chunk);
-            blarge[lb + ch] = item;
-        }
+        for (int ch = 0; ch < nch; ++ch)
+            blarge[lb + ch] = pack_item<T>(rp + (long long)ch * a.chunk, min(a.chunk, len - ch * a.chunk), push);
     }
-    reinterpret_cast<T*>(a.P)[(int64_t)t * n + fidx] = push;
 }
 
 // PREP of a W = 1 PPR/Katz local GD tile over candidates [beg, end): the
@@ -1260,26 +1295,25 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
         int fidx = 0;
         if (leader && node_in) {
             fidx = b0 + __popc(bf & below);
-            PushItem item;
-            item.rp = rp;
-            item.len = len;
-            item.fidx = fidx;
-            if (bucket == 0) bsmall[b1 + __popc(bs & below)] = item;
-            else if (bucket == 1) bmed_end[-(b2 + __popc(bm & below))] = item;
+            auto item_of = [&](long long at, int edges) {
+                if constexpr (W == 1) return pack_item<T>(at, edges, push.v[0]);
+                else return PushItem{at, edges, fidx};
+            };
+            if (bucket == 0) bsmall[b1 + __popc(bs & below)] = item_of(rp, len);
+            else if (bucket == 1) bmed_end[-(b2 + __popc(bm & below))] = item_of(rp, len);
             else {
                 int lb = b3 + (sc - lch);
-                for (int ch = 0; ch < nch; ++ch) {
-                    item.rp = rp + (long long)ch * a.chunk;
-                    item.len = min(a.chunk, len - ch * a.chunk);
-                    blarge[lb + ch] = item;
-                }
+                for (int ch = 0; ch < nch; ++ch)
+                    blarge[lb + ch] = item_of(rp + (long long)ch * a.chunk, min(a.chunk, len - ch * a.chunk));
             }
             if (dint) sum.ivol += di;
             else sum.vol += du;
             sum.cnt += 1;
         }
-        fidx = __shfl_sync(kFull, fidx, grp_w * L);
-        if (node_in) vstore<T, VEC>(Pw + (int64_t)fidx * W + c0, push);
+        if constexpr (W > 1) {
+            fidx = __shfl_sync(kFull, fidx, grp_w * L);
+            if (node_in) vstore<T, VEC>(Pw + (int64_t)fidx * W + c0, push);
+        }
     }
     total = sum;
 }
@@ -1535,35 +1569,30 @@ __device__ __forceinline__ void push_edge(const DevGraph& g, T* tgt, int64_t ld,
     vred<T, VEC>(tgt + (int64_t)v * ld + c0, q);
 }
 
-// Medium rows and chunks of long rows: one warp per work item, items
-// [beg, end) of `items` read with stride `step` (+1 for chunks, -1 for
-// medium rows, which fill the short-row array from its end; each item is at most a.med_max / a.chunk edges, a
-// few dependent warp iterations, so no hub row becomes the round's critical
-// path).  The item carries the row's start and length, so the warp goes
-// straight from the item to the column indices.
+// A medium row or a chunk of a long row, by one warp (at most a.med_max /
+// a.chunk edges, a few dependent warp iterations, so no hub row becomes the
+// round's critical path).  The item carries the row's start and length, so the
+// warp goes straight from the item to the column indices.
 template <typename T, int W>
-__device__ void scatter_warp_items(const PushArgs& a, const PushItem* items, int step,
-                                   const ScatterCtx<T, W>& c, long long beg, long long end) {
+__device__ __forceinline__ void scatter_item(const PushArgs& a, const ScatterCtx<T, W>& c, const PushItem& it, int beg,
+                                             int edges) {
     constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
     constexpr int L = W / VEC;
     constexpr int GPW = 32 / L;
-    const DevGraph& g = a.g;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const int lane_g = lane % L, grp_w = lane / L;
     const int c0 = lane_g * VEC;
     double theta[VEC];
     float theta_f[VEC];
     load_thetas<T, VEC>(c.cs, c0, c.cross, theta, theta_f);
-    for (long long k = beg + warp; k < end; k += kWarps) {
-        const PushItem it = items[k * step];
-        Vec<T, VEC> p;
-        vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
-        for (int j0 = 0; j0 < it.len; j0 += GPW) {
-            const int j = j0 + grp_w;
-            const bool ok = j < it.len;
-            const int v = ok ? g.col[it.rp + j] : 0;
-            edge_step<T, W, VEC, L>(a, c, ok, v, c0, lane_g, grp_w, p, theta, theta_f);
-        }
+    Vec<T, VEC> p;
+    vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
+    const int end = min(it.len, beg + edges);
+    for (int j0 = beg; j0 < end; j0 += GPW) {
+        const int j = j0 + grp_w;
+        const bool ok = j < end;
+        const int v = ok ? a.g.col[it.rp + j] : 0;
+        edge_step<T, W, VEC, L>(a, c, ok, v, c0, lane_g, grp_w, p, theta, theta_f);
     }
 }
 
@@ -1682,92 +1711,41 @@ __device__ __forceinline__ void load_edge(const DevGraph& g, long long j, int& v
     }
 }
 
-// W = 1 medium rows and long-row chunks: one warp per item, 32 * kEdgeILP
+// W = 1: a medium row or a chunk of a long row, by one warp, 32 * kEdgeILP
 // edges per warp iteration.  Lanes of one item target distinct nodes, so no
 // hub combine applies here.
 template <typename T>
-__device__ void scatter_warp_items_w1(const PushArgs& a, const PushItem* items, int step, const ScatterCtx<T, 1>& c,
-                                      long long beg, long long end) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double theta = c.cross ? c.cs[0].theta : 0.0;
+__device__ __forceinline__ void scatter_item_w1(const PushArgs& a, const ScatterCtx<T, 1>& c, const PushItem& it,
+                                                int beg, int edges, double theta) {
+    const int lane = threadIdx.x & 31;
     bool none[kEdgeILP];
+    T p[kEdgeILP];
+    long long rp;
+    int len;
+    const T pv = unpack_item<T>(it, rp, len);
 #pragma unroll
-    for (int u = 0; u < kEdgeILP; ++u) none[u] = false;
-    for (long long k = beg + warp; k < end; k += kWarps) {
-        const PushItem it = items[k * step];
-        const T pv = c.Pw[it.fidx];
-        T p[kEdgeILP];
+    for (int u = 0; u < kEdgeILP; ++u) {
+        none[u] = false;
+        p[u] = pv;
+    }
+    const int end = min(len, beg + edges);
+    for (int j0 = beg; j0 < end; j0 += 32 * kEdgeILP) {
+        bool ok[kEdgeILP];
+        int v[kEdgeILP];
+        uint32_t dc[kEdgeILP];
 #pragma unroll
-        for (int u = 0; u < kEdgeILP; ++u) p[u] = pv;
-#if GDE_VEC_COLS
-        // 128-bit column loads: the row's first 16-byte boundary, then each
-        // lane takes 4 consecutive column words with one load and pushes them
-        // kEdgeILP at a time
-        static_assert(4 % kEdgeILP == 0, "4 column words per lane split into kEdgeILP-edge steps");
-        if (a.g.col_deg && it.len >= 128) {
-            const int head = (int)((4 - (it.rp & 3)) & 3);
-            {
-                bool ok[kEdgeILP];
-                int v[kEdgeILP];
-                uint32_t dc[kEdgeILP];
-#pragma unroll
-                for (int u = 0; u < kEdgeILP; ++u) {
-                    ok[u] = (u == 0) && lane < head;
-                    v[u] = 0;
-                    dc[u] = 0;
-                    if (ok[u]) load_edge(a.g, it.rp + lane, v[u], dc[u]);
-                }
-                edges_w1<T>(a, c, ok, v, dc, p, theta, none, none);
-            }
-            const uint32_t* body = a.g.col_deg + it.rp + head;  // 16-byte aligned
-            const int nb = it.len - head;
-            const uint32_t mask = (1u << a.g.idx_bits) - 1u;
-            for (int b0 = 0; b0 < nb; b0 += 128) {
-                const int e = b0 + 4 * lane;
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
-                if (e + 3 < nb) {
-                    const uint4 q = *reinterpret_cast<const uint4*>(body + e);
-                    w[0] = q.x; w[1] = q.y; w[2] = q.z; w[3] = q.w;
-                } else {
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (e + i < nb) w[i] = body[e + i];
-                }
-#pragma unroll
-                for (int h = 0; h < 4; h += kEdgeILP) {
-                    bool ok[kEdgeILP];
-                    int v[kEdgeILP];
-                    uint32_t dc[kEdgeILP];
-#pragma unroll
-                    for (int u = 0; u < kEdgeILP; ++u) {
-                        ok[u] = e + h + u < nb;
-                        v[u] = (int)(w[h + u] & mask);
-                        dc[u] = w[h + u] >> a.g.idx_bits;
-                    }
-                    edges_w1<T>(a, c, ok, v, dc, p, theta, none, none);
-                }
-            }
-            continue;
+        for (int u = 0; u < kEdgeILP; ++u) {
+            const int j = j0 + u * 32 + lane;
+            ok[u] = j < end;
+            v[u] = 0;
+            dc[u] = 0;
+            if (ok[u]) load_edge(a.g, rp + j, v[u], dc[u]);
         }
-#endif
-        for (int j0 = 0; j0 < it.len; j0 += 32 * kEdgeILP) {
-            bool ok[kEdgeILP];
-            int v[kEdgeILP];
-            uint32_t dc[kEdgeILP];
-#pragma unroll
-            for (int u = 0; u < kEdgeILP; ++u) {
-                const int j = j0 + u * 32 + lane;
-                ok[u] = j < it.len;
-                v[u] = 0;
-                dc[u] = 0;
-                if (ok[u]) load_edge(a.g, it.rp + j, v[u], dc[u]);
-            }
-            edges_w1<T>(a, c, ok, v, dc, p, theta, none, none);
-        }
+        edges_w1<T>(a, c, ok, v, dc, p, theta, none, none);
     }
 }
 
-// W = 1 short rows flattened per warp: a warp takes GROUP consecutive items
+// W = 1 short rows flattened per warp: a warp takes up to 32 consecutive items
 // and spreads their edges evenly over its lanes, 32 * kEdgeILP edges per
 // step (the lane holding edge e finds its row by a binary search over the
 // warp's exclusive edge offsets), so a step carries every row's edges
@@ -1776,111 +1754,102 @@ __device__ void scatter_warp_items_w1(const PushArgs& a, const PushItem* items, 
 // global atomic; the crossing test on the combined add is the same test on
 // the stored value.  (Flattening medium rows the same way measured slower
 // than a warp per medium row.)
-template <typename T, int GROUP>
-__device__ void scatter_flat_w1(const PushArgs& a, const PushItem* items, int step, const ScatterCtx<T, 1>& c,
-                                long long beg, long long end) {
+template <typename T>
+__device__ void scatter_short_w1(const PushArgs& a, const PushItem* items, const ScatterCtx<T, 1>& c, int count,
+                                 double theta) {
     const DevGraph& g = a.g;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const double theta = c.cross ? c.cs[0].theta : 0.0;
     __shared__ T fagg[kWarps][32];
     __shared__ double faggd[kWarps][32];  // hub-prefix targets: the warp's sum in FP64
-    for (long long kb = beg + (long long)warp * GROUP; kb < end; kb += (long long)kWarps * GROUP) {
-        const long long k = kb + lane;
-        int len = 0;
-        long long rp = 0;
-        T pv = T(0);
-        if (lane < GROUP && k < end) {
-            const PushItem it = items[k * step];
-            rp = it.rp;
-            len = it.len;
-            pv = c.Pw[it.fidx];
-        }
-        int incl = len;
+    int len = 0;
+    long long rp = 0;
+    T pv = T(0);
+    if (lane < count) pv = unpack_item<T>(items[lane], rp, len);
+    int incl = len;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(kFull, incl, 31);
+    const int excl = incl - len;
+    for (int e0 = 0; e0 < total; e0 += 32 * kEdgeILP) {
+        bool ok[kEdgeILP], hub_done[kEdgeILP], hub_cr[kEdgeILP];
+        int v[kEdgeILP];
+        uint32_t dc[kEdgeILP];
+        T p[kEdgeILP];
+#pragma unroll
+        for (int u = 0; u < kEdgeILP; ++u) {
+            const int e = e0 + u * 32 + lane;
+            ok[u] = e < total;
+            // the row holding edge e: the last lane whose offset is <= e
+            int r = 0;
+#pragma unroll
+            for (int b = 16; b > 0; b >>= 1) {
+                const int ex = __shfl_sync(kFull, excl, (r + b) & 31);
+                if (r + b < 32 && ex <= e) r += b;
+            }
+            const long long rpr = __shfl_sync(kFull, rp, r);
+            const int exr = __shfl_sync(kFull, excl, r);
+            p[u] = __shfl_sync(kFull, pv, r);
+            v[u] = 0;
+            dc[u] = 0;
+            if (ok[u]) load_edge(g, rpr + (e - exr), v[u], dc[u]);
+            hub_done[u] = false;
+            hub_cr[u] = false;
         }
-        const int total = __shfl_sync(kFull, incl, 31);
-        const int excl = incl - len;
-        for (int e0 = 0; e0 < total; e0 += 32 * kEdgeILP) {
-            bool ok[kEdgeILP], hub_done[kEdgeILP], hub_cr[kEdgeILP];
-            int v[kEdgeILP];
-            uint32_t dc[kEdgeILP];
-            T p[kEdgeILP];
+        if (!c.tgt_scale) {
 #pragma unroll
             for (int u = 0; u < kEdgeILP; ++u) {
-                const int e = e0 + u * 32 + lane;
-                ok[u] = e < total;
-                // the row holding edge e: the last lane whose offset is <= e
-                int r = 0;
-#pragma unroll
-                for (int b = 16; b > 0; b >>= 1) {
-                    const int ex = __shfl_sync(kFull, excl, (r + b) & 31);
-                    if (r + b < GROUP && ex <= e) r += b;
+                const bool hub = ok[u] && v[u] < g.hub_cut;
+                if (!__any_sync(kFull, hub)) continue;
+                const unsigned peers = __match_any_sync(kFull, hub ? v[u] : -1 - lane);
+                const int leader = __ffs(peers) - 1;
+                const bool hd = hub && c.rh && v[u] < c.rh_cut;
+                if (hub && lane == leader) {
+                    fagg[warp][lane] = T(0);
+                    faggd[warp][lane] = 0.0;
                 }
-                const long long rpr = __shfl_sync(kFull, rp, r);
-                const int exr = __shfl_sync(kFull, excl, r);
-                p[u] = __shfl_sync(kFull, pv, r);
-                v[u] = 0;
-                dc[u] = 0;
-                if (ok[u]) load_edge(g, rpr + (e - exr), v[u], dc[u]);
-                hub_done[u] = false;
-                hub_cr[u] = false;
-            }
-            if (!c.tgt_scale) {
-#pragma unroll
-                for (int u = 0; u < kEdgeILP; ++u) {
-                    const bool hub = ok[u] && v[u] < g.hub_cut;
-                    if (!__any_sync(kFull, hub)) continue;
-                    const unsigned peers = __match_any_sync(kFull, hub ? v[u] : -1 - lane);
-                    const int leader = __ffs(peers) - 1;
-                    const bool hd = hub && c.rh && v[u] < c.rh_cut;
-                    if (hub && lane == leader) {
-                        fagg[warp][lane] = T(0);
-                        faggd[warp][lane] = 0.0;
-                    }
-                    __syncwarp();
-                    if (hd) atomicAdd(&faggd[warp][leader], (double)p[u]);
-                    else if (hub) atomicAdd(&fagg[warp][leader], p[u]);
-                    __syncwarp();
-                    if (hd && lane == leader) {
-                        // FP64 hub prefix: the combined add and the crossing test in FP64
-                        const double tot = faggd[warp][lane];
-                        const double old = atomicAdd(c.rh + v[u], tot);
+                __syncwarp();
+                if (hd) atomicAdd(&faggd[warp][leader], (double)p[u]);
+                else if (hub) atomicAdd(&fagg[warp][leader], p[u]);
+                __syncwarp();
+                if (hd && lane == leader) {
+                    // FP64 hub prefix: the combined add and the crossing test in FP64
+                    const double tot = faggd[warp][lane];
+                    const double old = atomicAdd(c.rh + v[u], tot);
+                    const double dv = (dc[u] != g.deg_esc) ? (double)dc[u]
+                                      : (g.degf_exact ? (double)g.degf[v[u]] : g.degd[v[u]]);
+                    const double thr = theta * dv;
+                    hub_cr[u] = (old < thr) && (old + tot >= thr);
+                } else if (hub && lane == leader) {
+                    const T tot = fagg[warp][lane];
+                    T* addr = c.tgt + (int64_t)v[u] * c.tld;
+                    if (c.cross) {
+                        const T old = atomicAdd(addr, tot);
+                        const T s = old + tot;
                         const double dv = (dc[u] != g.deg_esc) ? (double)dc[u]
                                           : (g.degf_exact ? (double)g.degf[v[u]] : g.degd[v[u]]);
-                        const double thr = theta * dv;
-                        hub_cr[u] = (old < thr) && (old + tot >= thr);
-                    } else if (hub && lane == leader) {
-                        const T tot = fagg[warp][lane];
-                        T* addr = c.tgt + (int64_t)v[u] * c.tld;
-                        if (c.cross) {
-                            const T old = atomicAdd(addr, tot);
-                            const T s = old + tot;
-                            const double dv = (dc[u] != g.deg_esc) ? (double)dc[u]
-                                              : (g.degf_exact ? (double)g.degf[v[u]] : g.degd[v[u]]);
-                            if constexpr (sizeof(T) == 4) {
-                                if (g.degf_exact) {
-                                    const float t32 = (float)theta * (float)dv;
-                                    hub_cr[u] = !ge_threshold(old, t32, theta, dv) && ge_threshold(s, t32, theta, dv);
-                                } else {
-                                    hub_cr[u] = ((double)old < theta * dv) && ((double)s >= theta * dv);
-                                }
+                        if constexpr (sizeof(T) == 4) {
+                            if (g.degf_exact) {
+                                const float t32 = (float)theta * (float)dv;
+                                hub_cr[u] = !ge_threshold(old, t32, theta, dv) && ge_threshold(s, t32, theta, dv);
                             } else {
-                                const double thr = theta * dv;
-                                hub_cr[u] = ((double)old < thr) && ((double)s >= thr);
+                                hub_cr[u] = ((double)old < theta * dv) && ((double)s >= theta * dv);
                             }
                         } else {
-                            atomicAdd(addr, tot);
+                            const double thr = theta * dv;
+                            hub_cr[u] = ((double)old < thr) && ((double)s >= thr);
                         }
+                    } else {
+                        atomicAdd(addr, tot);
                     }
-                    __syncwarp();
-                    hub_done[u] = hub;
                 }
+                __syncwarp();
+                hub_done[u] = hub;
             }
-            edges_w1<T>(a, c, ok, v, dc, p, theta, hub_done, hub_cr);
         }
+        edges_w1<T>(a, c, ok, v, dc, p, theta, hub_done, hub_cr);
     }
 }
 
@@ -1891,58 +1860,113 @@ __device__ void scatter_flat_w1(const PushArgs& a, const PushItem* items, int st
 // the groups' edge offsets), instead of one row per group and as many steps
 // as the warp's longest row (+4% on the 8-column InstantGNN push).
 template <typename T, int W>
-__device__ void scatter_small_flat(const PushArgs& a, int t, const ScatterCtx<T, W>& c, long long beg,
-                                   long long end) {
+__device__ void scatter_short(const PushArgs& a, const PushItem* items, const ScatterCtx<T, W>& c, int count) {
     constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
     constexpr int L = W / VEC;
     constexpr int GPW = 32 / L;
     const DevGraph& g = a.g;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const int lane_g = lane % L, grp_w = lane / L;
     const int c0 = lane_g * VEC;
-    const PushItem* bsmall = a.bsmall + (int64_t)t * a.g.n;
     double theta[VEC];
     float theta_f[VEC];
     load_thetas<T, VEC>(c.cs, c0, c.cross, theta, theta_f);
-    for (long long kb = beg + (long long)warp * GPW; kb < end; kb += (long long)kWarps * GPW) {
-        const long long k = kb + grp_w;
-        int len = 0;
-        long long rp = 0;
-        Vec<T, VEC> p;
+    int len = 0;
+    long long rp = 0;
+    Vec<T, VEC> p;
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) p.v[i] = T(0);
-        if (k < end) {
-            const PushItem it = bsmall[k];
-            rp = it.rp;
-            len = it.len;
-            vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
+    for (int i = 0; i < VEC; ++i) p.v[i] = T(0);
+    if (grp_w < count) {
+        const PushItem it = items[grp_w];
+        rp = it.rp;
+        len = it.len;
+        vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
+    }
+    // edge offsets by group: each group's first lane carries its row length
+    int incl = (lane_g == 0) ? len : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(kFull, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const int total = __shfl_sync(kFull, incl, 31);
+    const int excl = incl - ((lane_g == 0) ? len : 0);  // valid on each group's first lane
+    for (int e0 = 0; e0 < total; e0 += GPW) {
+        const int e = e0 + grp_w;
+        const bool ok = e < total;
+        // the group holding edge e: the last group whose offset is <= e
+        int r = 0;
+#pragma unroll
+        for (int b = GPW / 2; b > 0; b >>= 1) {
+            const int ex = __shfl_sync(kFull, excl, ((r + b) * L) & 31);
+            if (r + b < GPW && ex <= e) r += b;
         }
-        // edge offsets by group: each group's first lane carries its row length
-        int incl = (lane_g == 0) ? len : 0;
+        const long long rpr = __shfl_sync(kFull, rp, r * L);
+        const int exr = __shfl_sync(kFull, excl, r * L);
+        Vec<T, VEC> pr;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
+        for (int i = 0; i < VEC; ++i) pr.v[i] = __shfl_sync(kFull, p.v[i], r * L + lane_g);
+        const int v = ok ? g.col[rpr + (e - exr)] : 0;
+        edge_step<T, W, VEC, L>(a, c, ok, v, c0, lane_g, grp_w, pr, theta, theta_f);
+    }
+}
+
+// SCATTER of the group's live tiles, as units of one warp's work: a chunk of a
+// long row, a medium row, or a warp's worth of short rows.  Unit x goes to warp
+// x mod (warps of the group), spread over the blocks first: a round with few
+// units takes one unit's latency, not a long, a medium and a short one in turn
+// in every block.  Where the pieces would be few, chunks, medium rows and
+// groups of short rows are cut into pieces: a 256-edge item is 10 us of
+// dependent loads and atomics in one warp, half of a small round.  Up to 4
+// pieces per warp (1 / 2 / 4 / 16 measured: one FP64 query on 87k nodes 899 /
+// 878 / 858 / 815 us, one FP32 query on 2.36M nodes 1.53 / 1.53 / 1.53 / 1.62
+// ms).  With the items' push values and the one-word barrier, a query on 2.7k
+// nodes went from 0.78 to 0.52 ms in the kernel, the others above from 1.25
+// and 1.93 ms.
+template <typename T, int W>
+__device__ void scatter_units(const PushArgs& a, int ntl, const GroupInfo& gi) {
+    constexpr int SR = short_rows<T, W>();
+    const TileSlot* sl = tile_slots();
+    const long long total = sl[ntl].off[0];
+    const long long nw = (long long)gi.dim * kWarps;
+    long long lo = 0, hi = 0;
+    int k = -1, nl = 0, nm = 0, ns = 0;  // units of chunks and of medium rows; short rows
+    int cl = 1, cm = 1, edges = 0;       // pieces per chunk and per medium row; edges of a piece
+    int sr = SR;                         // short rows of a unit
+    double theta = 0.0;
+    const PushItem *bsmall = nullptr, *blarge = nullptr;
+    ScatterCtx<T, W> c{};
+    for (long long x = (long long)(threadIdx.x >> 5) * gi.dim + gi.blk; x < total; x += nw) {
+        if (x >= hi) {
+            do ++k;
+            while (x >= sl[k + 1].off[0]);
+            lo = sl[k].off[0];
+            hi = sl[k + 1].off[0];
+            const int t = sl[k].tile, par = sl[k].level & 1;
+            c = scatter_ctx<T, W>(a, t, sl[k].level, sl[k].flags);
+            const bool split = sl[k].split != 0;
+            cl = split ? pieces<T, W>(a.chunk) : 1;
+            cm = split ? pieces<T, W>(a.med_max) : 1;
+            edges = split ? piece_edges<T, W>() : 1 << 24;
+            sr = (split && SR >= 4) ? SR / 4 : SR;
+            nl = a.ts[t].large_cnt[par] * cl;
+            nm = a.ts[t].med_cnt[par] * cm;
+            ns = a.ts[t].small_cnt[par];
+            bsmall = a.bsmall + (int64_t)t * a.g.n;
+            blarge = a.blarge + (int64_t)t * a.large_cap;
+            if (W == 1) theta = c.cross ? c.cs[0].theta : 0.0;
         }
-        const int total = __shfl_sync(kFull, incl, 31);
-        const int excl = incl - ((lane_g == 0) ? len : 0);  // valid on each group's first lane
-        for (int e0 = 0; e0 < total; e0 += GPW) {
-            const int e = e0 + grp_w;
-            const bool ok = e < total;
-            // the group holding edge e: the last group whose offset is <= e
-            int r = 0;
-#pragma unroll
-            for (int b = GPW / 2; b > 0; b >>= 1) {
-                const int ex = __shfl_sync(kFull, excl, ((r + b) * L) & 31);
-                if (r + b < GPW && ex <= e) r += b;
-            }
-            const long long rpr = __shfl_sync(kFull, rp, r * L);
-            const int exr = __shfl_sync(kFull, excl, r * L);
-            Vec<T, VEC> pr;
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) pr.v[i] = __shfl_sync(kFull, p.v[i], r * L + lane_g);
-            const int v = ok ? g.col[rpr + (e - exr)] : 0;
-            edge_step<T, W, VEC, L>(a, c, ok, v, c0, lane_g, grp_w, pr, theta, theta_f);
+        const int u = (int)(x - lo);
+        if (u < nl + nm) {
+            const int i = u < nl ? u / cl : (u - nl) / cm;
+            const int piece = u < nl ? u - i * cl : u - nl - i * cm;
+            const PushItem it = u < nl ? blarge[i] : bsmall[(a.g.n - 1) - i];
+            if constexpr (W == 1) scatter_item_w1<T>(a, c, it, piece * edges, edges, theta);
+            else scatter_item<T, W>(a, c, it, piece * edges, edges);
+        } else {
+            const int s0 = (u - nl - nm) * sr;
+            if constexpr (W == 1) scatter_short_w1<T>(a, bsmall + s0, c, min(sr, ns - s0), theta);
+            else scatter_short<T, W>(a, bsmall + s0, c, min(sr, ns - s0));
         }
     }
 }
@@ -3040,8 +3064,8 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             t0 = t1;
         }
         // ---- SCATTER: flattened short rows / medium rows / long-row chunks ----
-        // a warp per space: short rows, medium rows, long-row chunks, retiring
-        // slots' nodes; another one the flags and the tiles that pull
+        // a warp each for the units of scatter work, the retiring slots' nodes,
+        // and the flags and the tiles that pull
         {
             auto pushes = [&](int k) {
                 const int t = sl[k].tile, lv = sl[k].level;
@@ -3050,21 +3074,23 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             };
             if (warp == 0)
                 warp_offsets(0, ntl, [&](int k) -> long long {
-                    return pushes(k) ? a.ts[sl[k].tile].small_cnt[sl[k].level & 1] : 0;
+                    const TileState& ts = a.ts[sl[k].tile];
+                    const int par = sl[k].level & 1;
+                    constexpr int SR = short_rows<T, W>();
+                    if (!pushes(k)) return 0;
+                    const long long nl = ts.large_cnt[par], nm = ts.med_cnt[par];
+                    const long long ns = (ts.small_cnt[par] + SR - 1) / SR;
+                    constexpr int SP = SR >= 4 ? SR / 4 : 1;
+                    const long long cut = nl * pieces<T, W>(a.chunk) + nm * pieces<T, W>(a.med_max) +
+                                          (ts.small_cnt[par] + SP - 1) / SP;
+                    sl[k].split = cut * ntl <= 4ll * gi.dim * kWarps;
+                    return sl[k].split ? cut : nl + nm + ns;
                 });
-            else if (warp == 1)
+            else if (warp == 1 && a.serve)
                 warp_offsets(1, ntl, [&](int k) -> long long {
-                    return pushes(k) ? a.ts[sl[k].tile].med_cnt[sl[k].level & 1] : 0;
-                });
-            else if (warp == 2)
-                warp_offsets(2, ntl, [&](int k) -> long long {
-                    return pushes(k) ? a.ts[sl[k].tile].large_cnt[sl[k].level & 1] : 0;
-                });
-            else if (warp == 3 && a.serve)
-                warp_offsets(3, ntl, [&](int k) -> long long {
                     return a.ts[sl[k].tile].front_cnt[sl[k].level & 1] == 0 ? n : 0;
                 });
-            else if (warp == 4) {
+            else if (warp == 2) {
                 int np = 0;
                 for (int k0 = 0; k0 < ntl; k0 += 32) {
                     const int k = k0 + lane;
@@ -3098,11 +3124,11 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             // slots whose query finished this round: extract + clear, every
             // block an equal share of the retiring slots' nodes
             long long lo, hi;
-            block_share(sl[ntl].off[3], lo, hi, gi);
+            block_share(sl[ntl].off[1], lo, hi, gi);
             if (lo < hi) {
-                for (int k = find_tile(3, ntl, lo); k < ntl && sl[k].off[3] < hi; ++k) {
-                    const long long b = max(lo, sl[k].off[3]) - sl[k].off[3];
-                    const long long e = min(hi, sl[k + 1].off[3]) - sl[k].off[3];
+                for (int k = find_tile(1, ntl, lo); k < ntl && sl[k].off[1] < hi; ++k) {
+                    const long long b = max(lo, sl[k].off[1]) - sl[k].off[1];
+                    const long long e = min(hi, sl[k + 1].off[1]) - sl[k].off[1];
                     if (b >= e) continue;
                     if (online) gather_online_range<T, W>(a, sl[k].tile, b, e);
                     else retire_range<T, W>(a, sl[k].tile, b, e);
@@ -3120,28 +3146,7 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
             }
         }
         trace_point(a, it, TP_SCAT_WORK);
-        // long-row chunks first (largest pieces), then medium, then short rows
-        for (int sp = 2; sp >= 0; --sp) {
-            long long lo, hi;
-            block_share(sl[ntl].off[sp], lo, hi, gi);
-            if (lo >= hi) continue;
-            for (int k = find_tile(sp, ntl, lo); k < ntl && sl[k].off[sp] < hi; ++k) {
-                const long long b = max(lo, sl[k].off[sp]) - sl[k].off[sp];
-                const long long e = min(hi, sl[k + 1].off[sp]) - sl[k].off[sp];
-                if (b >= e) continue;
-                const int t = sl[k].tile;
-                const ScatterCtx<T, W> c = scatter_ctx<T, W>(a, t, sl[k].level, sl[k].flags);
-                if constexpr (W == 1) {
-                    if (sp == 2) scatter_warp_items_w1<T>(a, a.blarge + (int64_t)t * a.large_cap, 1, c, b, e);
-                    else if (sp == 1) scatter_warp_items_w1<T>(a, a.bsmall + (int64_t)t * n + (n - 1), -1, c, b, e);
-                    else scatter_flat_w1<T, 32>(a, a.bsmall + (int64_t)t * n, 1, c, b, e);
-                } else {
-                    if (sp == 2) scatter_warp_items<T, W>(a, a.blarge + (int64_t)t * a.large_cap, 1, c, b, e);
-                    else if (sp == 1) scatter_warp_items<T, W>(a, a.bsmall + (int64_t)t * n + (n - 1), -1, c, b, e);
-                    else scatter_small_flat<T, W>(a, t, c, b, e);
-                }
-            }
-        }
+        scatter_units<T, W>(a, ntl, gi);
         // tiles whose round pulls have no work items above
         if (PULL && a.pull_div > 0) {
             if constexpr (PULL)

@@ -1,4 +1,4 @@
-"""Pull rounds: rows gather their neighbours' push values once a frontier holds a good part of the graph.
+"""Pull rounds, and the row items of push rounds: rows gather their neighbours' push values once a frontier holds a good part of the graph.
 
 Row lengths sit on both sides of every class boundary of the pull plan (16, 64, 256-edge chunks), frontiers
 cover the whole graph within a few rounds, and FP64 operation counts must stay those of the oracle's pushes.
@@ -131,3 +131,21 @@ def test_rows_that_do_not_match_are_pushed(W):
         xo, _, oo = O.ppr_gd(n, indptr, indices, deg, int(s), 0.1, 1e-6, True)
         assert res["oper"][i] == pytest.approx(oo, rel=OPER_RTOL)
         assert rel_l1(res["x"][i], xo) < FP64_L1
+
+
+@pytest.mark.parametrize("tuning", [None, {"small_max": 3, "med_max": 70, "chunk": 100},
+                                    {"small_max": 16, "med_max": 1000, "chunk": 1000}])
+@pytest.mark.parametrize("W", [1, 8])
+def test_row_items_and_their_pieces(tuning, W):
+    """Rows around every class limit, whole and cut into pieces, pushed by warps of one and of several columns."""
+    g = _hubs()
+    G = api.Graph(g.indptr, g.indices)
+    deg = g.degree.astype(np.float64)
+    seeds = np.arange(g.n - 14, g.n, 2, dtype=np.int32)  # the hubs push first
+    for eps in (1e-3, 1e-5):
+        e = np.minimum(eps, 1.0 / deg[seeds])
+        res = api.solve(G, L.PPR, L.LOCAL_GD, seeds, e, prec="fp64", alpha=0.1, tile_w=W, tuning=tuning)
+        for i, s in enumerate(seeds):
+            xo, _, oo = O.ppr_gd(g.n, g.indptr, g.indices, deg, int(s), 0.1, e[i], True)
+            assert res["oper"][i] == pytest.approx(oo, rel=OPER_RTOL)
+            assert rel_l1(res["x"][i], xo) < FP64_L1
