@@ -75,6 +75,41 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
     return t;
 }
 
+// FP64 comparisons |r| >= thr and r >= thr of a threshold thr >= 0, on the
+// bit patterns (the order of non-negative doubles is that of their bits; a
+// NaN compares false, as in FP64).  GB300 runs one FP64 instruction per SM
+// and warp in 16 cycles, an integer one in one: the FP64 tiles' tests, like
+// their divisions (DevGraph::rdeg), stay off that pipe where they can.
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+__device__ __forceinline__ bool ge_bits(long long r, long long thr) { return r >= thr && r <= kInfBits; }
+__device__ __forceinline__ bool ge_abs64(double r, double thr) {
+    return ge_bits(__double_as_longlong(r) & 0x7fffffffffffffffll, __double_as_longlong(thr));
+}
+
+// A work item of a one-column tile holds its push value instead of the
+// frontier index of a push row: the edges are one load away from the item.
+// Row starts take 40 bits and lengths 24 (the host caps the row classes).
+template <typename T>
+__device__ __forceinline__ PushItem pack_item(long long rp, int len, T push) {
+    PushItem it;
+    it.rp = rp | ((long long)len << 40);
+    if constexpr (sizeof(T) == 8) {
+        it.len = __double2hiint(push);
+        it.fidx = __double2loint(push);
+    } else {
+        it.len = 0;
+        it.fidx = __float_as_int(push);
+    }
+    return it;
+}
+template <typename T>
+__device__ __forceinline__ T unpack_item(const PushItem& it, long long& rp, int& len) {
+    rp = it.rp & ((1ll << 40) - 1);
+    len = (int)((unsigned long long)it.rp >> 40);
+    if constexpr (sizeof(T) == 8) return __hiloint2double(it.len, it.fidx);
+    else return __int_as_float(it.fidx);
+}
+
 // Append v to a candidate list once per stamp (mark dedup), one atomic per
 // warp for all appending lanes.  `mask` must name every lane executing the
 // call.

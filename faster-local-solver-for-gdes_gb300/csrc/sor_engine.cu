@@ -17,9 +17,10 @@
 // with no node at or above threshold.
 //
 // One persistent cooperative launch runs all queries (one residual vector
-// each) through the sweeps; per colour it has two phases separated by the
-// bounded grid barrier: RELAX (pending nodes of the colour: test, update x and
-// r, write push values) and PUSH (one warp per relaxed node's row, atomic
+// each, a group of blocks per query with its own barrier) through the sweeps;
+// per colour it has two phases separated by the bounded group barrier: RELAX
+// (pending nodes of the colour: test, update x and r, write the rows as work
+// items with their push values) and PUSH (one warp per 64-edge item, atomic
 // residual updates, pending appends).
 #include <cuda_runtime.h>
 
@@ -60,22 +61,25 @@ struct SorArgs {
     int32_t* plist;          // [nq][2][n] pending lists, colour c at [cstart[c], cstart[c+1])
     int* pcnt;               // [nq][2][C]
     int32_t* mark;           // [nq][n] 1 while pending
-    int32_t* front;          // [nq][n] nodes relaxed in this phase
-    void* pv;                // [nq][n] their push values (T)
-    int* fcnt;               // [nq][2] by phase parity
+    PushItem* items;         // [nq][item_cap] the relaxed rows, in pieces with their push values (pack_item)
+    int64_t item_cap;
+    int* fcnt;               // [nq][2] items by phase parity
     unsigned long long* gcnt;// [nq][2] global: nodes at or above threshold after a sweep
     const double* theta;     // [nq]
     double* oper;            // [nq]
     int* sweeps;             // [nq]
     int* done;               // [nq]
     int max_sweeps;
+    int groups;              // block groups, each with its own queries and barrier bar[g]
     GridBarrier* bar;
     int* err;
 };
 
+// |r| >= theta d: FP64 residuals on bit patterns (ge_abs64), FP32 ones in FP64.
 template <typename T>
 __device__ __forceinline__ bool at_or_above(T r, double theta, double d) {
-    return fabs((double)r) >= theta * d;
+    if constexpr (sizeof(T) == 8) return ge_abs64(r, theta * d);
+    else return fabs((double)r) >= theta * d;
 }
 
 // pending append of v (colour cv) into buffer b of query q
@@ -85,13 +89,20 @@ __device__ __forceinline__ void push_pending(const SorArgs& a, int q, int b, int
     a.plist[((int64_t)q * 2 + b) * n + a.cstart[cv] + slot] = v;
 }
 
+// The blocks that work on this block's queries: group g holds blocks
+// [ceil(g B / G), ceil((g+1) B / G)) and takes the queries g, g + G, ... in turn.
+struct SorGroup {
+    int id, blk, dim;
+};
+
+constexpr int kSorPiece = 64;  // edges of a work item: two loads per lane of a warp
+
 template <typename T>
-__device__ void relax_phase(const SorArgs& a, int q, int c, int p, int it) {
+__device__ void relax_phase(const SorArgs& a, int q, int c, int p, int it, const SorGroup& gi) {
     const int64_t n = a.g.n;
     T* R = reinterpret_cast<T*>(a.R) + (int64_t)q * n;
     double* X = a.X + (int64_t)q * n;
-    T* pv = reinterpret_cast<T*>(a.pv) + (int64_t)q * n;
-    int32_t* front = a.front + (int64_t)q * n;
+    PushItem* items = a.items + (int64_t)q * a.item_cap;
     int32_t* mark = a.mark + (int64_t)q * n;
     int* fc = &a.fcnt[q * 2 + (it & 1)];
     const double theta = a.theta[q];
@@ -107,28 +118,27 @@ __device__ void relax_phase(const SorArgs& a, int q, int c, int p, int it) {
         list = a.corder + cb;
     }
     double my_oper = 0.0;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < count; base += stride) {
+    const int64_t stride = (int64_t)gi.dim * blockDim.x;
+    for (int64_t base = (int64_t)gi.blk * blockDim.x; base < count; base += stride) {
         const int64_t i = base + threadIdx.x;
         bool act = false;
-        int u = 0;
+        int len = 0;
+        int64_t rp = 0;
         T push = T(0);
         if (i < count) {
-            u = list[i];
+            const int u = list[i];
             if (a.local) mark[u] = 0;
             const T r = R[u];
             const double d = a.g.degd[u];
             const double tf = (a.ign == 1) ? a.g.nfac[u] : d;  // threshold factor: d, or d^(1-beta)
+            rp = a.g.row_ptr[u];
+            len = a.katz ? (int)(a.g.row_ptr[u + 1] - rp) : a.g.row_len[u];
             act = a.local ? at_or_above(r, theta, tf) : (r != T(0));
-            if (act && a.ign) {
-                const int64_t rp = a.g.row_ptr[u];
-                const int len = a.g.row_len[u];
-                if (len == 0 || (len == 1 && a.g.col[rp] == u)) {
-                    // absorbing node: p = r, r = 0 (InstantGNN.py:81-84, ppr_solver.py:802-805)
-                    X[u] = (double)r;
-                    R[u] = T(0);
-                    act = false;
-                }
+            if (act && a.ign && (len == 0 || (len == 1 && a.g.col[rp] == u))) {
+                // absorbing node: p = r, r = 0 (InstantGNN.py:81-84, ppr_solver.py:802-805)
+                X[u] = (double)r;
+                R[u] = T(0);
+                act = false;
             }
             if (act && a.ign == 1) {
                 // InstantGNN.py:85-88
@@ -156,48 +166,60 @@ __device__ void relax_phase(const SorArgs& a, int q, int c, int p, int it) {
                 }
             }
         }
-        const unsigned b = __ballot_sync(0xffffffffu, act);
-        if (b) {
-            int slot = 0;
-            if (lane == 0) slot = atomicAdd(fc, __popc(b));
-            slot = __shfl_sync(0xffffffffu, slot, 0) + __popc(b & ((1u << lane) - 1u));
-            if (act) {
-                front[slot] = u;
-                pv[slot] = push;
-            }
+        // the row as items of kSorPiece edges, which other warps pick up
+        const int np = act ? (len + kSorPiece - 1) / kSorPiece : 0;
+        int inc = np;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
         }
+        const int total = __shfl_sync(0xffffffffu, inc, 31);
+        if (total == 0) continue;
+        int slot = 0;
+        if (lane == 0) slot = atomicAdd(fc, total);
+        slot = __shfl_sync(0xffffffffu, slot, 0) + inc - np;
+        for (int k = 0; k < np; ++k)
+            items[slot + k] = pack_item<T>(rp + (long long)k * kSorPiece, min(kSorPiece, len - k * kSorPiece), push);
     }
     if (a.local && my_oper != 0.0) atomicAdd(&a.oper[q], my_oper);
 }
 
 template <typename T>
-__device__ void push_phase(const SorArgs& a, int q, int c, int p, int it) {
+__device__ void push_phase(const SorArgs& a, int q, int c, int p, int it, const SorGroup& gi) {
     const int64_t n = a.g.n;
     T* R = reinterpret_cast<T*>(a.R) + (int64_t)q * n;
-    const T* pv = reinterpret_cast<const T*>(a.pv) + (int64_t)q * n;
-    const int32_t* front = a.front + (int64_t)q * n;
+    const PushItem* items = a.items + (int64_t)q * a.item_cap;
     int32_t* mark = a.mark + (int64_t)q * n;
     const int nf = a.fcnt[q * 2 + (it & 1)];
     const double theta = a.theta[q];
     const int lane = threadIdx.x & 31;
-    const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t f = warp; f < nf; f += nwarps) {
-        const int u = front[f];
-        const T val = pv[f];
-        const int64_t rp = a.g.row_ptr[u];
-        const int len = a.katz ? (int)(a.g.row_ptr[u + 1] - rp) : a.g.row_len[u];
-        for (int j = lane; j < len; j += 32) {
-            const int v = a.g.col[rp + j];
+    const int nwarps = gi.dim * (kSorThreads / 32);
+    // (spread over the blocks first: few items keep few warps per SM busy)
+    for (int f = (threadIdx.x >> 5) * gi.dim + gi.blk; f < nf; f += nwarps) {
+        long long rp;
+        int len;
+        const T val = unpack_item<T>(items[f], rp, len);
+        constexpr int K = kSorPiece / 32;
+        int v[K];
+        T add[K], old[K];
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = (lane + 32 * k < len) ? a.g.col[rp + lane + 32 * k] : -1;
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
             // InstantGNN divides by d_v^beta at the target (InstantGNN.py:90)
-            const T add = (a.ign == 1) ? (T)((double)val / a.g.tfac[v]) : val;
-            const T old = atomicAdd(R + v, add);
-            if (a.local) {
-                const T now = old + add;
-                const double tf = (a.ign == 1) ? a.g.nfac[v] : a.g.degd[v];
-                if (at_or_above(now, theta, tf) && mark[v] == 0 && atomicExch(&mark[v], 1) == 0) {
-                    const int cv = a.color[v];
-                    push_pending(a, q, (cv > c) ? p : (p ^ 1), v, cv);
+            add[k] = (a.ign == 1 && v[k] >= 0) ? (T)((double)val / a.g.tfac[v[k]]) : val;
+            old[k] = v[k] >= 0 ? atomicAdd(R + v[k], add[k]) : T(0);
+        }
+        if (a.local) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                if (v[k] < 0) continue;
+                const T now = old[k] + add[k];
+                const double tf = (a.ign == 1) ? a.g.nfac[v[k]] : a.g.degd[v[k]];
+                if (at_or_above(now, theta, tf) && mark[v[k]] == 0 && atomicExch(&mark[v[k]], 1) == 0) {
+                    const int cv = a.color[v[k]];
+                    push_pending(a, q, (cv > c) ? p : (p ^ 1), v[k], cv);
                 }
             }
         }
@@ -206,85 +228,90 @@ __device__ void push_phase(const SorArgs& a, int q, int c, int p, int it) {
 
 // nodes at or above threshold after a global sweep
 template <typename T>
-__device__ void count_phase(const SorArgs& a, int q, int b) {
+__device__ void count_phase(const SorArgs& a, int q, int b, const SorGroup& gi) {
     const int64_t n = a.g.n;
     const T* R = reinterpret_cast<const T*>(a.R) + (int64_t)q * n;
     const double theta = a.theta[q];
     unsigned long long cnt = 0;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += (int64_t)gridDim.x * blockDim.x)
+    for (int64_t u = (int64_t)gi.blk * blockDim.x + threadIdx.x; u < n; u += (int64_t)gi.dim * blockDim.x)
         cnt += at_or_above(R[u], theta, a.g.degd[u]) ? 1ull : 0ull;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&a.gcnt[q * 2 + b], cnt);
 }
 
+// Each group of blocks runs its queries one after another, with sweeps and a
+// barrier of its own: a colour's two phases are a handful of dependent L2 round
+// trips, so queries that shared every barrier of the whole grid waited for each
+// other's chains, colour by colour.  87k nodes, FP64, omega 1.2 to 1.3: 6
+// queries 51.5 -> 4.7 ms, 60 queries 38 -> 1.6 ms, one query 11.6 -> 2.6 ms
+// (with the 64-edge items and the skipped empty colours); what bounds it is
+// the chain of two phases and two barriers per pending colour.
 template <typename T>
-__global__ void __launch_bounds__(kSorThreads) sor_kernel(SorArgs a) {
-    __shared__ int s_live;
-    __shared__ int s_work;
+__global__ void __launch_bounds__(kSorThreads) sor_kernel(const __grid_constant__ SorArgs a) {
+    __shared__ int s_next;
     const int C = a.ncolors;
+    const int lane = threadIdx.x & 31;
+    SorGroup gi;
+    {
+        const long long B = gridDim.x, G = a.groups;
+        gi.id = (int)(blockIdx.x * G / B);
+        const int start = (int)((gi.id * B + G - 1) / G), end = (int)(((gi.id + 1) * B + G - 1) / G);
+        gi.blk = (int)blockIdx.x - start;
+        gi.dim = end - start;
+    }
+    GridBarrier* bar = a.bar + gi.id;
     int it = 0;  // phase-pair counter (fcnt parity)
-    for (int sweep = 0;; ++sweep) {
-        const int p = sweep & 1;
-        // ---- sweep start: which queries are still going (identical in every block) ----
-        if (threadIdx.x == 0) {
-            int live = 0;
-            for (int q = 0; q < a.nq; ++q) {
-                if (a.done[q]) continue;
-                bool more;
-                if (a.local) {
-                    long long pend = 0;
-                    for (int c = 0; c < C; ++c) pend += a.pcnt[((int64_t)q * 2 + p) * C + c];
-                    more = pend > 0;
-                } else {
-                    more = (sweep == 0) || a.gcnt[q * 2 + (p ^ 1)] > 0;
-                }
-                if (!more || sweep >= a.max_sweeps) {
-                    if (blockIdx.x == 0) {
-                        a.done[q] = more ? 2 : 1;  // 2: stopped at max_sweeps
-                        a.sweeps[q] = sweep;
+    for (int q = gi.id; q < a.nq; q += a.groups) {
+        for (int sweep = 0;; ++sweep) {
+            const int p = sweep & 1;
+            const int* pend = a.pcnt + ((int64_t)q * 2 + p) * C;
+            for (int c = -1;;) {
+                // the next colour with pending nodes (global: the next one): the
+                // same answer in every block, from counts settled by the barrier
+                if (threadIdx.x < 32) {
+                    int next = C;
+                    if (!a.local) {
+                        next = (c >= 0 || sweep == 0 || a.gcnt[q * 2 + (p ^ 1)] > 0) ? c + 1 : C;
+                    } else {
+                        for (int c0 = c + 1; c0 < C && next == C; c0 += 32) {
+                            const unsigned b = __ballot_sync(0xffffffffu, c0 + lane < C && pend[c0 + lane] > 0);
+                            if (b) next = c0 + __ffs(b) - 1;
+                        }
                     }
-                } else {
-                    live = 1;
+                    if (lane == 0) s_next = next;
                 }
-            }
-            s_live = live;
-        }
-        __syncthreads();
-        if (!s_live) break;
-        if (!grid_barrier(a.bar, a.err)) return;  // done flags settled before anyone moves on
-        for (int c = 0; c < C; ++c) {
-            // skip a colour with nothing pending in any live query (same answer in every block)
-            if (threadIdx.x == 0) {
-                int work = 0;
-                for (int q = 0; q < a.nq && !work; ++q)
-                    if (!a.done[q]) work = !a.local || a.pcnt[((int64_t)q * 2 + p) * C + c] > 0;
-                s_work = work;
-            }
-            __syncthreads();
-            if (!s_work) continue;
-            for (int q = 0; q < a.nq; ++q)
-                if (!a.done[q]) relax_phase<T>(a, q, c, p, it);
-            if (!grid_barrier(a.bar, a.err)) return;
-            for (int q = 0; q < a.nq; ++q)
-                if (!a.done[q]) push_phase<T>(a, q, c, p, it);
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                for (int q = 0; q < a.nq; ++q) {
+                __syncthreads();
+                const int next = s_next;
+                __syncthreads();
+                if (next >= C || (c < 0 && sweep >= a.max_sweeps)) {
+                    if (c < 0) {  // a sweep that has nothing to do, or one too many, ends the query
+                        if (gi.blk == 0 && threadIdx.x == 0) {
+                            a.done[q] = next < C ? 2 : 1;  // 2: stopped at max_sweeps
+                            a.sweeps[q] = sweep;
+                        }
+                        goto next_query;
+                    }
+                    break;
+                }
+                c = next;
+                relax_phase<T>(a, q, c, p, it, gi);
+                if (!grid_barrier(bar, a.err, 0, gi.dim)) return;
+                push_phase<T>(a, q, c, p, it, gi);
+                if (gi.blk == 0 && threadIdx.x == 0) {
                     a.pcnt[((int64_t)q * 2 + p) * C + c] = 0;  // consumed (no PUSH appends to colour c)
                     a.fcnt[q * 2 + ((it + 1) & 1)] = 0;
                 }
+                ++it;
+                if (!grid_barrier(bar, a.err, 0, gi.dim)) return;
             }
-            ++it;
-            if (!grid_barrier(a.bar, a.err)) return;
+            if (!a.local) {
+                if (gi.blk == 0 && threadIdx.x == 0) a.gcnt[q * 2 + (p ^ 1)] = 0;
+                count_phase<T>(a, q, p, gi);
+                if (!grid_barrier(bar, a.err, 0, gi.dim)) return;
+            }
         }
-        if (!a.local) {
-            if (blockIdx.x == 0 && threadIdx.x == 0)
-                for (int q = 0; q < a.nq; ++q) a.gcnt[q * 2 + (p ^ 1)] = 0;
-            if (!grid_barrier(a.bar, a.err)) return;
-            for (int q = 0; q < a.nq; ++q)
-                if (!a.done[q]) count_phase<T>(a, q, p);
-            if (!grid_barrier(a.bar, a.err)) return;
-        }
+    next_query:;
     }
 }
 
@@ -433,15 +460,15 @@ int sor_prepare(gde_ctx* ctx, gde_graph* G, int64_t nq, int prec64, const std::v
     a.plist = (int32_t*)ws("sor_plist", (size_t)nq * 2 * n * 4);
     a.pcnt = (int*)ws("sor_pcnt", (size_t)nq * 2 * C * 4);
     a.mark = (int32_t*)ws("sor_mark", (size_t)nq * n * 4);
-    a.front = (int32_t*)ws("sor_front", (size_t)nq * n * 4);
-    a.pv = ws("sor_pv", (size_t)nq * n * es);
+    a.item_cap = n + G->g.cap / kSorPiece + 1;
+    a.items = (PushItem*)ws("sor_items", (size_t)nq * a.item_cap * sizeof(PushItem));
     a.fcnt = (int*)ws("sor_fcnt", (size_t)nq * 2 * 4);
     a.gcnt = (unsigned long long*)ws("sor_gcnt", (size_t)nq * 2 * 8);
     double* d_theta = (double*)ws("sor_theta", (size_t)nq * 8);
     a.oper = (double*)ws("sor_oper", (size_t)nq * 8);
     a.sweeps = (int*)ws("sor_sweeps", (size_t)nq * 4);
     a.done = (int*)ws("sor_done", (size_t)nq * 4);
-    if (!d_color || !d_corder || !d_cstart || !a.R || !a.X || !a.plist || !a.pcnt || !a.mark || !a.front || !a.pv ||
+    if (!d_color || !d_corder || !d_cstart || !a.R || !a.X || !a.plist || !a.pcnt || !a.mark || !a.items ||
         !a.fcnt || !a.gcnt || !d_theta || !a.oper || !a.sweeps || !a.done)
         return gde_internal_fail(ctx, GDE_ENOMEM, "device memory exhausted (SOR workspace)");
     a.color = d_color;
@@ -469,12 +496,14 @@ int sor_prepare(gde_ctx* ctx, gde_graph* G, int64_t nq, int prec64, const std::v
 int sor_run(gde_ctx* ctx, SorArgs& a, int prec64, std::vector<double>& hop, std::vector<int>& hsw, bool* capped,
             float* ms) {
     cudaStream_t st = ctx->stream;
-    SO_CK(cudaMemsetAsync(ctx->bar, 0, sizeof(GridBarrier), st));
+    SO_CK(cudaMemsetAsync(ctx->bar, 0, kMaxGroups * sizeof(GridBarrier), st));
     SO_CK(cudaMemsetAsync(ctx->derr, 0, sizeof(int), st));
     int per_sm = 0;
     if (prec64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sor_kernel<double>, kSorThreads, 0);
     else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sor_kernel<float>, kSorThreads, 0);
     const int grid = std::max(1, std::min(per_sm, 4)) * ctx->sms;
+    // a group per query while it leaves each at least four blocks
+    a.groups = (int)std::max<int64_t>(1, std::min<int64_t>({(int64_t)a.nq, (int64_t)grid / 4, (int64_t)kMaxGroups}));
     void* args[] = {&a};
     SO_CK(cudaEventRecord(ctx->ev[0], st));
     if (prec64) SO_CK(cudaLaunchCooperativeKernel((void*)sor_kernel<double>, grid, kSorThreads, args, 0, st));
