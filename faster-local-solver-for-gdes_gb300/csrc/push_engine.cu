@@ -747,12 +747,11 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
 // PREP of a W > 1 tile whose round pulls (every method but Chebyshev and the
 // relaxed heat kernel): most visited nodes push, so every load of a node --
 // residual, solution, Kahan term, degree, divisor -- is issued before any is
-// used, for kPullPrep nodes per lane group at a time, and the push row goes to
-// P by node id with no work items.  The arithmetic is prep_nodes'.  PREP of
-// the 128-column FP64 push went from 90 to 64 ms with it; it is bound by the
-// latency of the node loads and by FP64 issue.
-constexpr int kPullPrep = 2;
-
+// used, and the push row goes to P by node id with no work items.  The
+// arithmetic is prep_nodes'.  PREP of the 128-column FP64 InstantGNN push went
+// from 90 to 41 ms with it, of global GD FP32 on 2.36M nodes from 28 to 17; a
+// second to fourth node per lane group at a time measured 7 to 17% slower (the
+// registers).  It is bound by instruction issue, FP64's first.
 template <typename T, int W>
 struct PrepSums {
     static constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
@@ -765,184 +764,160 @@ struct PrepSums {
 };
 
 template <typename T, int W>
-__device__ void prep_pull(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
-                          PrepSums<T, W>& sum) {
+__device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
+                                       PrepSums<T, W>& total) {
     constexpr int VEC = PrepSums<T, W>::VEC;
     constexpr int L = W / VEC;
     constexpr int GPW = 32 / L;
-    constexpr int Q = kPullPrep;
+    constexpr bool F64 = sizeof(T) == 8;
     const DevGraph& g = a.g;
     const int64_t n = g.n;
-    const int par = sh.parity, kind = sh.tp.kind;
-    const bool global = method_is_global(sh.tp.method), hk = kind == KIND_HK, ign = kind == KIND_IGN;
+    const int kind = sh.tp.kind;
+    const bool hk = kind == KIND_HK, ign = kind == KIND_IGN, katz = kind == KIND_KATZ;
     const bool lone = ign || kind == KIND_UPPR;  // nodes without neighbours absorb their residual
+    const bool all = method_is_global(sh.tp.method);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int lane_g = lane % L, grp_w = lane / L;
-    const int c0 = lane_g * VEC;
-    const int32_t* cand = a.cand + ((int64_t)t * 2 + par) * n;
-    uint32_t* bits = tile_bits(a, t, par);
-    T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W;
-    T* R = slab_ptr<T>((hk && (sh.level & 1)) ? a.R2 : a.R, a, t);
-    T* X = xslab_ptr<T>(a.X, a, t);
-    float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) : nullptr;
+    const int grp_w = lane / L, c0 = (lane % L) * VEC;
+    const int32_t* cand = a.cand + ((int64_t)t * 2 + sh.parity) * n;
+    uint32_t* bits = tile_bits(a, t, sh.parity);
+    T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W + c0;
+    T* R = slab_ptr<T>((hk && (sh.level & 1)) ? a.R2 : a.R, a, t) + c0;
+    T* X = xslab_ptr<T>(a.X, a, t) + c0;
+    float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
     const int64_t xld = x_ld(a);
-    const double alpha = sh.tp.alpha;
-    const double* rdiv = (sizeof(T) == 8 && kind != KIND_KATZ) ? (ign ? g.rnf : g.rdeg) : nullptr;
-    const bool f32 = (sizeof(T) == 4) && g.degf_exact;
+    const bool f32 = !F64 && g.degf_exact;
     const bool dint = g.degf_exact != 0;
+    // a push is (coef r) / div with div = the degree, InstantGNN's d^(1-beta)
+    // or (Katz) 1; the solution takes gain r
     const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
-    const double hkc = hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.)) : 0.0;
-    const float hkc_f = (float)hkc, alpha_f = (float)alpha, omalpha_f = (float)(1. - alpha);
-    const double x_gain = ign ? sh.tp.x_gain : 1.0;
-    const float xgain_f = (float)x_gain;
-    double theta[VEC], scale0 = 0.0;
+    const double coef = hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.))
+                           : (katz ? sh.tp.alpha : 1. - sh.tp.alpha);
+    const float coef_f = (float)coef;
+    const T gain = (T)(ign ? sh.tp.x_gain : 1.0);
+    const double* rdiv = F64 && !katz ? (ign ? g.rnf : g.rdeg) : nullptr;
     float thr_f[VEC];
-    bool live[VEC], same = true;
+    unsigned live = 0;
+    bool same = true;
 #pragma unroll
     for (int k = 0; k < VEC; ++k) {
-        live[k] = sh.col_live[c0 + k] != 0;
-        theta[k] = sh.col_theta[c0 + k];
-        same &= theta[k] == theta[0];
-        thr_f[k] = (float)(hk ? theta[k] / hk_div : theta[k]);
+        live |= sh.col_live[c0 + k] ? 1u << k : 0u;
+        same &= sh.col_theta[c0 + k] == sh.col_theta[c0];
+        thr_f[k] = (float)(hk ? sh.col_theta[c0 + k] / hk_div : sh.col_theta[c0 + k]);
     }
-    scale0 = hk ? theta[0] / hk_div : theta[0];
-    for (long long base = beg + (long long)warp * GPW * Q; base < end; base += (long long)kWarps * GPW * Q) {
-        int u[Q], len[Q];
-        float df[Q];
-        double nf[Q], rd[Q], dd[Q];
-        Vec<T, VEC> r[Q], x[Q];
-        Vec<float, VEC> xc[Q];
-        bool valid[Q];
-#pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            const long long i = base + q * GPW + grp_w;
-            valid[q] = i < end;
-            u[q] = valid[q] ? (sh.dense ? (int)i : cand[i]) : 0;
+    const double scale0 = hk ? sh.col_theta[c0] / hk_div : sh.col_theta[c0];
+    PrepSums<T, W> sum = total;
+    for (long long base = beg + (long long)warp * GPW; base < end; base += (long long)kWarps * GPW) {
+        int len = 2;
+        float df = 1.f;
+        double nf = 0.0, rd = 1.0;
+        Vec<T, VEC> r, x;
+        Vec<float, VEC> xc;
+        const long long i = base + grp_w;
+        const int u = i < end ? (sh.dense ? (int)i : cand[i]) : -1;
+        if (u >= 0) {
+            vload<T, VEC>(R + (int64_t)u * a.ld, r);
+            vload<T, VEC>(X + (int64_t)u * xld, x);
+            if (!F64 && XC) vload<float, VEC>(XC + (int64_t)u * xld, xc);
+            df = g.degf[u];
+            if (ign) nf = g.nfac[u];
+            if (F64 && rdiv) rd = rdiv[u];
+            if (lone) len = g.row_len[u];
         }
+        unsigned act = 0;  // active columns of this lane
+        bool absorb = false;
+        Vec<T, VEC> push;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            if (!valid[q]) continue;
-            vload<T, VEC>(R + (int64_t)u[q] * a.ld + c0, r[q]);
-            vload<T, VEC>(X + (int64_t)u[q] * xld + c0, x[q]);
-            if (XC) vload<float, VEC>(XC + (int64_t)u[q] * xld + c0, xc[q]);
-            df[q] = g.degf[u[q]];
-            dd[q] = dint ? 0.0 : g.degd[u[q]];
-            nf[q] = ign ? g.nfac[u[q]] : 0.0;
-            rd[q] = rdiv ? rdiv[u[q]] : 0.0;
-            len[q] = lone ? g.row_len[u[q]] : 2;
-        }
+        for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
+        const int di = u >= 0 ? (int)df : 0;
+        if (u >= 0) {
+            const double base64 = ign ? nf : (dint ? (double)df : g.degd[u]);
+            const float base_f = ign ? (float)base64 : df;
+            const double thr64 = F64 && !all ? scale0 * base64 : 0.0;
 #pragma unroll
-        for (int q = 0; q < Q; ++q) {
-            bool any = false, absorb = false;
-            Vec<T, VEC> push;
+            for (int k = 0; k < VEC; ++k) {
+                auto exact = [&] {
+                    const double th = sh.col_theta[c0 + k] * base64;
+                    return hk ? (th / (double)sh.tp.n_levels) / sh.psi : th;
+                };
+                bool ge;
+                if (all) ge = r.v[k] != T(0);
+                else if (f32) ge = ge_band(fabsf((float)r.v[k]), thr_f[k] * base_f, exact);
+                else if (hk) ge = ge_band64((double)r.v[k],
+                                            same ? thr64 : (sh.col_theta[c0 + k] / hk_div) * base64, exact);
+                else ge = ge_abs64((double)r.v[k], F64 && same ? thr64 : sh.col_theta[c0 + k] * base64);
+                act |= ge ? 1u << k : 0u;
+            }
+            act &= live;
+            if (act && lone && len <= 1 && (len == 0 || g.col[g.row_ptr[u]] == u)) {
+                absorb = true;  // (a zero residual has nothing to absorb)
 #pragma unroll
-            for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
-            const int di = valid[q] ? (int)df[q] : 0;
-            double du = 0.0;
-            if (valid[q]) {
-                du = dint ? (double)df[q] : dd[q];
-                const double thr_base = ign ? nf[q] : du;
-                const float base_f = ign ? (float)thr_base : df[q];
-                const double thr64 = f32 ? 0.0 : scale0 * thr_base;
-                bool act[VEC];
+                for (int k = 0; k < VEC; ++k)
+                    if (r.v[k] == T(0)) act &= ~(1u << k);
+            }
+            if (act) {
+                const float div_f = katz ? 1.f : (ign ? (float)g.npush[u] : df);
+                const double per = F64 || !f32
+                                       ? coef * (rdiv ? rd : katz ? 1.0 : 1.0 / (ign ? g.npush[u] : base64))
+                                       : 0.0;
 #pragma unroll
                 for (int k = 0; k < VEC; ++k) {
-                    act[k] = false;
-                    if (!live[k]) continue;
-                    auto hk_thr = [&] { return ((theta[k] * thr_base) / (double)sh.tp.n_levels) / sh.psi; };
-                    if (global) act[k] = r[q].v[k] != T(0);
-                    else if (f32)
-                        act[k] = ge_band(fabsf((float)r[q].v[k]), thr_f[k] * base_f,
-                                         [&] { return hk ? hk_thr() : theta[k] * thr_base; });
-                    else if (hk)
-                        act[k] = ge_band64((double)r[q].v[k], same ? thr64 : (theta[k] / hk_div) * thr_base, hk_thr);
-                    else act[k] = ge_abs64((double)r[q].v[k], same ? thr64 : theta[k] * thr_base);
-                    any |= act[k];
-                }
-                if (any && lone) {
-                    absorb = len[q] == 0 || (len[q] == 1 && g.col[g.row_ptr[u[q]]] == u[q]);
+                    if (!(act >> k & 1)) continue;
+                    const T rk = r.v[k];
+                    r.v[k] = T(0);
+                    sum.nodes[k] += 1;
                     if (absorb) {
-                        // (a zero residual has nothing to absorb)
-                        any = false;
-#pragma unroll
-                        for (int k = 0; k < VEC; ++k) {
-                            act[k] = act[k] && r[q].v[k] != T(0);
-                            any |= act[k];
-                        }
+                        // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
+                        x.v[k] = rk;
+                        if (!F64 && XC) xc.v[k] = 0.f;
+                        continue;
+                    }
+                    if (f32) push.v[k] = (T)((coef_f * (float)rk) / div_f);
+                    else push.v[k] = (T)(per * (double)rk);
+                    const T xadd = gain * rk;
+                    if (dint) sum.deg[k] += di;
+                    else sum.oper[k] += g.degd[u];
+                    if (!F64 && XC) {
+                        // Kahan-compensated FP32 accumulation of the solution
+                        const float y = (float)xadd - xc.v[k];
+                        const float s = (float)x.v[k] + y;
+                        xc.v[k] = (s - (float)x.v[k]) - y;
+                        x.v[k] = (T)s;
+                    } else {
+                        x.v[k] = x.v[k] + xadd;
                     }
                 }
-                if (any) {
-                    const float div_f = (f32 && ign) ? (float)g.npush[u[q]] : df[q];
-                    const double gain = (hk ? hkc : 1. - alpha) * rd[q];  // the push per unit of residual
-#pragma unroll
-                    for (int k = 0; k < VEC; ++k) {
-                        if (!act[k]) continue;
-                        const T rk = r[q].v[k];
-                        T pv, xadd;
-                        if (f32) {
-                            const float rf = (float)rk;
-                            pv = (T)(kind == KIND_KATZ ? alpha_f * rf
-                                     : (hk ? (sh.final_level ? rf : hkc_f * rf) : omalpha_f * rf) / div_f);
-                            xadd = (ign && !absorb) ? (T)(xgain_f * rf) : rk;
-                        } else {
-                            const double rv = (double)rk;
-                            if (rdiv) pv = (T)(gain * rv);
-                            else if (kind == KIND_KATZ) pv = (T)(alpha * rv);
-                            else pv = (T)((hk ? (sh.final_level ? rv : hkc * rv) : (1. - alpha) * rv) /
-                                          (ign ? g.npush[u[q]] : du));
-                            xadd = (ign && !absorb) ? (T)(x_gain * rv) : rk;
-                        }
-                        push.v[k] = absorb ? T(0) : pv;
-                        r[q].v[k] = T(0);
-                        sum.nodes[k] += 1;
-                        if (absorb) {
-                            // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
-                            x[q].v[k] = xadd;
-                            if (XC) xc[q].v[k] = 0.f;
-                            continue;
-                        }
-                        if (dint) sum.deg[k] += di;
-                        else sum.oper[k] += du;
-                        if (XC) {
-                            // Kahan-compensated FP32 accumulation of the solution
-                            const float y = (float)xadd - xc[q].v[k];
-                            const float s = (float)x[q].v[k] + y;
-                            xc[q].v[k] = (s - (float)x[q].v[k]) - y;
-                            x[q].v[k] = (T)s;
-                        } else {
-                            x[q].v[k] = x[q].v[k] + xadd;
-                        }
-                    }
-                    vstore<T, VEC>(R + (int64_t)u[q] * a.ld + c0, r[q]);
-                    vstore<T, VEC>(X + (int64_t)u[q] * xld + c0, x[q]);
-                    if (XC) vstore<float, VEC>(XC + (int64_t)u[q] * xld + c0, xc[q]);
+                if (act) {
+                    vstore<T, VEC>(R + (int64_t)u * a.ld, r);
+                    vstore<T, VEC>(X + (int64_t)u * xld, x);
+                    if (!F64 && XC) vstore<float, VEC>(XC + (int64_t)u * xld, xc);
                 }
-            }
-            // the node pushes when any of its columns does (OR over the lane group)
-            const unsigned bal = __ballot_sync(kFull, any);
-            if (bal == 0) continue;  // warp-uniform
-            const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
-            const bool node_in = valid[q] && (bal & gmask) != 0 && !absorb;
-            if (node_in) vstore<T, VEC>(Pw + (int64_t)u[q] * W + c0, push);
-            const bool in = lane_g == 0 && node_in;
-            if (in) {
-                if (dint) sum.ivol += di;
-                else sum.vol += du;
-                sum.cnt += 1;
-            }
-            if (sh.dense) {
-                // consecutive nodes: their bits lie in two words at most
-                const int w0 = (int)((base + q * GPW) >> 5);
-                const uint32_t bit = in ? 1u << (u[q] & 31) : 0u;
-                const uint32_t b0 = __reduce_or_sync(kFull, (u[q] >> 5) == w0 ? bit : 0u);
-                const uint32_t b1 = __reduce_or_sync(kFull, (u[q] >> 5) == w0 ? 0u : bit);
-                if (lane == 0 && b0) atomicOr(bits + w0, b0);
-                if (lane == 0 && b1) atomicOr(bits + w0 + 1, b1);
-            } else if (in) {
-                atomicOr(bits + (u[q] >> 5), 1u << (u[q] & 31));
             }
         }
+        // the node pushes when any of its columns does (OR over the lane group)
+        const unsigned bal = __ballot_sync(kFull, act != 0);
+        if (bal == 0) continue;  // warp-uniform
+        const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
+        const bool node_in = u >= 0 && (bal & gmask) != 0 && !absorb;
+        if (node_in) vstore<T, VEC>(Pw + (int64_t)u * W, push);
+        const bool in = c0 == 0 && node_in;
+        if (in) {
+            if (dint) sum.ivol += di;
+            else sum.vol += g.degd[u];
+            sum.cnt += 1;
+        }
+        if (sh.dense) {
+            // consecutive nodes: their bits lie in two words at most
+            const int w0 = (int)(base >> 5);
+            const uint32_t bit = in ? 1u << (u & 31) : 0u;
+            const uint32_t b0 = __reduce_or_sync(kFull, (u >> 5) == w0 ? bit : 0u);
+            const uint32_t b1 = __reduce_or_sync(kFull, (u >> 5) == w0 ? 0u : bit);
+            if (lane == 0 && b0) atomicOr(bits + w0, b0);
+            if (lane == 0 && b1) atomicOr(bits + w0 + 1, b1);
+        } else if (in) {
+            atomicOr(bits + (u >> 5), 1u << (u & 31));
+        }
     }
+    total = sum;
 }
 
 // PREP of any tile and round: tests each candidate per column, then compacts
