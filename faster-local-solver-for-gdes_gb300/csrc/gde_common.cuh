@@ -180,7 +180,8 @@ struct OnlineSlot {           // the query a slot holds (copied out of the ring 
 struct alignas(128) TileState {  // device-updated
     int cand_cnt[3];          // candidate list sizes (by level mod 3)
     int front_cnt[2];         // frontier sizes (by parity)
-    int small_cnt[2], med_cnt[2], large_cnt[2];
+    int large_cnt[2];         // chunks of long rows
+    unsigned long long row_cnt[2];  // short rows | medium rows << 32
     int dense_next[2];        // 1: the PREP of that parity scans all nodes
     int pull[2];              // 1: the round of that parity pulls (push values by node, rows gather them)
     int t0;                   // launch iteration at which the tile's level 0 ran
@@ -300,12 +301,12 @@ struct GridBarrier {
 
 // A piece of push work: `len` edges of one frontier row starting at col[rp]
 // (a whole short/medium row, or one chunk of a long row), and the row's
-// frontier index (its push values are P[fidx][0..W)).  One-column tiles pack
+// node (its push values are P[node][0..W)).  One-column tiles pack
 // start, length and push value into the same 16 bytes instead (pack_item).
 struct PushItem {
     long long rp;
     int len;
-    int fidx;
+    int node;
 };
 
 // Engine launch parameters (passed by value to the persistent kernel).

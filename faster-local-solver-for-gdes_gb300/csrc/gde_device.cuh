@@ -95,10 +95,10 @@ __device__ __forceinline__ PushItem pack_item(long long rp, int len, T push) {
     it.rp = rp | ((long long)len << 40);
     if constexpr (sizeof(T) == 8) {
         it.len = __double2hiint(push);
-        it.fidx = __double2loint(push);
+        it.node = __double2loint(push);
     } else {
         it.len = 0;
-        it.fidx = __float_as_int(push);
+        it.node = __float_as_int(push);
     }
     return it;
 }
@@ -106,8 +106,8 @@ template <typename T>
 __device__ __forceinline__ T unpack_item(const PushItem& it, long long& rp, int& len) {
     rp = it.rp & ((1ll << 40) - 1);
     len = (int)((unsigned long long)it.rp >> 40);
-    if constexpr (sizeof(T) == 8) return __hiloint2double(it.len, it.fidx);
-    else return __int_as_float(it.fidx);
+    if constexpr (sizeof(T) == 8) return __hiloint2double(it.len, it.node);
+    else return __int_as_float(it.node);
 }
 
 // Append v to a candidate list once per stamp (mark dedup), one atomic per

@@ -206,7 +206,6 @@ __device__ __forceinline__ double* rh_ptr(const PushArgs& a, int t) {
 // Per-tile data staged in shared memory at the start of each tile's phase.
 struct TileSh {
     TileParams tp;
-    int cand_cnt, front_cnt, small_cnt, med_cnt, large_cnt;
     int dense, pull, parity, level, stamp, m3;
     double psi;             // HK: psi[level]
     double coef1, coef2;    // Chebyshev coefficients of this round
@@ -250,11 +249,6 @@ __device__ void load_tile(const PushArgs& a, int t, int it, TileSh& sh) {
         int par = sh.level & 1;
         sh.parity = par;
         sh.m3 = sh.level % 3;
-        sh.cand_cnt = ts.cand_cnt[sh.m3];
-        sh.front_cnt = ts.front_cnt[par];
-        sh.small_cnt = ts.small_cnt[par];
-        sh.med_cnt = ts.med_cnt[par];
-        sh.large_cnt = ts.large_cnt[par];
         sh.dense = ts.dense_next[par];
         sh.pull = ts.pull[par];
         sh.stamp = ts.stamp + sh.level + 1;
@@ -567,6 +561,25 @@ struct PrepSh {
     double acc_col_vol, acc_union_vol;
 };
 
+// Room in tile ts's item lists of parity par for the warp's short rows, medium
+// rows and chunks (warp-uniform counts): one 64-bit atomic for the two row
+// counts, whose same-address updates by every warp of a tile are the limit of
+// a large frontier's compaction, and a second only for chunks.
+__device__ __forceinline__ void reserve_items(TileState& ts, int par, int small, int med, int chunks, int& b1, int& b2,
+                                              int& b3) {
+    unsigned long long rows = 0;
+    b3 = 0;
+    if ((threadIdx.x & 31) == 0) {
+        if (small | med)
+            rows = atomicAdd(&ts.row_cnt[par], ((unsigned long long)(unsigned)med << 32) | (unsigned)small);
+        if (chunks) b3 = atomicAdd(&ts.large_cnt[par], chunks);
+    }
+    rows = __shfl_sync(kFull, rows, 0);
+    b1 = (int)(unsigned)rows;
+    b2 = (int)(rows >> 32);
+    b3 = __shfl_sync(kFull, b3, 0);
+}
+
 // Frontier compaction of one node per lane (W = 1): degree bucket and work
 // items, which carry the push value.
 template <typename T>
@@ -592,16 +605,8 @@ __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, 
         if (lane >= o) sc += y;
     }
     const int wch = __shfl_sync(kFull, sc, 31);
-    int b1 = 0, b2 = 0, b3 = 0;
-    if (lane == 0) {
-        atomicAdd(&ts.front_cnt[par], __popc(bf));
-        if (bs) b1 = atomicAdd(&ts.small_cnt[par], __popc(bs));
-        if (bm) b2 = atomicAdd(&ts.med_cnt[par], __popc(bm));
-        if (wch) b3 = atomicAdd(&ts.large_cnt[par], wch);
-    }
-    b1 = __shfl_sync(kFull, b1, 0);
-    b2 = __shfl_sync(kFull, b2, 0);
-    b3 = __shfl_sync(kFull, b3, 0);
+    int b1, b2, b3;
+    reserve_items(ts, par, __popc(bs), __popc(bm), wch, b1, b2, b3);
     if (!node_in) return;
     const unsigned below = (1u << lane) - 1u;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;
@@ -1221,24 +1226,13 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
             if (lane >= o) sc += y;
         }
         const int wch = __shfl_sync(kFull, sc, 31);
-        int b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-        if (lane == 0) {
-            b0 = atomicAdd(&ts.front_cnt[par], __popc(bf));
-            if (bs) b1 = atomicAdd(&ts.small_cnt[par], __popc(bs));
-            if (bm) b2 = atomicAdd(&ts.med_cnt[par], __popc(bm));
-            if (wch) b3 = atomicAdd(&ts.large_cnt[par], wch);
-        }
-        b0 = __shfl_sync(kFull, b0, 0);
-        b1 = __shfl_sync(kFull, b1, 0);
-        b2 = __shfl_sync(kFull, b2, 0);
-        b3 = __shfl_sync(kFull, b3, 0);
+        int b1, b2, b3;
+        reserve_items(ts, par, __popc(bs), __popc(bm), wch, b1, b2, b3);
         const unsigned below = (1u << lane) - 1u;
-        int fidx = 0;
         if (leader && node_in) {
-            fidx = b0 + __popc(bf & below);
             auto item_of = [&](long long at, int edges) {
                 if constexpr (W == 1) return pack_item<T>(at, edges, push.v[0]);
-                else return PushItem{at, edges, fidx};
+                else return PushItem{at, edges, u};
             };
             if (bucket == 0) bsmall[b1 + __popc(bs & below)] = item_of(rp, len);
             else if (bucket == 1) bmed_end[-(b2 + __popc(bm & below))] = item_of(rp, len);
@@ -1252,8 +1246,7 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
             sum.cnt += 1;
         }
         if constexpr (W > 1) {
-            fidx = __shfl_sync(kFull, fidx, grp_w * L);
-            if (node_in) vstore<T, VEC>(Pw + (int64_t)fidx * W + c0, push);
+            if (node_in) vstore<T, VEC>(Pw + (int64_t)u * W + c0, push);
         }
     }
     total = sum;
@@ -1313,7 +1306,7 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
     }
     if (threadIdx.x == 0 && ps.nodes) {
         atomicAdd(&ts.union_vol[par], ps.vol);
-        if (PULL && sh.pull) atomicAdd(&ts.front_cnt[par], ps.nodes);  // push rounds count while they compact
+        atomicAdd(&ts.front_cnt[par], ps.nodes);
         ps.acc_union_nodes += (unsigned long long)ps.nodes;
         ps.acc_union_vol += ps.vol;
     }
@@ -1329,8 +1322,7 @@ __device__ void zero_next_counters(const PushArgs& a, int t, int level) {
     if (threadIdx.x == 0) {
         ts.cand_cnt[(level + 2) % 3] = 0;
         ts.front_cnt[np] = 0;
-        ts.small_cnt[np] = 0;
-        ts.med_cnt[np] = 0;
+        ts.row_cnt[np] = 0;
         ts.large_cnt[np] = 0;
         ts.union_vol[np] = 0.0;
     }
@@ -1527,7 +1519,7 @@ __device__ __forceinline__ void scatter_item(const PushArgs& a, const ScatterCtx
     float theta_f[VEC];
     load_thetas<T, VEC>(c.cs, c0, c.cross, theta, theta_f);
     Vec<T, VEC> p;
-    vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
+    vload<T, VEC>(c.Pw + (int64_t)it.node * W + c0, p);
     const int end = min(it.len, beg + edges);
     for (int j0 = beg; j0 < end; j0 += GPW) {
         const int j = j0 + grp_w;
@@ -1821,7 +1813,7 @@ __device__ void scatter_short(const PushArgs& a, const PushItem* items, const Sc
         const PushItem it = items[grp_w];
         rp = it.rp;
         len = it.len;
-        vload<T, VEC>(c.Pw + (int64_t)it.fidx * W + c0, p);
+        vload<T, VEC>(c.Pw + (int64_t)it.node * W + c0, p);
     }
     // edge offsets by group: each group's first lane carries its row length
     int incl = (lane_g == 0) ? len : 0;
@@ -1891,8 +1883,8 @@ __device__ void scatter_units(const PushArgs& a, int ntl, const GroupInfo& gi) {
             edges = split ? piece_edges<T, W>() : 1 << 24;
             sr = (split && SR >= 4) ? SR / 4 : SR;
             nl = a.ts[t].large_cnt[par] * cl;
-            nm = a.ts[t].med_cnt[par] * cm;
-            ns = a.ts[t].small_cnt[par];
+            nm = (int)(a.ts[t].row_cnt[par] >> 32) * cm;
+            ns = (int)(unsigned)a.ts[t].row_cnt[par];
             bsmall = a.bsmall + (int64_t)t * a.g.n;
             blarge = a.blarge + (int64_t)t * a.large_cap;
             if (W == 1) theta = c.cross ? c.cs[0].theta : 0.0;
@@ -2313,7 +2305,8 @@ __device__ void admit_query(const PushArgs& a, int t, int it) {
     ts.stamp = ts.stamp + (it - ts.t0) + 2;
     for (int i = 0; i < 3; ++i) ts.cand_cnt[i] = 0;
     for (int i = 0; i < 2; ++i) {
-        ts.front_cnt[i] = ts.small_cnt[i] = ts.med_cnt[i] = ts.large_cnt[i] = 0;
+        ts.front_cnt[i] = ts.large_cnt[i] = 0;
+        ts.row_cnt[i] = 0;
         ts.dense_next[i] = ts.pull[i] = 0;
         ts.union_vol[i] = 0.0;
     }
@@ -2510,7 +2503,8 @@ __device__ bool admit_online(const PushArgs& a, int t, int it) {
     ts.stamp = ts.stamp + max(it - ts.t0, 0) + 2;
     for (int i = 0; i < 3; ++i) ts.cand_cnt[i] = 0;
     for (int i = 0; i < 2; ++i) {
-        ts.front_cnt[i] = ts.small_cnt[i] = ts.med_cnt[i] = ts.large_cnt[i] = 0;
+        ts.front_cnt[i] = ts.large_cnt[i] = 0;
+        ts.row_cnt[i] = 0;
         ts.dense_next[i] = ts.pull[i] = 0;
         ts.union_vol[i] = 0.0;
     }
@@ -3019,11 +3013,12 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
                     const int par = sl[k].level & 1;
                     constexpr int SR = short_rows<T, W>();
                     if (!pushes(k)) return 0;
-                    const long long nl = ts.large_cnt[par], nm = ts.med_cnt[par];
-                    const long long ns = (ts.small_cnt[par] + SR - 1) / SR;
+                    const long long nl = ts.large_cnt[par], nm = (long long)(ts.row_cnt[par] >> 32);
+                    const long long rows = (long long)(unsigned)ts.row_cnt[par];
+                    const long long ns = (rows + SR - 1) / SR;
                     constexpr int SP = SR >= 4 ? SR / 4 : 1;
                     const long long cut = nl * pieces<T, W>(a.chunk) + nm * pieces<T, W>(a.med_max) +
-                                          (ts.small_cnt[par] + SP - 1) / SP;
+                                          (rows + SP - 1) / SP;
                     sl[k].split = cut * ntl <= 4ll * gi.dim * kWarps;
                     return sl[k].split ? cut : nl + nm + ns;
                 });
