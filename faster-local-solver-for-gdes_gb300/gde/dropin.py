@@ -3,63 +3,77 @@
 The reference's functions take numpy CSR arrays on every call and its GPU
 path uploads them each time (``ppr_solver.py:103-105``).  Here a graph is
 uploaded once and reused while the caller passes arrays with the same
-contents.  The key is a CRC-32 of every byte of ``indptr``, ``indices`` and
-``degree`` (plus shapes and dtypes), so an in-place edit of any entry is
-seen and the graph is uploaded again; functions that edit the arrays
-through the library (``updeta_graph``, ``updetaGraph``, the dynamic
-updates) re-key the resident graph instead, since its device copy already
-holds the edit.
+contents.  Each resident graph keeps a host copy of the bytes it was
+uploaded from, and a call's ``indptr``, ``indices`` and ``degree`` are
+compared with it (``memcmp``: 4.2 MB in 0.15 ms, a CRC-32 of them took 0.9 ms
+of a 2.2 ms call on an 87k-node graph), so an in-place edit of any entry is
+seen and the graph is uploaded again; functions that edit the arrays through
+the library (``updeta_graph``, ``updetaGraph``, the dynamic updates) re-key
+the resident graph instead, since its device copy already holds the edit.
 """
 from __future__ import annotations
 
+import ctypes
 import time
-import zlib
 
 import numpy as np
 
 from . import api
 
-_CACHE: dict = {}
-_MAX = 4
+_MAX = 4                # resident graphs
+_CACHE: list = []       # (contents, graph), oldest first
+_memcmp = ctypes.CDLL(None).memcmp
+_memcmp.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t]
+_memcmp.restype = ctypes.c_int
 
 
-def _fingerprint(a) -> tuple:
-    a = np.ascontiguousarray(a)
-    return (a.shape, str(a.dtype), zlib.crc32(memoryview(a).cast("B")) if a.size else 0)
+class _Contents:
+    """The arrays a graph was uploaded from: their shapes, types and every byte."""
+
+    def __init__(self, arrays, padded: bool):
+        self.padded = padded
+        self.arrays = [None if a is None else np.array(a, order="C") for a in arrays]
+
+    def equal(self, arrays, padded: bool) -> bool:
+        if padded != self.padded:
+            return False
+        for a, b in zip(arrays, self.arrays):
+            if (a is None) != (b is None) or (a is not None and (a.shape != b.shape or a.dtype != b.dtype)):
+                return False
+        return all(a is None or a.nbytes == 0 or _memcmp(a.ctypes.data, b.ctypes.data, a.nbytes) == 0
+                   for a, b in zip(arrays, self.arrays))
 
 
-def _key(indptr, indices, degree, padded: bool) -> tuple:
-    return (_fingerprint(indptr), _fingerprint(indices), None if degree is None else _fingerprint(degree), padded)
+def _arrays(indptr, indices, degree) -> list:
+    return [None if a is None else np.ascontiguousarray(a) for a in (indptr, indices, degree)]
 
 
 def graph_for(indptr, indices, degree=None, padded: bool = False) -> api.Graph:
     """Resident graph for these numpy arrays (uploaded on first use or when their contents change)."""
+    arrays = _arrays(indptr, indices, degree)
+    for contents, g in reversed(list(_CACHE)):
+        if contents.equal(arrays, padded):
+            return g
+    while len(_CACHE) >= _MAX:
+        _CACHE.pop(0)
     deg = None if degree is None else np.asarray(degree)
-    key = _key(indptr, indices, deg, padded)
-    g = _CACHE.get(key)
-    if g is not None:
-        return g
-    if len(_CACHE) >= _MAX:
-        _CACHE.pop(next(iter(_CACHE)))
     if padded:
         g = api.Graph(indptr, indices, row_len=np.asarray(degree, dtype=np.int64),
                       degree=np.asarray(degree, dtype=np.float64))
     else:
         g = api.Graph(indptr, indices, degree=None if deg is None else deg.astype(np.float64))
-    _CACHE[key] = g
+    _CACHE.append((_Contents(arrays, padded), g))
     return g
 
 
 def forget(g: api.Graph) -> None:
-    for k, v in list(_CACHE.items()):
-        if v is g:
-            del _CACHE[k]
+    _CACHE[:] = [e for e in _CACHE if e[1] is not g]
 
 
 def rekey(g: api.Graph, indptr, indices, degree, padded: bool = True) -> None:
     """The caller's arrays were edited through the library: ``g`` (already edited on the device) is their graph."""
     forget(g)
-    _CACHE[_key(indptr, indices, None if degree is None else np.asarray(degree), padded)] = g
+    _CACHE.append((_Contents(_arrays(indptr, indices, degree), padded), g))
 
 
 def oper_like(degree, value: float):
