@@ -7,7 +7,7 @@
 namespace gde {
 
 // Persistent push engine (push_engine.cu).
-// (max_grid goes by the launch's ntiles, groups and pull_div: they are set before it)
+// (max_grid goes by the launch's ntiles, groups, pull_div and serve: they are set before it)
 int engine_max_grid(const PushArgs& a, int prec64, int W, int sms);
 cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st);
 

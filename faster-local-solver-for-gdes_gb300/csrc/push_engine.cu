@@ -52,8 +52,8 @@ namespace {
 #ifndef GDE_MIN_BLOCKS_W1
 #define GDE_MIN_BLOCKS_W1 5
 #endif
-#ifndef GDE_VEC_COLS
-#define GDE_VEC_COLS 0  // 1: 128-bit column-word loads for rows of 128 edges and more (W = 1)
+#ifndef GDE_MIN_BLOCKS_SERVE64
+#define GDE_MIN_BLOCKS_SERVE64 4
 #endif
 #ifndef GDE_EDGE_ILP
 #define GDE_EDGE_ILP 2
@@ -2873,13 +2873,11 @@ __device__ __forceinline__ void trace_point(const PushArgs& a, int it, int k) {
         a.trace[((size_t)it * gridDim.x + blockIdx.x) * kTracePoints + k] = globaltimer_ns();
 }
 
-// PULL: the launch may pull (a.pull_div > 0).  One-column launches that never
-// do run an instantiation without that code: its registers cost the served
-// FP32 slots 4%.
-template <typename T, int W, bool PULL>
-__global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_MIN_BLOCKS_W1
-                                           : (W <= 8 && sizeof(T) == 4) ? GDE_MIN_BLOCKS_F32
-                                                                        : GDE_MIN_BLOCKS)
+// PULL: the launch may pull (a.pull_div > 0); one-column launches that never
+// do run an instantiation without that code.  MB: blocks per SM asked of the
+// compiler.
+template <typename T, int W, bool PULL, int MB>
+__global__ void __launch_bounds__(kThreads, MB)
     push_kernel(const __grid_constant__ PushArgs a) {
     __shared__ TileSh sh;
     __shared__ PrepSh ps;
@@ -3182,60 +3180,52 @@ __global__ void __launch_bounds__(kThreads, (W == 1 && sizeof(T) == 4)   ? GDE_M
 
 }  // namespace
 
-// Host-side launcher: picks the instantiation for (T, W, PULL) and launches
-// it cooperatively with the largest co-resident grid.
 static size_t tiles_smem(int ntiles, int groups) {
     const int G = groups > 1 ? groups : 1;
     return (size_t)((ntiles + G - 1) / G + 1) * sizeof(TileSlot);
 }
 
-template <typename T, int W, bool PULL>
-static int max_grid_t(int sms, size_t smem) {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, push_kernel<T, W, PULL>, kThreads, smem);
-    return per_sm * sms;
+using PushKernel = void (*)(const PushArgs);
+
+template <typename T, int W>
+constexpr int min_blocks() {
+    return (W == 1 && sizeof(T) == 4) ? GDE_MIN_BLOCKS_W1 : (W <= 8 && sizeof(T) == 4) ? GDE_MIN_BLOCKS_F32 : GDE_MIN_BLOCKS;
 }
 
-template <typename T, int W, bool PULL>
-static cudaError_t launch_t(const PushArgs& a, int grid, cudaStream_t st) {
-    void* args[] = {const_cast<PushArgs*>(&a)};
-    return cudaLaunchCooperativeKernel((void*)push_kernel<T, W, PULL>, dim3(grid), dim3(kThreads), args,
-                                       tiles_smem(a.ntiles, a.groups), st);
-}
-
+// The instantiation of a launch.  Served FP64 slots take a fourth block per
+// SM (50 queries on 87k nodes 6.7 -> 6.3 ms, the R-MAT mix 72 -> 66): their
+// PPR and Katz rounds have the registers for it, the general rounds of other
+// one-column FP64 launches spill (InstantGNN, one column: 6.5 -> 7.3 ms).
 template <typename T>
-static int max_grid_w(int W, bool pull, int sms, size_t smem) {
+static PushKernel kernel_of(const PushArgs& a, int W) {
+    constexpr int MB1 = min_blocks<T, 1>(), MBS = sizeof(T) == 8 ? GDE_MIN_BLOCKS_SERVE64 : MB1;
     switch (W) {
-        case 1: return pull ? max_grid_t<T, 1, true>(sms, smem) : max_grid_t<T, 1, false>(sms, smem);
-        case 2: return max_grid_t<T, 2, true>(sms, smem);
-        case 4: return max_grid_t<T, 4, true>(sms, smem);
-        case 8: return max_grid_t<T, 8, true>(sms, smem);
-        case 16: return max_grid_t<T, 16, true>(sms, smem);
-        case 32: return max_grid_t<T, 32, true>(sms, smem);
+        case 1:
+            if (a.serve) return a.pull_div > 0 ? push_kernel<T, 1, true, MBS> : push_kernel<T, 1, false, MBS>;
+            return a.pull_div > 0 ? push_kernel<T, 1, true, MB1> : push_kernel<T, 1, false, MB1>;
+        case 2: return push_kernel<T, 2, true, min_blocks<T, 2>()>;
+        case 4: return push_kernel<T, 4, true, min_blocks<T, 4>()>;
+        case 8: return push_kernel<T, 8, true, min_blocks<T, 8>()>;
+        case 16: return push_kernel<T, 16, true, min_blocks<T, 16>()>;
+        case 32: return push_kernel<T, 32, true, min_blocks<T, 32>()>;
     }
-    return 0;
-}
-
-template <typename T>
-static cudaError_t launch_w(const PushArgs& a, int W, int grid, cudaStream_t st) {
-    switch (W) {
-        case 1: return a.pull_div > 0 ? launch_t<T, 1, true>(a, grid, st) : launch_t<T, 1, false>(a, grid, st);
-        case 2: return launch_t<T, 2, true>(a, grid, st);
-        case 4: return launch_t<T, 4, true>(a, grid, st);
-        case 8: return launch_t<T, 8, true>(a, grid, st);
-        case 16: return launch_t<T, 16, true>(a, grid, st);
-        case 32: return launch_t<T, 32, true>(a, grid, st);
-    }
-    return cudaErrorInvalidValue;
+    return nullptr;
 }
 
 int engine_max_grid(const PushArgs& a, int prec64, int W, int sms) {
-    const size_t smem = tiles_smem(a.ntiles, a.groups);
-    return prec64 ? max_grid_w<double>(W, a.pull_div > 0, sms, smem) : max_grid_w<float>(W, a.pull_div > 0, sms, smem);
+    const PushKernel k = prec64 ? kernel_of<double>(a, W) : kernel_of<float>(a, W);
+    int per_sm = 0;
+    if (!k || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, tiles_smem(a.ntiles, a.groups)) !=
+                  cudaSuccess)
+        return 0;
+    return per_sm * sms;
 }
 
 cudaError_t engine_launch(const PushArgs& a, int prec64, int W, int grid, cudaStream_t st) {
-    return prec64 ? launch_w<double>(a, W, grid, st) : launch_w<float>(a, W, grid, st);
+    const PushKernel k = prec64 ? kernel_of<double>(a, W) : kernel_of<float>(a, W);
+    if (!k) return cudaErrorInvalidValue;
+    void* args[] = {const_cast<PushArgs*>(&a)};
+    return cudaLaunchCooperativeKernel((void*)k, dim3(grid), dim3(kThreads), args, tiles_smem(a.ntiles, a.groups), st);
 }
 
 }  // namespace gde

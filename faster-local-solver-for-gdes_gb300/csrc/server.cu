@@ -279,6 +279,7 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
     // ---- device workspace: S one-column slots ----
     PushArgs& a = s->a;
     a = base;
+    a.serve = 1;
     a.g = G->g;
     a.ntiles = S;
     a.ld = 1;
@@ -361,7 +362,6 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
             return rc;
         }
     }
-    a.serve = 1;
     a.round_budget = 0x7fffffff;
     // ---- heat-kernel psi tables for every Taylor length the server accepts ----
     std::vector<double> psi_all;
