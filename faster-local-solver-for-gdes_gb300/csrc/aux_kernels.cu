@@ -165,6 +165,34 @@ __global__ void query_rows_scatter_kernel(const float* XI, int64_t xtile, const 
     }
 }
 
+// Solves on a merged graph: the entry of a seed that has twins.  Round 0 moved
+// its residual r0 into its own solution only (rounds > 0), or left it there as
+// its own residual only; the rows hold the merged node's values for all twins.
+// The seed's entry is formed in FP64 from the interleaved {x, c} slab where the
+// rows came from one (XI), else from the row.
+template <typename O>
+__global__ void seed_entries_kernel(const SeedFix* fix, int nf, const int* rounds, int64_t rstride, const float* XI,
+                                    int64_t xtile, const int32_t* perm, int64_t n, O* x_out, O* r_out,
+                                    int64_t ld_out) {
+    for (int i = blockIdx.y; i < nf; i += gridDim.y) {
+        const SeedFix f = fix[i];
+        const int ran = *reinterpret_cast<const int*>(reinterpret_cast<const char*>(rounds) + f.col * rstride);
+        if (x_out && blockIdx.x == 0 && threadIdx.x == 0) {
+            O* e = x_out + f.row * ld_out + f.seed;
+            double x = (double)*e * f.scale;
+            if (XI) {
+                const float2 xc = *reinterpret_cast<const float2*>(XI + f.row * xtile + 2 * (int64_t)f.node);
+                x = (double)xc.x - (double)xc.y;
+            }
+            *e = (O)((x + (ran > 0 ? f.r0 : 0.0)) / f.scale + f.add);
+        }
+        if (r_out && ran == 0)
+            for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n;
+                 u += (int64_t)gridDim.x * blockDim.x)
+                if (perm[u] == f.node && u != f.seed) r_out[f.row * f.r_levels * ld_out + u] = (O)0;
+    }
+}
+
 // Per-node degree tables of the nodes an edge batch touched (rec[i] for node
 // ids[i]); the InstantGNN tables only when nf is given.
 __global__ void node_tables_kernel(int64_t nn, const NodeTables* rec, int32_t* row_len, double* degd, float* degf,
@@ -300,6 +328,20 @@ cudaError_t query_rows(const float* XI, int64_t xtile, const int32_t* perm, cons
     else
         query_rows_kernel<float><<<blocks, 256, 0, st>>>(XI, xtile, perm, n, nq, seed_int, kinds, seed_add, hk_scale,
                                                           (float*)out, ld_out);
+    return cudaGetLastError();
+}
+
+cudaError_t seed_entries(const SeedFix* fix, int nf, const int* rounds, int64_t rstride, const float* XI,
+                         int64_t xtile, const int32_t* perm, int64_t n, void* x_out, void* r_out, int out64,
+                         int64_t ld_out, cudaStream_t st) {
+    if (nf == 0 || (!x_out && !r_out)) return cudaSuccess;
+    const dim3 grid(r_out ? (unsigned)std::min<int64_t>((n + 255) / 256, 512) : 1u, (unsigned)std::min(nf, 65535));
+    if (out64)
+        seed_entries_kernel<double><<<grid, 256, 0, st>>>(fix, nf, rounds, rstride, XI, xtile, perm, n, (double*)x_out,
+                                                          (double*)r_out, ld_out);
+    else
+        seed_entries_kernel<float><<<grid, 256, 0, st>>>(fix, nf, rounds, rstride, XI, xtile, perm, n, (float*)x_out,
+                                                         (float*)r_out, ld_out);
     return cudaGetLastError();
 }
 

@@ -238,14 +238,15 @@ int alloc_large(gde_ctx* ctx, gde_graph* G, int ntiles, TileWs& tw) {
 }
 
 // Pull plan of the graph's row capacities: static rows are already in
-// descending order of length; padded rows get an order by capacity (a row's
-// capacity bounds its length through every edit until a repad).
+// descending order of length; padded and merged rows get an order by capacity
+// (a row's capacity bounds its length through every edit until a repad).
 int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
     const int64_t n = G->g.n;
     std::vector<int32_t> ord;
     std::vector<int2> chunks;
+    const bool sorted = G->relabeled && !G->g.merged;  // (a merged graph's ids go by its nodes' own degrees)
     auto capacity = [&](int64_t u) { return G->h_indptr[u + 1] - G->h_indptr[u]; };
-    if (!G->relabeled) {
+    if (!sorted) {
         int64_t most = 0;
         for (int64_t u = 0; u < n; u++) most = std::max(most, capacity(u));
         std::vector<int64_t> at(most + 2, 0);
@@ -256,13 +257,13 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
     }
     int64_t i = 0;
     for (; i < n; i++) {
-        const int32_t u = G->relabeled ? (int32_t)i : ord[i];
+        const int32_t u = sorted ? (int32_t)i : ord[i];
         const int64_t c = capacity(u);
         if (c <= kPullLong) break;
         for (int64_t b = 0; b < c; b += kPullChunk) chunks.push_back(make_int2(u, (int)b));
     }
     G->g.pull_long = (int)i;
-    while (i < n && capacity(G->relabeled ? i : ord[i]) > kPullMid) i++;
+    while (i < n && capacity(sorted ? i : ord[i]) > kPullMid) i++;
     G->g.pull_mid = (int)i;
     G->g.npchunk = (int)chunks.size();
     cudaFree(G->pord);
@@ -272,7 +273,7 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
     G->g.pord = nullptr;
     G->g.pchunk = nullptr;
     if (cudaMalloc(&G->pchunk, std::max<size_t>(chunks.size(), 1) * sizeof(int2)) != cudaSuccess ||
-        (!G->relabeled && cudaMalloc(&G->pord, n * sizeof(int32_t)) != cudaSuccess)) {
+        (!sorted && cudaMalloc(&G->pord, n * sizeof(int32_t)) != cudaSuccess)) {
         cudaGetLastError();
         return fail(ctx, GDE_ENOMEM, "device memory exhausted (pull plan)");
     }
@@ -289,6 +290,7 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
 // 1/div of the graph's volume.  Needs a symmetric adjacency (checked on the
 // device, once per graph and edit) and room for the frontier bitmaps; without
 // either the launch pushes in every round.
+int check_symmetric(gde_ctx* ctx, gde_graph* G, int* yes);
 int enable_pull(gde_ctx* ctx, gde_graph* G, PushArgs& a, int W, int div) {
     a.pull_div = 0;
     const double row_cost = W == 1 ? kPullRowW1 * (double)G->g.n : 0.0;
@@ -298,16 +300,9 @@ int enable_pull(gde_ctx* ctx, gde_graph* G, PushArgs& a, int W, int div) {
         if (rc == GDE_ENOMEM) { ctx->err.clear(); return GDE_OK; }
         if (rc != GDE_OK) return rc;
     }
-    if (G->symmetric < 0) {
-        unsigned long long* sums = (unsigned long long*)wsget(ctx, "sym_sums", 16);
-        if (!sums) return GDE_OK;
-        unsigned long long h[2];
-        CK(symmetry_sums(G->g, sums, ctx->stream));
-        CK(cudaMemcpyAsync(h, sums, 16, cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-        G->symmetric = (h[0] | h[1]) == 0 ? 1 : 0;
-    }
-    if (!G->symmetric) return GDE_OK;
+    int sym = 0;
+    const int rs = check_symmetric(ctx, G, &sym);
+    if (rs != GDE_OK || !sym) return rs;
     const int64_t words = (G->g.n + 31) / 32 + 1;
     a.bits = (uint32_t*)wsget(ctx, "bits", (size_t)a.ntiles * 2 * words * 4);
     if (!a.bits) return GDE_OK;
@@ -499,7 +494,7 @@ int build_static_records(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     const int64_t n = G->g.n, cap = G->g.cap;
     std::vector<NodeRec> rec(n);
     for (int64_t u = 0; u < n; u++) {
-        rec[u].rp = G->h_indptr[u];
+        rec[u].rp = G->h_indptr[u] | ((long long)G->twins((int32_t)u) << kRowBits);
         rec[u].len = (int)G->h_len[u];
         rec[u].degf = (float)G->h_deg[u];
     }
@@ -536,6 +531,119 @@ int build_static_records(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     return GDE_OK;
 }
 
+// Is the adjacency symmetric?  (on the device, once per graph and edit;
+// *yes = 0 without memory to tell)
+int check_symmetric(gde_ctx* ctx, gde_graph* G, int* yes) {
+    *yes = 0;
+    if (G->symmetric < 0) {
+        unsigned long long* sums = (unsigned long long*)wsget(ctx, "sym_sums", 16);
+        if (!sums) return GDE_OK;
+        unsigned long long h[2];
+        CK(symmetry_sums(G->g, sums, ctx->stream));
+        CK(cudaMemcpyAsync(h, sums, 16, cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        G->symmetric = (h[0] | h[1]) == 0 ? 1 : 0;
+    }
+    *yes = G->symmetric;
+    return GDE_OK;
+}
+
+// The graph with the leaves of each node merged into one: nodes whose row is
+// the same single neighbour, with the same degree, receive the same additions
+// in every round, so from round 1 on (when a seed among them has pushed its own
+// residual away) they hold equal residuals and push together.  On the
+// wiki-talk shape 2.36M nodes and 9.4M entries become 1.53M and 7.7M, a query's
+// frontier nodes 58% and its pushes 82%.  Symmetric graphs only (an equal row
+// then means equal senders), and only where it drops a fifth of the nodes.
+int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
+    const int64_t n = G->g.n;
+    std::vector<int32_t> id(n, -1), rep, twins;  // internal id -> merged id; merged id -> its first node, its twins
+    std::vector<int32_t> leaf(n, -1);            // parent -> merged id of its leaves
+    int64_t leaves = 0;
+    for (int64_t u = 0; u < n; u++) leaves += G->h_len[u] == 1;
+    if (leaves * 5 < n) return GDE_OK;
+    rep.reserve(n);
+    twins.reserve(n);
+    for (int64_t u = 0; u < n; u++) {
+        int32_t* to = G->h_len[u] == 1 ? &leaf[col[G->h_indptr[u]]] : nullptr;
+        if (to && *to >= 0 && G->h_deg[rep[*to]] == G->h_deg[u] && twins[*to] < (1 << 22)) {
+            id[u] = *to;
+            twins[*to]++;
+            continue;
+        }
+        id[u] = (int32_t)rep.size();
+        if (to) *to = id[u];
+        rep.push_back((int32_t)u);
+        twins.push_back(0);
+    }
+    const int64_t m = (int64_t)rep.size();
+    if (m * 5 > n * 4 || G->g.cap >= (int64_t)1 << kRowBits) return GDE_OK;
+    int sym = 0;
+    int rc = check_symmetric(ctx, G, &sym);
+    if (rc != GDE_OK || !sym) return rc;
+    gde_graph* M = new gde_graph();
+    M->ctx = ctx;
+    M->relabeled = true;
+    M->symmetric = 1;  // a kept row keeps exactly the kept ones among its neighbours
+    M->deg_is_len = false;
+    M->h_perm.resize(n);
+    for (int64_t u = 0; u < n; u++) M->h_perm[u] = id[G->h_perm[u]];
+    M->h_indptr.assign(m + 1, 0);
+    M->h_len.resize(m);
+    M->h_deg.resize(m);
+    std::vector<int32_t> mcol;
+    mcol.reserve(G->g.cap);
+    for (int64_t v = 0; v < m; v++) {
+        const int64_t u = rep[v], rp = G->h_indptr[u];
+        for (int64_t j = 0; j < G->h_len[u]; j++) {
+            const int32_t w = col[rp + j];
+            if (rep[id[w]] == w) mcol.push_back(id[w]);
+        }
+        M->h_indptr[v + 1] = (int64_t)mcol.size();
+        M->h_len[v] = M->h_indptr[v + 1] - M->h_indptr[v];
+        M->h_deg[v] = G->h_deg[u];
+    }
+    M->h_twins = std::move(twins);
+    const int64_t cap = (int64_t)mcol.size();
+    M->g.n = m;
+    M->g.cap = cap;
+    M->g.merged = 1;
+    // a graph that does not fit twice is solved unmerged
+    if (cudaMalloc(&M->row_ptr, (m + 3) * sizeof(int64_t)) != cudaSuccess ||
+        cudaMalloc(&M->col, std::max<int64_t>(cap, 1) * sizeof(int32_t)) != cudaSuccess ||
+        cudaMalloc(&M->row_len, m * sizeof(int32_t)) != cudaSuccess ||
+        cudaMalloc(&M->degf, m * sizeof(float)) != cudaSuccess ||
+        cudaMalloc(&M->degd, m * sizeof(double)) != cudaSuccess ||
+        cudaMalloc(&M->perm_d, n * sizeof(int32_t)) != cudaSuccess) {
+        cudaGetLastError();
+        gde_graph_free(M);
+        return GDE_OK;
+    }
+    G->merged = M;  // (freed with G from here on)
+    CK(cudaMemsetAsync(M->row_ptr, 0, (m + 3) * sizeof(int64_t), ctx->stream));
+    CK(cudaMemcpyAsync(M->row_ptr, M->h_indptr.data(), (m + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
+    if (cap > 0) CK(cudaMemcpyAsync(M->col, mcol.data(), cap * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(M->perm_d, M->h_perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
+    M->g.perm = M->perm_d;
+    M->g.row_ptr = M->row_ptr;
+    M->g.col = M->col;
+    M->g.row_len = M->row_len;
+    M->g.degf = M->degf;
+    M->g.degd = M->degd;
+    // hubs by their own degree, as in the whole graph
+    while (M->g.hub_cut < m && G->h_len[rep[M->g.hub_cut]] > kHubLen) M->g.hub_cut++;
+    rc = upload_degrees(ctx, M);  // (waits for the copies above)
+    M->g.vol = G->g.vol;
+    if (rc == GDE_OK) rc = build_static_records(ctx, M, mcol.data());
+    if (rc == GDE_ENOMEM) {
+        ctx->err.clear();
+        gde_graph_free(M);
+        G->merged = nullptr;
+        return GDE_OK;
+    }
+    return rc;
+}
+
 // Served solve of PPR / Katz local GD: `slots` single-column tiles cycle
 // through a device queue of the nq queries inside one persistent launch.  A
 // finished query's solution row is written (caller node order) and its slot
@@ -562,6 +670,10 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
                  const double* eps, const double* arrival_ms, void* x_out, void* r_out, int out64, int out_mem,
                  int64_t ld_out, double* oper_out, int32_t* rounds_out, float* lat_ms_out, gde_stats* stats,
                  const int32_t* kinds = nullptr, const double* alphas = nullptr, double budget_bytes = 0.0) {
+    // on the graph with merged leaves where there is one (hash-table queries
+    // keep to single nodes); rows and seeds stay the caller's n_out nodes
+    const int64_t n_out = G->g.n;
+    if (G->merged && p->sparse_blocks <= 0) G = G->merged;
     const int64_t n = G->g.n;
     const int kind = p->kind;
     const int prec64 = (p->prec == GDE_FP64);
@@ -671,6 +783,7 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
     if (a.R2) CK(cudaMemsetAsync(a.R2, 0, slab, ctx->stream));
     if (a.XC && !a.xld) CK(cudaMemsetAsync(a.XC, 0, (size_t)S * n * 4, ctx->stream));
     // ---- the query queue on the device ----
+    std::vector<SeedFix> fix;  // seeds with twins in a merged graph
     std::vector<int32_t> qs(nq), qk(nq), qnl(kinds ? nq : 0), qpo(kinds ? nq : 0);
     std::vector<double> qt(nq), qr0(nq), qal(nq);
     std::vector<long long> qarr(arrival_ms ? nq : 0);
@@ -696,6 +809,9 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
             qnl[q] = (int32_t)N;
             qpo[q] = psi_at[N];
         }
+        if (G->twins(qs[q]) > 0)
+            fix.push_back(SeedFix{q, q, seeds[q], qs[q], qr0[q], k == KIND_HK ? std::exp(p->tau) : 1.0,
+                                  k == KIND_KATZ ? -1.0 : 0.0, 1});
         if (arrival_ms) qarr[q] = (long long)(arrival_ms[q] * 1e6);
     }
     auto dev = [&](const char* name, size_t bytes) { return wsget(ctx, name, std::max<size_t>(bytes, 8)); };
@@ -887,10 +1003,24 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
     rc = run_engine(ctx, a, prec64, 1, stats, &kernel_ms);
     if (rc != GDE_OK) return rc;
     // ---- results ----
+    // seeds with twins get their entries below, not the merged node's Katz correction
+    const int32_t* d_seed_add = d_seed;
+    SeedFix* d_fix = nullptr;
+    if (!fix.empty()) {
+        std::vector<int32_t> qa = qs;
+        for (const SeedFix& f : fix) qa[f.row] = -1;
+        int32_t* d_qa = (int32_t*)dev("q_seed_add", nq * 4);
+        d_fix = (SeedFix*)dev("q_fix", fix.size() * sizeof(SeedFix));
+        if (!d_qa || !d_fix) return fail(ctx, GDE_ENOMEM, "query queue");
+        CK(cudaMemcpyAsync(d_qa, qa.data(), nq * 4, cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(d_fix, fix.data(), fix.size() * sizeof(SeedFix), cudaMemcpyHostToDevice, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));  // qa is released here
+        d_seed_add = d_qa;
+    }
     // per-query solution slabs: every solution row at once, in caller order
     if (a.xq)
-        CK(query_rows((const float*)a.X, a.xtile, G->perm_d, x_direct ? nullptr : G->iperm_d, n, nq, d_seed, d_kind,
-                      Q.seed_add, Q.hk_scale, dx, out64, ld_out, ctx->stream));
+        CK(query_rows((const float*)a.X, a.xtile, G->perm_d, x_direct ? nullptr : G->iperm_d, n_out, nq, d_seed_add,
+                      d_kind, Q.seed_add, Q.hk_scale, dx, out64, ld_out, ctx->stream));
     // retired rows are in internal node order: permute them to caller order
     // through a wave buffer of a few rows (random reads stay in L2)
     if (G->perm_d) {
@@ -905,10 +1035,13 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
                 char* at = (char*)rows + (size_t)q0 * ld_out * oes;
                 CK(cudaMemcpy2DAsync(tmp, row_bytes, at, ld_out * oes, row_bytes, w, cudaMemcpyDeviceToDevice,
                                      ctx->stream));
-                CK(permute_entries(tmp, n, at, ld_out, G->perm_d, n, w, (int)oes, ctx->stream));
+                CK(permute_entries(tmp, n, at, ld_out, G->perm_d, n_out, w, (int)oes, ctx->stream));
             }
         }
     }
+    if (d_fix)
+        CK(seed_entries(d_fix, (int)fix.size(), d_rounds, sizeof(int), a.xq ? (const float*)a.X : nullptr, a.xtile,
+                        G->perm_d, n_out, dx, dr, out64, ld_out, ctx->stream));
     if (out_mem != GDE_MEM_DEVICE) {
         if (x_out && !x_direct)
             CK(cudaMemcpyAsync(x_out, dx, (size_t)nq * ld_out * oes, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1249,6 +1382,7 @@ int gde_graph_upload(gde_ctx* ctx, int64_t n, int64_t cap, const int64_t* indptr
     if (rc != GDE_OK) { gde_graph_free(G); return rc; }
     if (G->relabeled) {
         rc = build_static_records(ctx, G, col_src);
+        if (rc == GDE_OK) rc = build_merged(ctx, G, col_src);
         if (rc != GDE_OK) { gde_graph_free(G); return rc; }
     }
     *out = G;
@@ -1265,6 +1399,7 @@ int gde_graph_free(gde_graph* G) {
     cudaFree(G->pord); cudaFree(G->pchunk);
     cudaFree(G->rdeg); cudaFree(G->rnf); cudaFree(G->rtf);
     cudaFree(G->pw1); cudaFree(G->pwb);
+    if (G->merged) gde_graph_free(G->merged);
     delete G;
     return GDE_OK;
 }
@@ -1315,6 +1450,10 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         return solve_served(ctx, G, p, nq, seeds, eps, nullptr, x_out, r_out, out64, out_mem, ld_out, oper_out,
                             rounds_out, lat_ms_out, stats);
 
+    // gradient descent and the unrelaxed heat kernel run on the graph with
+    // merged leaves where there is one (a Chebyshev seed differs from its twins
+    // in every round); rows, seeds and volumes stay the caller's
+    if (G->merged && !method_is_cheby(method) && !relax) G = G->merged;
     int W = p->tile_w;
     if (W <= 0) W = (nq == 1) ? 1 : (prec64 ? 4 : 8);
     while (W > 1 && W > nq * 2) W >>= 1;
@@ -1340,7 +1479,8 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
 
     // Memory per tile; launch groups sized to the free device memory.
     const size_t es = prec64 ? 8 : 4;
-    size_t per_tile = (size_t)n * W * es * (3 + (hk ? 1 : 0) + (method_is_cheby(method) ? 1 : 0)) +
+    const int64_t n_in = G->g.n;
+    size_t per_tile = (size_t)n_in * W * es * (3 + (hk ? 1 : 0) + (method_is_cheby(method) ? 1 : 0)) +
                       (size_t)n * W * (prec64 ? 0 : 4) + (size_t)n * 4 * 6 + 4096;
     size_t freeb = 0, totalb = 0;
     cudaMemGetInfo(&freeb, &totalb);
@@ -1399,17 +1539,18 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         rc = enable_pull(ctx, G, a, W, kPullDiv);
         if (rc == GDE_OK && prec64) rc = enable_reciprocals(ctx, G, a, kind);
         if (rc != GDE_OK) return rc;
-        const size_t slab = (size_t)nt * n * W * es;
+        const size_t slab = (size_t)nt * n_in * W * es;
         CK(cudaMemsetAsync(a.R, 0, slab, ctx->stream));
         CK(cudaMemsetAsync(a.X, 0, a.xld ? 2 * slab : slab, ctx->stream));  // interleaved: X and XC
         if (a.R2) CK(cudaMemsetAsync(a.R2, 0, slab, ctx->stream));
         if (a.DX) CK(cudaMemsetAsync(a.DX, 0, slab, ctx->stream));
-        if (a.XC && !a.xld) CK(cudaMemsetAsync(a.XC, 0, (size_t)nt * n * W * 4, ctx->stream));
+        if (a.XC && !a.xld) CK(cudaMemsetAsync(a.XC, 0, (size_t)nt * n_in * W * 4, ctx->stream));
         std::vector<TileParams> tp(nt);
         std::vector<TileState> ts(nt);
         std::vector<ColState> cs((size_t)nt * W);
         std::vector<InitCol> ic;
         std::vector<ExtractCol> ec;
+        std::vector<SeedFix> fix;  // seeds with twins in a merged graph
         for (int t = 0; t < nt; t++) {
             const TileDef& td = tiles[t0 + t];
             TileParams& P = tp[t];
@@ -1470,6 +1611,11 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
                 E.seed_add = -1.0;  // xt[s_node] -= 1. (katz_solver.py:243)
                 E.scale = hk ? std::exp(p->tau) : 1.0;  // xt /= np.exp(tau)
                 E.r_levels = (hk && method != M_HK_TAYLOR) ? 2 : 1;
+                if (G->twins(I.seed) > 0) {
+                    fix.push_back(SeedFix{q, (int64_t)t * W + c, seeds[q], I.seed, I.r0, E.scale,
+                                          E.seed >= 0 ? E.seed_add : 0.0, E.r_levels});
+                    E.seed = -1;
+                }
                 ec.push_back(E);
             }
         }
@@ -1487,12 +1633,25 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         // results
         const size_t oes = out64 ? 8 : 4;
         const int rl = (hk && method != M_HK_TAYLOR) ? 2 : 1;
+        SeedFix* d_fix = nullptr;
+        if (!fix.empty() && (x_out || r_out)) {
+            d_fix = (SeedFix*)wsget(ctx, "seed_fix", fix.size() * sizeof(SeedFix));
+            if (!d_fix) return fail(ctx, GDE_ENOMEM, "column tables");
+        }
+        const int* d_rounds = &a.cs->rounds;
         if (out_mem == GDE_MEM_DEVICE) {
             CK(extract_columns(a, prec64, W, d_ec, (int)ec.size(), x_out, r_out, out64, ld_out, n, 0, ctx->stream));
+            if (d_fix) {
+                CK(cudaMemcpyAsync(d_fix, fix.data(), fix.size() * sizeof(SeedFix), cudaMemcpyHostToDevice,
+                                   ctx->stream));
+                CK(seed_entries(d_fix, (int)fix.size(), d_rounds, sizeof(ColState), nullptr, 0, G->perm_d, n, x_out,
+                                r_out, out64, ld_out, ctx->stream));
+            }
         } else if (x_out || r_out) {
             // stage through device memory in chunks of columns
             size_t row_b = (size_t)ld_out * oes;
             int64_t per = std::max<int64_t>(1, (int64_t)((size_t)512 << 20) / (int64_t)(row_b * (1 + rl)));
+            size_t fi = 0;
             for (size_t e0 = 0; e0 < ec.size(); e0 += per) {
                 size_t ne = std::min<size_t>(per, ec.size() - e0);
                 std::vector<ExtractCol> sub(ec.begin() + e0, ec.begin() + e0 + ne);
@@ -1503,6 +1662,18 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
                 if (!d_sub || (x_out && !sx) || (r_out && !sr)) return fail(ctx, GDE_ENOMEM, "staging buffers");
                 CK(cudaMemcpyAsync(d_sub, sub.data(), ne * sizeof(ExtractCol), cudaMemcpyHostToDevice, ctx->stream));
                 CK(extract_columns(a, prec64, W, d_sub, (int)ne, sx, sr, out64, ld_out, n, 0, ctx->stream));
+                std::vector<SeedFix> here;  // (fix lists its seeds in ec's order)
+                for (size_t i = 0; i < ne && d_fix; i++)
+                    if (fi < fix.size() && fix[fi].row == ec[e0 + i].out_row) {
+                        here.push_back(fix[fi++]);
+                        here.back().row = (int64_t)i;
+                    }
+                if (!here.empty()) {
+                    CK(cudaMemcpyAsync(d_fix, here.data(), here.size() * sizeof(SeedFix), cudaMemcpyHostToDevice,
+                                       ctx->stream));
+                    CK(seed_entries(d_fix, (int)here.size(), d_rounds, sizeof(ColState), nullptr, 0, G->perm_d, n, sx,
+                                    sr, out64, ld_out, ctx->stream));
+                }
                 for (size_t i = 0; i < ne; i++) {
                     int64_t q = ec[e0 + i].out_row;
                     if (x_out)

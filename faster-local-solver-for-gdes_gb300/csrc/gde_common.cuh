@@ -47,10 +47,14 @@ __host__ __device__ inline bool method_is_hk(int m) { return m == M_HK_LOCAL || 
 // Per-node record of a static graph: one 16-byte load gives a frontier
 // node's row and degree.
 struct __align__(16) NodeRec {
-    long long rp;             // row start in col[]
+    long long rp;             // row start in col[] (40 bits), and above them the node's twins (DevGraph::twins)
     int len;                  // row length
     float degf;               // arithmetic degree
 };
+
+constexpr int kRowBits = 40;
+__host__ __device__ inline long long rec_row(const NodeRec& r) { return r.rp & ((1ll << kRowBits) - 1); }
+__host__ __device__ inline int rec_twins(const NodeRec& r) { return (int)(r.rp >> kRowBits); }
 
 struct DevGraph {
     int64_t n;
@@ -79,6 +83,12 @@ struct DevGraph {
     int idx_bits;
     uint32_t deg_esc;
     const NodeRec* rec;       // [n] (nullptr: not built)
+    // 1: a graph whose node v stands for 1 + twins(v) nodes of one neighbour and
+    // one degree (gde_graph::merged).  After round 0 they hold the same
+    // residual, so v's push and counts are theirs together; in round 0 v is the
+    // query's seed alone, and its push into the solution is added to the
+    // seed's entry after the solve.
+    int merged;
     // Pull plan (pull rounds, symmetric graphs only; PushArgs::pull_div > 0):
     // node ids by descending row capacity, the first pull_long of them cut
     // into the chunks of pchunk, the next ones up to pull_mid shared by

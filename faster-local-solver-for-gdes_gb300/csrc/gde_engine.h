@@ -64,6 +64,22 @@ cudaError_t query_rows(const float* XI, int64_t xtile, const int32_t* perm, cons
                        int64_t nq, const int32_t* seed_int, const int32_t* kinds, double seed_add, double hk_scale,
                        void* out, int out64, int64_t ld_out, cudaStream_t st);
 
+// A seed that has twins in a merged graph: after the rows are written in
+// caller order, its entry becomes (x + r0) / scale + add if the query ran a
+// round, and its twins' residual 0 if it ran none.  rounds[col] (byte stride
+// rstride) counts the query's rounds.
+struct SeedFix {
+    int64_t row;        // output row
+    int64_t col;        // index into rounds
+    int32_t seed;       // caller id
+    int32_t node;       // merged id
+    double r0, scale, add;
+    int r_levels;       // 2: heat-kernel residual [2, n] rows
+};
+cudaError_t seed_entries(const SeedFix* fix, int nf, const int* rounds, int64_t rstride, const float* XI,
+                         int64_t xtile, const int32_t* perm, int64_t n, void* x_out, void* r_out, int out64,
+                         int64_t ld_out, cudaStream_t st);
+
 // One touched node's degree tables after an edge batch.
 struct NodeTables {
     int32_t id, len;

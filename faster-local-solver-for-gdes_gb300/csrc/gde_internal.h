@@ -82,6 +82,10 @@ struct gde_graph {
     double lam_max_est = NAN;    // adjacency spectral radius from gde_katz_spectral_bounds (NaN: none)
     uint32_t* col_deg = nullptr;
     gde::NodeRec* rec = nullptr;
+    // the same graph with the leaves of each node merged into one (static graphs
+    // where that drops a fifth of the nodes or more; nullptr: none).  Its h_perm /
+    // perm_d take caller ids to merged ids, many to one.
+    gde_graph* merged = nullptr;
     // pull plan of the row capacities (DevGraph::pord, pchunk), built on first
     // use, and whether the live rows are symmetric (-1: not checked since the last edit)
     int32_t* pord = nullptr;
@@ -93,5 +97,7 @@ struct gde_graph {
     double* rnf = nullptr;
     double* rtf = nullptr;
     bool rdeg_ok = false, rign_ok = false;
+    int twins(int32_t v) const { return g.merged ? h_twins[v] : 0; }
+    std::vector<int32_t> h_twins;  // merged graphs: twins of each node
     int32_t node_in(int64_t u) const { return relabeled ? h_perm[u] : (int32_t)u; }
 };

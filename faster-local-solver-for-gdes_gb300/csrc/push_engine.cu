@@ -666,11 +666,11 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
         T r[kPrepILP], xv[kPrepILP];
         double rd[kPrepILP];  // the FP64 residual of a hub-prefix node (RH), else unused
         float df[kPrepILP], xc[kPrepILP];
-        int len[kPrepILP];
+        int len[kPrepILP], tw[kPrepILP];  // (tw: the node's twins)
         long long rp[kPrepILP];
 #pragma unroll
         for (int q = 0; q < kPrepILP; ++q) {
-            r[q] = T(0); rd[q] = 0.0; xv[q] = T(0); df[q] = 1.f; xc[q] = 0.f; len[q] = 0; rp[q] = 0;
+            r[q] = T(0); rd[q] = 0.0; xv[q] = T(0); df[q] = 1.f; xc[q] = 0.f; len[q] = 0; rp[q] = 0; tw[q] = 0;
             if (val[q]) {
                 const int64_t off = (int64_t)u[q] * ld, xoff = (int64_t)u[q] * xld;
                 if (RH && u[q] < rh_cut) {
@@ -683,7 +683,8 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
                 if (XC) xc[q] = XC[xoff];
                 if (g.rec) {
                     const NodeRec nr = g.rec[u[q]];
-                    rp[q] = nr.rp;
+                    rp[q] = rec_row(nr);
+                    tw[q] = rec_twins(nr);
                     len[q] = nr.len;
                     df[q] = nr.degf;
                 } else {
@@ -720,7 +721,10 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
                     const int64_t off = (int64_t)u[q] * ld, xoff = (int64_t)u[q] * xld;
                     if (RH && u[q] < rh_cut) RH[u[q]] = 0.0;
                     else R[off] = T(0);
-                    if (XC) {
+                    int m = 1;  // nodes that push
+                    if (tw[q] > 0 && sh.level == 0) {
+                        // the seed alone: its entry of the solution is set after the solve
+                    } else if (XC) {
                         // Kahan-compensated FP32 accumulation of the solution
                         const float y = (float)r[q] - xc[q];
                         const float s = (float)xv[q] + y;
@@ -729,10 +733,14 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
                     } else {
                         X[xoff] = xv[q] + r[q];
                     }
-                    my_nodes += 1;
-                    if (g.degf_exact) ideg += (long long)df[q];
-                    else { my_oper += du; my_vol += du; }
-                    my_cnt += 1;
+                    if (tw[q] > 0 && sh.level > 0) {
+                        m += tw[q];
+                        push = push * (T)m;
+                    }
+                    my_nodes += m;
+                    if (g.degf_exact) ideg += (long long)df[q] * m;
+                    else { my_oper += du * m; my_vol += du * m; }
+                    my_cnt += m;
                 }
             }
             if (PULL && bits) {
@@ -768,7 +776,7 @@ struct PrepSums {
     int cnt;
 };
 
-template <typename T, int W>
+template <typename T, int W, bool MERGED>
 __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
                                        PrepSums<T, W>& total) {
     constexpr int VEC = PrepSums<T, W>::VEC;
@@ -833,7 +841,11 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
         Vec<T, VEC> push;
 #pragma unroll
         for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
-        const int di = u >= 0 ? (int)df : 0;
+        // nodes that u stands for, and whether u is the seed of some column only
+        const int tw = (MERGED && u >= 0) ? rec_twins(g.rec[u]) : 0;
+        const int m = sh.level > 0 ? 1 + tw : 1;
+        const bool seed = tw > 0 && sh.level == 0;
+        const long long di = u >= 0 ? (long long)((int)df) * m : 0;
         if (u >= 0) {
             const double base64 = ign ? nf : (dint ? (double)df : g.degd[u]);
             const float base_f = ign ? (float)base64 : df;
@@ -869,7 +881,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
                     if (!(act >> k & 1)) continue;
                     const T rk = r.v[k];
                     r.v[k] = T(0);
-                    sum.nodes[k] += 1;
+                    sum.nodes[k] += m;
                     if (absorb) {
                         // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
                         x.v[k] = rk;
@@ -878,10 +890,13 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
                     }
                     if (f32) push.v[k] = (T)((coef_f * (float)rk) / div_f);
                     else push.v[k] = (T)(per * (double)rk);
+                    if (tw > 0 && m > 1) push.v[k] = push.v[k] * (T)m;
                     const T xadd = gain * rk;
                     if (dint) sum.deg[k] += di;
-                    else sum.oper[k] += g.degd[u];
-                    if (!F64 && XC) {
+                    else sum.oper[k] += g.degd[u] * m;
+                    if (seed) {
+                        // its entry of the solution is set after the solve
+                    } else if (!F64 && XC) {
                         // Kahan-compensated FP32 accumulation of the solution
                         const float y = (float)xadd - xc.v[k];
                         const float s = (float)x.v[k] + y;
@@ -907,8 +922,8 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
         const bool in = c0 == 0 && node_in;
         if (in) {
             if (dint) sum.ivol += di;
-            else sum.vol += g.degd[u];
-            sum.cnt += 1;
+            else sum.vol += g.degd[u] * m;
+            sum.cnt += m;
         }
         if (sh.dense) {
             // consecutive nodes: their bits lie in two words at most
@@ -928,7 +943,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
 // PREP of any tile and round: tests each candidate per column, then compacts
 // the frontier.  (Out of line: its registers would cost the one-column
 // crossing tiles, which never come here.)
-template <typename T, int W, bool PULL>
+template <typename T, int W, bool PULL, bool MERGED>
 __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
                                         PrepSums<T, W>& total) {
     constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
@@ -1002,7 +1017,8 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
         bool any = false;
         Vec<T, VEC> r;
         float df = 1.f;
-        int di = 1;
+        long long di = 1;
+        int tw = 0, m = 1;  // u's twins, and the nodes that push with it
         if (valid) {
             u = sh.dense ? (int)i : cand[i];
             const int64_t off = (int64_t)u * a.ld + c0;
@@ -1011,7 +1027,11 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
             // fast test first: most scanned nodes are below every threshold
             df = g.degf[u];
             du = g.degf_exact ? (double)df : g.degd[u];
-            di = (int)df;
+            if constexpr (MERGED) {
+                tw = rec_twins(g.rec[u]);
+                if (sh.level > 0) m += tw;
+            }
+            di = (long long)((int)df) * m;
             const double thr_base = (kind == KIND_IGN) ? g.nfac[u] : du;
             const float base_f = (kind == KIND_IGN) ? (float)thr_base : df;
             double thr64 = 0.0;
@@ -1090,11 +1110,11 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                             else if (kind == KIND_KATZ) pvf = alpha_f * rf;
                             else if (kind == KIND_HK) pvf = sh.final_level ? rf / df : (hkc_f * rf) / df;
                             else pvf = (omalpha_f * rf) / npush_f;
-                            push.v[k] = absorb ? T(0) : (T)pvf;
+                            push.v[k] = absorb ? T(0) : MERGED ? (T)pvf * (T)m : (T)pvf;
                             xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(xgain_f * rf) : r.v[k];
                             r.v[k] = T(0);
                             wrote = true;
-                            sum.nodes[k] += 1;
+                            sum.nodes[k] += m;
                             if (!absorb) sum.deg[k] += di;
                             continue;
                         }
@@ -1109,7 +1129,7 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                             pv = ((1. - alpha) * rv) / g.npush[u];  // InstantGNN.py:28
                         }
                         if (absorb) pv = 0.0;
-                        push.v[k] = (T)pv;
+                        push.v[k] = MERGED ? (T)pv * (T)m : (T)pv;
                         xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(sh.tp.x_gain * rv) : r.v[k];
                         r.v[k] = T(0);
                         if constexpr (sizeof(T) == 8) {  // HK relaxation runs in FP64 only (host-checked)
@@ -1128,10 +1148,10 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                         }
                     }
                     wrote = true;
-                    sum.nodes[k] += 1;
+                    sum.nodes[k] += m;
                     if (!absorb) {
                         if (dint) sum.deg[k] += di;
-                        else sum.oper[k] += du;
+                        else sum.oper[k] += du * m;
                     }
                 }
                 if (wrote) {
@@ -1139,7 +1159,9 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                     if (cheby) vstore<T, VEC>(DX + off, dxv);
                     Vec<T, VEC> xv;
                     vload<T, VEC>(X + xoff, xv);
-                    if (absorb) {
+                    if (tw > 0 && sh.level == 0) {
+                        // a seed with twins: its entry of the solution is set after the solve
+                    } else if (absorb) {
                         // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
 #pragma unroll
                         for (int k = 0; k < VEC; ++k)
@@ -1188,8 +1210,8 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
             const bool in = leader && node_in;
             if (in) {
                 if (dint) sum.ivol += di;
-                else sum.vol += du;
-                sum.cnt += 1;
+                else sum.vol += du * m;
+                sum.cnt += m;
             }
             if (sh.dense) {
                 const int w0 = (int)(base >> 5);
@@ -1242,8 +1264,8 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                     blarge[lb + ch] = item_of(rp + (long long)ch * a.chunk, min(a.chunk, len - ch * a.chunk));
             }
             if (dint) sum.ivol += di;
-            else sum.vol += du;
-            sum.cnt += 1;
+            else sum.vol += du * m;
+            sum.cnt += m;
         }
         if constexpr (W > 1) {
             if (node_in) vstore<T, VEC>(Pw + (int64_t)u * W + c0, push);
@@ -1276,12 +1298,15 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
         if (tile_crosses(sh.tp) && !sh.dense && sh.col_live[0])
             prep_w1_cross<T, PULL>(a, t, sh, beg, end, sum.oper[0], sum.nodes[0], sum.vol, sum.cnt);
         else
-            prep_nodes<T, W, PULL>(a, t, sh, beg, end, sum);
+            a.g.merged ? prep_nodes<T, W, PULL, true>(a, t, sh, beg, end, sum)
+                       : prep_nodes<T, W, PULL, false>(a, t, sh, beg, end, sum);
     } else {
         if (sh.pull && !method_is_cheby(sh.tp.method) && !(sh.tp.kind == KIND_HK && hk_relaxed(sh.tp)))
-            prep_pull<T, W>(a, t, sh, beg, end, sum);
+            a.g.merged ? prep_pull<T, W, true>(a, t, sh, beg, end, sum)
+                       : prep_pull<T, W, false>(a, t, sh, beg, end, sum);
         else
-            prep_nodes<T, W, PULL>(a, t, sh, beg, end, sum);
+            a.g.merged ? prep_nodes<T, W, PULL, true>(a, t, sh, beg, end, sum)
+                       : prep_nodes<T, W, PULL, false>(a, t, sh, beg, end, sum);
     }
     // ---- flush per-column counters (one global atomic per column per block) ----
 #pragma unroll
@@ -2047,7 +2072,7 @@ __device__ __forceinline__ void pull_rows(const PushArgs& a, const ScatterCtx<T,
         v = g.pord ? g.pord[i] : (int)i;
         if (g.rec) {
             const NodeRec nr = g.rec[v];
-            rp = nr.rp;
+            rp = rec_row(nr);
             len = nr.len;
         } else {
             rp = g.row_ptr[v];
@@ -2387,7 +2412,8 @@ __device__ void retire_range(const PushArgs& a, int t, long long beg, long long 
         const int64_t o = v * a.ld, xo = v * xld;
         double x = (double)__ldcs(X + xo);
         if (XC) x -= (double)__ldcs(XC + xo);  // Kahan: the sum is X - XC
-        if (v == si) x = x + seed_add;
+        // (a seed with twins: after the solve, DevGraph::merged)
+        if (v == si && (!a.g.merged || rec_twins(a.g.rec[v]) == 0)) x = x + seed_add;
         if (xdiv != 1.0) x = x / xdiv;
         if (xo32) __stcs(xo32 + v, (float)x);
         if (xo64) __stcs(xo64 + v, x);
