@@ -940,7 +940,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
     total = sum;
 }
 
-// PREP of any tile and round: tests each candidate per column, then compacts
+// PREP of the other tiles and rounds: tests each candidate per column, then compacts
 // the frontier.  (Out of line: its registers would cost the one-column
 // crossing tiles, which never come here.)
 template <typename T, int W, bool PULL, bool MERGED>
@@ -954,15 +954,12 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     const int par = sh.parity;
     const int kind = sh.tp.kind, method = sh.tp.method;
     const bool global = method_is_global(method);
-    const bool cheby = method_is_cheby(method);
     const bool hk = method_is_hk(method);
     const bool ign = (kind == KIND_IGN || kind == KIND_UPPR);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int lane_g = lane % L, grp_w = lane / L;
     const int c0 = lane_g * VEC;
     const int32_t* cand = a.cand + ((int64_t)t * 2 + par) * n;
-    int32_t* next = a.cand + ((int64_t)t * 2 + (par ^ 1)) * n;
-    int32_t* mark = a.mark + (int64_t)t * n;
     uint32_t* bits = (PULL && sh.pull) ? tile_bits(a, t, par) : nullptr;
     T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;       // short rows grow up from 0,
@@ -973,9 +970,7 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     T* X = xslab_ptr<T>(a.X, a, t);
     float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) : nullptr;
     const int64_t xld = x_ld(a);
-    T* DX = cheby ? slab_ptr<T>(a.DX, a, t) : nullptr;
     const double alpha = sh.tp.alpha;
-    int* next_cnt = &ts.cand_cnt[(sh.level + 1) % 3];
 
     PrepSums<T, W> sum = total;
     double thr_scale[VEC];
@@ -984,8 +979,8 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     // path does: each threshold test is exact through the FP64 band
     // (ge_band), and the push value is formed in FP32, the tile's precision.
     // FP64 is a small fraction of the FP32 rate on GB300, and a dense round
-    // visits every node and column.  Chebyshev keeps its recurrence in FP64.
-    const bool f32 = (sizeof(T) == 4) && g.degf_exact && !cheby;
+    // visits every node and column.
+    const bool f32 = (sizeof(T) == 4) && g.degf_exact;
     float thr_f[VEC];
     const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
     // FP64 tiles: one threshold per node when the columns share theta, and
@@ -1059,24 +1054,11 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                 act[k] = a_k;
                 any |= a_k;
             }
-            if (cheby && global) {
-                // global Chebyshev updates every node whose three-term step is non-zero
-                Vec<T, VEC> dxv;
-                vload<T, VEC>(DX + off, dxv);
-#pragma unroll
-                for (int k = 0; k < VEC; ++k) {
-                    if (!live[k]) continue;
-                    act[k] = (r.v[k] != T(0)) || (dxv.v[k] != T(0));
-                    any |= act[k];
-                }
-            }
             if (any) {
                 absorb = ign && is_absorbing(g, u);
                 const float npush_f = (f32 && kind == KIND_IGN) ? (float)g.npush[u] : 1.f;
                 const double rd = rdiv ? rdiv[u] : 0.0;
                 const double gain = hk ? hkc * rd : (1. - alpha) * rd;  // the push per unit of residual
-                Vec<T, VEC> dxv;
-                if (cheby) vload<T, VEC>(DX + off, dxv);
                 Vec<T, VEC> xadd;
                 bool wrote = false;
 #pragma unroll
@@ -1084,67 +1066,51 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                     xadd.v[k] = T(0);
                     if (!act[k]) continue;
                     const double rv = (double)r.v[k];
-                    if (cheby) {
-                        // ppr_solver.py:642-646 / katz_solver.py:407-411
-                        double tmp;
-                        if (kind == KIND_KATZ) tmp = sh.coef1 * rv - sh.coef2 * (double)dxv.v[k];
-                        else tmp = sh.coef1 * rv + (sh.coef1 - 1.) * (double)dxv.v[k];
-                        if (global && tmp == 0.0) { act[k] = false; continue; }
-                        T tmpT = (T)tmp;
-                        xadd.v[k] = tmpT;
-                        dxv.v[k] = tmpT;
-                        r.v[k] = (T)(rv - (double)tmpT);  // rt[u] += -delta_xt[u] (:657)
-                        double pv;
-                        if (kind == KIND_KATZ) pv = alpha * (double)tmpT;
-                        else pv = rdiv ? gain * (double)tmpT : ((1. - alpha) * (double)tmpT) / du;
-                        push.v[k] = (T)pv;
-                    } else {
-                        // An absorbing node (threshold 0) is visited once by the
-                        // reference's initial scan and never re-enqueued; with a
-                        // zero residual it has nothing to absorb.
-                        if (absorb && r.v[k] == T(0)) { act[k] = false; continue; }
-                        if (f32) {
-                            const float rf = (float)r.v[k];
-                            float pvf;
-                            if (kind == KIND_PPR || kind == KIND_UPPR) pvf = (omalpha_f * rf) / df;
-                            else if (kind == KIND_KATZ) pvf = alpha_f * rf;
-                            else if (kind == KIND_HK) pvf = sh.final_level ? rf / df : (hkc_f * rf) / df;
-                            else pvf = (omalpha_f * rf) / npush_f;
-                            push.v[k] = absorb ? T(0) : MERGED ? (T)pvf * (T)m : (T)pvf;
-                            xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(xgain_f * rf) : r.v[k];
-                            r.v[k] = T(0);
-                            wrote = true;
-                            sum.nodes[k] += m;
-                            if (!absorb) sum.deg[k] += di;
-                            continue;
-                        }
-                        double pv;
-                        if (rdiv) pv = gain * rv;
-                        else if (kind == KIND_PPR || kind == KIND_UPPR) pv = ((1. - alpha) * rv) / du;
-                        else if (kind == KIND_KATZ) pv = alpha * rv;
-                        else if (kind == KIND_HK) {
-                            if (sh.final_level) pv = rv / du;  // hk_solver.py:254-256
-                            else pv = ((sh.tp.tau / ((double)sh.level + 1.)) * rv) / du;
-                        } else {
-                            pv = ((1. - alpha) * rv) / g.npush[u];  // InstantGNN.py:28
-                        }
-                        if (absorb) pv = 0.0;
-                        push.v[k] = MERGED ? (T)pv * (T)m : (T)pv;
-                        xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(sh.tp.x_gain * rv) : r.v[k];
+                    // An absorbing node (threshold 0) is visited once by the
+                    // reference's initial scan and never re-enqueued; with a
+                    // zero residual it has nothing to absorb.
+                    if (absorb && r.v[k] == T(0)) { act[k] = false; continue; }
+                    if (f32) {
+                        const float rf = (float)r.v[k];
+                        float pvf;
+                        if (kind == KIND_PPR || kind == KIND_UPPR) pvf = (omalpha_f * rf) / df;
+                        else if (kind == KIND_KATZ) pvf = alpha_f * rf;
+                        else if (kind == KIND_HK) pvf = sh.final_level ? rf / df : (hkc_f * rf) / df;
+                        else pvf = (omalpha_f * rf) / npush_f;
+                        push.v[k] = absorb ? T(0) : MERGED ? (T)pvf * (T)m : (T)pvf;
+                        xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(xgain_f * rf) : r.v[k];
                         r.v[k] = T(0);
-                        if constexpr (sizeof(T) == 8) {  // HK relaxation runs in FP64 only (host-checked)
-                            if (kind == KIND_HK && hk_relaxed(sh.tp)) {
-                                const double thr = ((thr_scale[k] * du) / (double)sh.tp.n_levels) / sh.psi;
-                                int subs;
-                                double left;
-                                const double moved = hk_relax(rv, sh.tp.omega, thr,
-                                                              global ? sh.col_sweeps[c0 + k] : 0, &subs, &left);
-                                if (sh.final_level) push.v[k] = moved / du;
-                                else push.v[k] = ((sh.tp.tau / ((double)sh.level + 1.)) * moved) / du;
-                                xadd.v[k] = moved;
-                                r.v[k] = left;
-                                sum.oper[k] += (double)(subs - 1) * du;  // the first sub-push is counted below
-                            }
+                        wrote = true;
+                        sum.nodes[k] += m;
+                        if (!absorb) sum.deg[k] += di;
+                        continue;
+                    }
+                    double pv;
+                    if (rdiv) pv = gain * rv;
+                    else if (kind == KIND_PPR || kind == KIND_UPPR) pv = ((1. - alpha) * rv) / du;
+                    else if (kind == KIND_KATZ) pv = alpha * rv;
+                    else if (kind == KIND_HK) {
+                        if (sh.final_level) pv = rv / du;  // hk_solver.py:254-256
+                        else pv = ((sh.tp.tau / ((double)sh.level + 1.)) * rv) / du;
+                    } else {
+                        pv = ((1. - alpha) * rv) / g.npush[u];  // InstantGNN.py:28
+                    }
+                    if (absorb) pv = 0.0;
+                    push.v[k] = MERGED ? (T)pv * (T)m : (T)pv;
+                    xadd.v[k] = (kind == KIND_IGN && !absorb) ? (T)(sh.tp.x_gain * rv) : r.v[k];
+                    r.v[k] = T(0);
+                    if constexpr (sizeof(T) == 8) {  // HK relaxation runs in FP64 only (host-checked)
+                        if (kind == KIND_HK && hk_relaxed(sh.tp)) {
+                            const double thr = ((thr_scale[k] * du) / (double)sh.tp.n_levels) / sh.psi;
+                            int subs;
+                            double left;
+                            const double moved = hk_relax(rv, sh.tp.omega, thr,
+                                                          global ? sh.col_sweeps[c0 + k] : 0, &subs, &left);
+                            if (sh.final_level) push.v[k] = moved / du;
+                            else push.v[k] = ((sh.tp.tau / ((double)sh.level + 1.)) * moved) / du;
+                            xadd.v[k] = moved;
+                            r.v[k] = left;
+                            sum.oper[k] += (double)(subs - 1) * du;  // the first sub-push is counted below
                         }
                     }
                     wrote = true;
@@ -1156,7 +1122,6 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                 }
                 if (wrote) {
                     vstore<T, VEC>(R + off, r);
-                    if (cheby) vstore<T, VEC>(DX + off, dxv);
                     Vec<T, VEC> xv;
                     vload<T, VEC>(X + xoff, xv);
                     if (tw > 0 && sh.level == 0) {
@@ -1200,8 +1165,6 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
         const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
         const bool node_act = valid && (bal & gmask) != 0;
         const bool leader = (lane_g == 0);
-        // Chebyshev moves r[u] by -dx[u]: u itself is a candidate next round
-        if (cheby && !global) append_once(leader && node_act, u, mark, sh.stamp, next, next_cnt, kFull);
         const bool node_in = node_act && !absorb;  // absorbed nodes do not push
         if (PULL && bits) {
             // a pull round: the push row by node, and the node's frontier
@@ -1274,6 +1237,180 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     total = sum;
 }
 
+// PREP of a Chebyshev tile (PPR and Katz, local and global).  The general loop
+// followed one dependent load or atomic with the next -- candidate, residual,
+// step, solution, mark, candidate counter, row bounds, item counters; here a
+// node's loads go out together, and its solution is finished behind the two
+// counters.  A node is visited once per PREP, so its entry in the next round's
+// candidates (r moves by -dx at u itself) needs no atomic on its mark.
+// 12 FP64 queries on 2.36M nodes: PREP 19.1 -> 10.1 ms of 28 -> 20 (global
+// Chebyshev on 87k nodes 4.9 -> 4.0 ms); FP64 issue and the two counters' round
+// trip bound it.
+template <typename T, int W, bool PULL>
+__device__ __noinline__ void prep_cheby(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
+                                        PrepSums<T, W>& total) {
+    constexpr int VEC = PrepSums<T, W>::VEC;
+    constexpr int L = W / VEC;
+    constexpr int GPW = 32 / L;
+    const DevGraph& g = a.g;
+    const int64_t n = g.n;
+    const bool katz = sh.tp.kind == KIND_KATZ, global = method_is_global(sh.tp.method);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int grp_w = lane / L, c0 = (lane % L) * VEC;
+    const int32_t* cand = a.cand + ((int64_t)t * 2 + sh.parity) * n;
+    int32_t* next = a.cand + ((int64_t)t * 2 + (sh.parity ^ 1)) * n;
+    int32_t* mark = a.mark + (int64_t)t * n;
+    uint32_t* bits = (PULL && sh.pull) ? tile_bits(a, t, sh.parity) : nullptr;
+    PushItem* bsmall = a.bsmall + (int64_t)t * n;
+    PushItem* blarge = a.blarge + (int64_t)t * a.large_cap;
+    TileState& ts = a.ts[t];
+    T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W + c0;
+    T* R = slab_ptr<T>(a.R, a, t) + c0;
+    T* D = slab_ptr<T>(a.DX, a, t) + c0;
+    T* X = xslab_ptr<T>(a.X, a, t) + c0;
+    float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
+    const int64_t xld = x_ld(a);
+    const bool dint = g.degf_exact != 0;
+    const double* rdiv = katz ? nullptr : g.rdeg;
+    // step = c1 r + c2 dx (ppr_solver.py:642-646 / katz_solver.py:407-411)
+    const double c1 = sh.coef1, c2 = katz ? -sh.coef2 : sh.coef1 - 1.;
+    const double coef = katz ? sh.tp.alpha : 1. - sh.tp.alpha;
+    unsigned live = 0;
+    bool same = true;
+#pragma unroll
+    for (int k = 0; k < VEC; ++k) {
+        live |= sh.col_live[c0 + k] ? 1u << k : 0u;
+        same &= sh.col_theta[c0 + k] == sh.col_theta[c0];
+    }
+    const double theta0 = sh.col_theta[c0];
+    PrepSums<T, W> sum = total;
+    for (long long base = beg + (long long)warp * GPW; base < end; base += (long long)kWarps * GPW) {
+        const long long i = base + grp_w;
+        const int u = i < end ? (sh.dense ? (int)i : cand[i]) : -1;
+        unsigned act = 0;
+        Vec<T, VEC> r, dx, push;
+        int len = 0, di = 0;
+        long long rp = 0;
+        double du = 0.0;
+#pragma unroll
+        for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
+        if (u >= 0) {
+            vload<T, VEC>(R + (int64_t)u * a.ld, r);
+            vload<T, VEC>(D + (int64_t)u * a.ld, dx);
+            const float df = g.degf[u];
+            const double rd = rdiv ? rdiv[u] : 1.0;
+            if (g.rec) {
+                const NodeRec nr = g.rec[u];
+                rp = rec_row(nr);
+                len = nr.len;
+            } else {
+                rp = g.row_ptr[u];
+                len = g.row_len[u];
+            }
+            du = dint ? (double)df : g.degd[u];
+            di = (int)df;
+            const double thr = theta0 * du;
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) {
+                const bool on = global ? r.v[k] != T(0) || dx.v[k] != T(0)
+                                       : ge_abs64((double)r.v[k], same ? thr : sh.col_theta[c0 + k] * du);
+                act |= on ? 1u << k : 0u;
+            }
+            act &= live;
+            if (act) {
+                const double per = rdiv || katz ? coef * rd : coef / du;
+#pragma unroll
+                for (int k = 0; k < VEC; ++k) {
+                    if (!(act >> k & 1)) continue;
+                    const T step = (T)(c1 * (double)r.v[k] + c2 * (double)dx.v[k]);
+                    if (global && step == T(0)) {
+                        act &= ~(1u << k);
+                        continue;
+                    }
+                    dx.v[k] = step;
+                    r.v[k] = (T)((double)r.v[k] - (double)step);  // rt[u] += -delta_xt[u] (:657)
+                    push.v[k] = (T)(per * (double)step);
+                    sum.nodes[k] += 1;
+                    if (dint) sum.deg[k] += di;
+                    else sum.oper[k] += du;
+                }
+            }
+        }
+        const unsigned bal = __ballot_sync(kFull, act != 0);
+        if (bal == 0) continue;  // warp-uniform
+        const unsigned gmask = ((L == 32) ? kFull : ((1u << L) - 1u)) << (grp_w * L);
+        const bool in = u >= 0 && (bal & gmask) != 0;
+        const bool lead = in && c0 == 0;
+        Vec<T, VEC> x;
+        Vec<float, VEC> xc;
+        if (act) {
+            vstore<T, VEC>(R + (int64_t)u * a.ld, r);
+            vstore<T, VEC>(D + (int64_t)u * a.ld, dx);
+            vload<T, VEC>(X + (int64_t)u * xld, x);
+            if (XC) vload<float, VEC>(XC + (int64_t)u * xld, xc);
+        }
+        if (in) vstore<T, VEC>(Pw + (int64_t)u * W, push);
+        if (lead) {
+            if (dint) sum.ivol += di;
+            else sum.vol += du;
+            sum.cnt += 1;
+        }
+        const unsigned bl = __ballot_sync(kFull, lead), below = (1u << lane) - 1u;
+        int nb = 0;
+        if (!global && lane == 0) nb = atomicAdd(&ts.cand_cnt[(sh.level + 1) % 3], __popc(bl));
+        if (PULL && bits) {
+            if (lead) atomicOr(bits + (u >> 5), 1u << (u & 31));
+        } else {
+            const int nch = lead && len > a.med_max ? (len + a.chunk - 1) / a.chunk : 0;
+            const bool small = lead && len <= a.small_max, med = lead && !small && nch == 0;
+            const unsigned bs = __ballot_sync(kFull, small), bm = __ballot_sync(kFull, med);
+            int sc = nch;  // inclusive warp scan of chunk counts
+            if (__any_sync(kFull, nch > 0)) {
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(kFull, sc, o);
+                    if (lane >= o) sc += y;
+                }
+            }
+            int b1, b2, b3;
+            reserve_items(ts, sh.parity, __popc(bs), __popc(bm), __shfl_sync(kFull, sc, 31), b1, b2, b3);
+            auto item_of = [&](long long at, int edges) {
+                if constexpr (W == 1) return pack_item<T>(at, edges, push.v[0]);
+                else return PushItem{at, edges, u};
+            };
+            if (small) bsmall[b1 + __popc(bs & below)] = item_of(rp, len);
+            if (med) bsmall[(n - 1) - (b2 + __popc(bm & below))] = item_of(rp, len);
+            for (int ch = 0; ch < nch; ++ch)
+                blarge[b3 + (sc - nch) + ch] = item_of(rp + (long long)ch * a.chunk, min(a.chunk, len - ch * a.chunk));
+        }
+        if (!global) {
+            nb = __shfl_sync(kFull, nb, 0);
+            if (lead) {
+                next[nb + __popc(bl & below)] = u;
+                mark[u] = sh.stamp;  // SCATTER's touches of u this round are no further candidates
+            }
+        }
+        if (act) {
+#pragma unroll
+            for (int k = 0; k < VEC; ++k) {
+                if (!(act >> k & 1)) continue;
+                if (XC) {
+                    // Kahan-compensated FP32 accumulation of the solution
+                    const float y = (float)dx.v[k] - xc.v[k];
+                    const float s = (float)x.v[k] + y;
+                    xc.v[k] = (s - (float)x.v[k]) - y;
+                    x.v[k] = (T)s;
+                } else {
+                    x.v[k] = x.v[k] + dx.v[k];
+                }
+            }
+            vstore<T, VEC>(X + (int64_t)u * xld, x);
+            if (XC) vstore<float, VEC>(XC + (int64_t)u * xld, xc);
+        }
+    }
+    total = sum;
+}
+
 // PREP over candidates [beg, end) of tile t, by the loop that fits the tile,
 // then this block's counts into the tile's.
 template <typename T, int W, bool PULL>
@@ -1295,13 +1432,17 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
         // A W = 1 crossing tile visits exactly the nodes that crossed their
         // threshold last round: every candidate is active, so all its loads are
         // issued at once.
-        if (tile_crosses(sh.tp) && !sh.dense && sh.col_live[0])
+        if (method_is_cheby(sh.tp.method))
+            prep_cheby<T, W, PULL>(a, t, sh, beg, end, sum);
+        else if (tile_crosses(sh.tp) && !sh.dense && sh.col_live[0])
             prep_w1_cross<T, PULL>(a, t, sh, beg, end, sum.oper[0], sum.nodes[0], sum.vol, sum.cnt);
         else
             a.g.merged ? prep_nodes<T, W, PULL, true>(a, t, sh, beg, end, sum)
                        : prep_nodes<T, W, PULL, false>(a, t, sh, beg, end, sum);
     } else {
-        if (sh.pull && !method_is_cheby(sh.tp.method) && !(sh.tp.kind == KIND_HK && hk_relaxed(sh.tp)))
+        if (method_is_cheby(sh.tp.method))
+            prep_cheby<T, W, PULL>(a, t, sh, beg, end, sum);
+        else if (sh.pull && !(sh.tp.kind == KIND_HK && hk_relaxed(sh.tp)))
             a.g.merged ? prep_pull<T, W, true>(a, t, sh, beg, end, sum)
                        : prep_pull<T, W, false>(a, t, sh, beg, end, sum);
         else
