@@ -237,6 +237,21 @@ int alloc_large(gde_ctx* ctx, gde_graph* G, int ntiles, TileWs& tw) {
     return GDE_OK;
 }
 
+// Ids 0..n-1 by descending key (>= 0), equal keys in order: a counting sort
+// (row lengths are small integers; the stable comparison sort that gave the
+// same order was the longer part of what merged leaves add to an upload).
+template <typename F>
+std::vector<int32_t> descending(int64_t n, F key) {
+    int64_t most = 0;
+    for (int64_t u = 0; u < n; u++) most = std::max<int64_t>(most, key(u));
+    std::vector<int64_t> at(most + 2, 0);
+    for (int64_t u = 0; u < n; u++) at[most - key(u) + 1]++;
+    for (int64_t c = 0; c <= most; c++) at[c + 1] += at[c];
+    std::vector<int32_t> ord(n);
+    for (int64_t u = 0; u < n; u++) ord[at[most - key(u)]++] = (int32_t)u;
+    return ord;
+}
+
 // Pull plan of the graph's row capacities: static rows are already in
 // descending order of length; padded and merged rows get an order by capacity
 // (a row's capacity bounds its length through every edit until a repad).
@@ -246,15 +261,7 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
     std::vector<int2> chunks;
     const bool sorted = G->relabeled && !G->g.merged;  // (a merged graph's ids go by its nodes' own degrees)
     auto capacity = [&](int64_t u) { return G->h_indptr[u + 1] - G->h_indptr[u]; };
-    if (!sorted) {
-        int64_t most = 0;
-        for (int64_t u = 0; u < n; u++) most = std::max(most, capacity(u));
-        std::vector<int64_t> at(most + 2, 0);
-        for (int64_t u = 0; u < n; u++) at[most - capacity(u) + 1]++;
-        for (int64_t c = 0; c <= most; c++) at[c + 1] += at[c];
-        ord.resize(n);
-        for (int64_t u = 0; u < n; u++) ord[at[most - capacity(u)]++] = (int32_t)u;
-    }
+    if (!sorted) ord = descending(n, capacity);
     int64_t i = 0;
     for (; i < n; i++) {
         const int32_t u = sorted ? (int32_t)i : ord[i];
@@ -490,7 +497,7 @@ constexpr int64_t kHubLen = 64;  // rows longer than this are hubs (warp-combine
 // Static graphs: node records {row start, length, degree} and, when every
 // degree is an exact integer, column words carrying the target's degree in
 // the bits above the node id.  A graph that is edited later never gets them.
-int build_static_records(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
+int build_static_records(gde_ctx* ctx, gde_graph* G) {
     const int64_t n = G->g.n, cap = G->g.cap;
     std::vector<NodeRec> rec(n);
     for (int64_t u = 0; u < n; u++) {
@@ -510,19 +517,12 @@ int build_static_records(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     const int dbits = 32 - bits;
     if (G->g.degf_exact && dbits >= 4 && cap > 0) {
         const uint32_t esc = (1u << dbits) - 1u;
-        std::vector<uint32_t> packed(cap);
-        for (int64_t j = 0; j < cap; j++) {
-            const int32_t v = col[j];
-            const double d = G->h_deg[v];
-            const uint32_t code = (d >= 0.0 && d < (double)esc && d == std::floor(d)) ? (uint32_t)d : esc;
-            packed[j] = (uint32_t)v | (code << bits);
-        }
         if (cudaMalloc(&G->col_deg, cap * sizeof(uint32_t)) != cudaSuccess) {
             cudaGetLastError();
             G->col_deg = nullptr;
             return fail(ctx, GDE_ENOMEM, "device memory exhausted (packed columns)");
         }
-        CK(cudaMemcpyAsync(G->col_deg, packed.data(), cap * sizeof(uint32_t), cudaMemcpyHostToDevice, ctx->stream));
+        CK(pack_columns(G->g.col, G->g.degd, cap, bits, esc, G->col_deg, ctx->stream));
         G->g.col_deg = G->col_deg;
         G->g.idx_bits = bits;
         G->g.deg_esc = esc;
@@ -558,6 +558,7 @@ int check_symmetric(gde_ctx* ctx, gde_graph* G, int* yes) {
 int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     const int64_t n = G->g.n;
     std::vector<int32_t> id(n, -1), rep, twins;  // internal id -> merged id; merged id -> its first node, its twins
+    std::vector<int32_t> kept(n, -1);            // id of a first node, -1 of its twins
     std::vector<int32_t> leaf(n, -1);            // parent -> merged id of its leaves
     int64_t leaves = 0;
     for (int64_t u = 0; u < n; u++) leaves += G->h_len[u] == 1;
@@ -571,7 +572,7 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
             twins[*to]++;
             continue;
         }
-        id[u] = (int32_t)rep.size();
+        id[u] = kept[u] = (int32_t)rep.size();
         if (to) *to = id[u];
         rep.push_back((int32_t)u);
         twins.push_back(0);
@@ -596,8 +597,8 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     for (int64_t v = 0; v < m; v++) {
         const int64_t u = rep[v], rp = G->h_indptr[u];
         for (int64_t j = 0; j < G->h_len[u]; j++) {
-            const int32_t w = col[rp + j];
-            if (rep[id[w]] == w) mcol.push_back(id[w]);
+            const int32_t w = kept[col[rp + j]];
+            if (w >= 0) mcol.push_back(w);
         }
         M->h_indptr[v + 1] = (int64_t)mcol.size();
         M->h_len[v] = M->h_indptr[v + 1] - M->h_indptr[v];
@@ -634,7 +635,7 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     while (M->g.hub_cut < m && G->h_len[rep[M->g.hub_cut]] > kHubLen) M->g.hub_cut++;
     rc = upload_degrees(ctx, M);  // (waits for the copies above)
     M->g.vol = G->g.vol;
-    if (rc == GDE_OK) rc = build_static_records(ctx, M, mcol.data());
+    if (rc == GDE_OK) rc = build_static_records(ctx, M);
     if (rc == GDE_ENOMEM) {
         ctx->err.clear();
         gde_graph_free(M);
@@ -1314,9 +1315,7 @@ int gde_graph_upload(gde_ctx* ctx, int64_t n, int64_t cap, const int64_t* indptr
     if (!row_len) {
         // static CSR: relabel by descending degree (stable), rows sorted
         G->relabeled = true;
-        std::vector<int32_t> iperm(n);
-        for (int64_t u = 0; u < n; u++) iperm[u] = (int32_t)u;
-        std::stable_sort(iperm.begin(), iperm.end(), [&](int32_t a, int32_t b) { return len0[a] > len0[b]; });
+        const std::vector<int32_t> iperm = descending(n, [&](int64_t u) { return len0[u]; });
         G->h_perm.resize(n);
         for (int64_t k = 0; k < n; k++) G->h_perm[iperm[k]] = (int32_t)k;
         G->h_indptr.assign(n + 1, 0);
@@ -1381,7 +1380,7 @@ int gde_graph_upload(gde_ctx* ctx, int64_t n, int64_t cap, const int64_t* indptr
     int rc = upload_degrees(ctx, G);
     if (rc != GDE_OK) { gde_graph_free(G); return rc; }
     if (G->relabeled) {
-        rc = build_static_records(ctx, G, col_src);
+        rc = build_static_records(ctx, G);
         if (rc == GDE_OK) rc = build_merged(ctx, G, col_src);
         if (rc != GDE_OK) { gde_graph_free(G); return rc; }
     }

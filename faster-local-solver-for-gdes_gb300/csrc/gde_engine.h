@@ -96,6 +96,11 @@ cudaError_t symmetry_sums(const DevGraph& g, unsigned long long* out, cudaStream
 // out[i] = 1 / in[i] (aux_kernels.cu).
 cudaError_t reciprocals(const double* in, double* out, int64_t n, cudaStream_t st);
 
+// DevGraph::col_deg of every entry: the column, and above its idx_bits bits
+// the target's degree where that is an integer below esc, else esc.
+cudaError_t pack_columns(const int32_t* col, const double* degd, int64_t cap, int idx_bits, uint32_t esc,
+                         uint32_t* out, cudaStream_t st);
+
 // Graph helpers (aux_kernels.cu).
 cudaError_t graph_apply_entries(int32_t* col, const int64_t* pos, const int32_t* val, int64_t k, cudaStream_t st);
 
