@@ -237,9 +237,8 @@ int alloc_large(gde_ctx* ctx, gde_graph* G, int ntiles, TileWs& tw) {
     return GDE_OK;
 }
 
-// Ids 0..n-1 by descending key (>= 0), equal keys in order: a counting sort
-// (row lengths are small integers; the stable comparison sort that gave the
-// same order was the longer part of what merged leaves add to an upload).
+// Ids 0..n-1 by descending key (>= 0), equal keys in order: a counting sort,
+// since row lengths and capacities are small integers.
 template <typename F>
 std::vector<int32_t> descending(int64_t n, F key) {
     int64_t most = 0;

@@ -6,17 +6,18 @@
 //
 //   PREP    (per tile) visit the candidates (the nodes touched last round, or
 //           every node when the frontier was dense), test |r| >= threshold per
-//           column in FP64, move the active residual into the solution
-//           (Kahan-compensated in FP32), compute the push row P[f][0..W), and
-//           compact the union frontier with a warp ballot + block prefix sum +
-//           one global atomic per block, bucketed by degree.
-//   SCATTER (per tile) push P rows along the CSR rows: long rows in CTA-sized
-//           chunks, medium rows one warp per row, short rows one lane group
-//           per row; W columns move per edge with one vector atomic; touched
-//           nodes are appended (deduplicated by a round stamp) as the next
-//           round's candidates unless the next round scans densely.  A round
-//           with a large frontier pulls instead: PREP writes push rows by
-//           node, and every row gathers its neighbours' (see PULL).
+//           column, move the active residual into the solution
+//           (Kahan-compensated in FP32), compute the node's push row P[v][0..W),
+//           and compact the union frontier with warp ballots into work items
+//           bucketed by degree.
+//   SCATTER (per tile) push P rows along the CSR rows in units of one warp: a
+//           chunk of a long row, a medium row, or a warp's worth of short
+//           rows, cut into pieces where a round has fewer units than warps; W
+//           columns move per edge with one vector atomic; touched nodes are
+//           appended (deduplicated by a round stamp) as the next round's
+//           candidates unless the next round scans densely.  A round with a
+//           large frontier pulls instead: PREP writes push rows by node, and
+//           every row gathers its neighbours' (see PULL).
 //
 // Semantics follow the reference's synchronous round of ppr_gd local
 // (ppr_solver.py:246-288): the frontier of round t+1 is exactly the set of
