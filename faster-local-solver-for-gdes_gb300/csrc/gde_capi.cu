@@ -1448,10 +1448,18 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         return solve_served(ctx, G, p, nq, seeds, eps, nullptr, x_out, r_out, out64, out_mem, ld_out, oper_out,
                             rounds_out, lat_ms_out, stats);
 
+    // FP32 whole-graph solves push along the caller's own edges.  A merged leaf
+    // adds its twins' pushes as one product and a gather adds a row up before
+    // it adds it: tens of thousands of equal pushes into a hub then round once
+    // instead of one by one, and rows moved by up to 3.8e-5 (relative, 8 columns
+    // on 2.36M nodes; two runs of the pushes differ by 1e-6 to 1e-5).  FP64 rows
+    // agree to 1e-15, and local FP32 solves stay within the threshold flips that
+    // they have in any order of additions.
+    const bool one_by_one = !prec64 && method_is_global(method);
     // gradient descent and the unrelaxed heat kernel run on the graph with
     // merged leaves where there is one (a Chebyshev seed differs from its twins
     // in every round); rows, seeds and volumes stay the caller's
-    if (G->merged && !method_is_cheby(method) && !relax) G = G->merged;
+    if (G->merged && !method_is_cheby(method) && !relax && !one_by_one) G = G->merged;
     int W = p->tile_w;
     if (W <= 0) W = (nq == 1) ? 1 : (prec64 ? 4 : 8);
     while (W > 1 && W > nq * 2) W >>= 1;
@@ -1534,7 +1542,8 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         a.dense_div = base.dense_div; a.max_rounds = base.max_rounds; a.allow_dense = base.allow_dense;
         rc = alloc_large(ctx, G, nt, tw);
         if (rc != GDE_OK) return rc;
-        rc = enable_pull(ctx, G, a, W, kPullDiv);
+        a.pull_div = 0;
+        if (!one_by_one) rc = enable_pull(ctx, G, a, W, kPullDiv);
         if (rc == GDE_OK && prec64) rc = enable_reciprocals(ctx, G, a, kind);
         if (rc != GDE_OK) return rc;
         const size_t slab = (size_t)nt * n_in * W * es;
