@@ -469,6 +469,13 @@ int upload_ign_tables(gde_ctx* ctx, gde_graph* G, double beta) {
     return GDE_OK;
 }
 
+// What a degree leaves of DevGraph::degf_exact and deg_int (a caller's degree
+// array may hold fractions, which FP32 can hold exactly too).
+void note_degree(gde_graph* G, double d) {
+    if ((double)(float)d != d) G->g.degf_exact = 0;
+    if (!(d >= 0.0 && d <= 16777216.0 && d == (double)(int32_t)d)) G->g.deg_int = 0;
+}
+
 int upload_degrees(gde_ctx* ctx, gde_graph* G) {
     const int64_t n = G->g.n;
     std::vector<int32_t> len(n);
@@ -484,10 +491,8 @@ int upload_degrees(gde_ctx* ctx, gde_graph* G) {
     CK(cudaMemcpyAsync(G->degf, df.data(), n * 4, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     G->g.vol = vol;
-    int exact = 1;
-    for (int64_t u = 0; u < n; u++)
-        if ((double)df[u] != G->h_deg[u]) { exact = 0; break; }
-    G->g.degf_exact = exact;
+    G->g.degf_exact = G->g.deg_int = 1;
+    for (int64_t u = 0; u < n; u++) note_degree(G, G->h_deg[u]);
     return GDE_OK;
 }
 
@@ -2017,7 +2022,7 @@ int gde_internal_graph_refresh_nodes(gde_ctx* ctx, gde_graph* G, const int64_t* 
         G->g.vol += d - G->h_deg[u];
         G->h_len[u] = h_degree[u];
         G->h_deg[u] = d;
-        if ((double)(float)d != d) G->g.degf_exact = 0;
+        note_degree(G, d);
         NodeTables& r = rec[i];
         r.id = (int32_t)u;
         r.len = (int32_t)h_degree[u];

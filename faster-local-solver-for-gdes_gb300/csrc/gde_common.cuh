@@ -73,7 +73,8 @@ struct DevGraph {
     const double* rnf;        // [n]
     const double* rtf;        // [n]
     double vol;               // sum of degrees (m)
-    int degf_exact;           // 1 when every degree is an integer < 2^24 (degf == degd exactly)
+    int degf_exact;           // 1 when degf == degd exactly
+    int deg_int;              // 1 when every degree is an integer from 0 to 2^24 (counts may sum them as integers)
     const int32_t* perm;      // caller id -> internal id (nullptr: identity)
     int32_t hub_cut;          // internal ids < hub_cut are hubs (degree-sorted graphs; 0: none)
     // Static graphs with exact integer degrees: col_deg[j] = col[j] | code << idx_bits,

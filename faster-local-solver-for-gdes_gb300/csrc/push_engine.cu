@@ -68,8 +68,8 @@ constexpr unsigned kFull = 0xffffffffu;
 // Threshold test r >= theta * d without FP64 arithmetic in the common case.
 // GB300 issues FP64 at a small fraction of the FP32 rate, so the FP32 path
 // decides in FP32 whenever r is clearly on one side: t32 = fl32(fl32(theta) *
-// d) is within 2^-23 (relative) of theta * d for an integer degree d < 2^24,
-// so r >= t32 * (1 + 2^-20) implies r > theta * d and r < t32 * (1 - 2^-20)
+// d) is within 2^-23 (relative) of theta * d for a degree d that FP32 holds
+// exactly, so r >= t32 * (1 + 2^-20) implies r > theta * d and r < t32 * (1 - 2^-20)
 // implies r < theta * d.  Only inside that band is the FP64 product formed.
 // The result is exactly that of (double)r >= theta * d.
 // ---------------------------------------------------------------------------
@@ -365,7 +365,7 @@ __device__ void check_phase(const PushArgs& a, int t, int it, int* s_cnt) {
         s_cnt[threadIdx.x] = 0;
     }
     __syncthreads();
-    // FP32 tiles on integer degrees test in FP32 (exact through the band of
+    // FP32 tiles on exact degrees test in FP32 (exact through the band of
     // ge_threshold) and read the 4-byte degree: FP64 is a small fraction of
     // the FP32 rate on GB300, and this phase touches every node.
     const bool f32 = (sizeof(T) == 4) && a.g.degf_exact;
@@ -653,7 +653,7 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
     double* RH = (sizeof(T) == 4) ? rh_ptr(a, t) : nullptr;  // hub prefix in FP64
     const int rh_cut = a.rh_cut;
     uint32_t* bits = (PULL && sh.pull) ? tile_bits(a, t, par) : nullptr;
-    long long ideg = 0;  // sum of (integer) degrees of the pushed nodes
+    long long ideg = 0;  // sum of the pushed nodes' degrees, each cut to an integer (ppr_solver.py:249-250)
     for (long long base = beg + (long long)warp * 32 * kPrepILP; base < end;
          base += (long long)kWarps * 32 * kPrepILP) {
         bool val[kPrepILP];
@@ -770,7 +770,7 @@ template <typename T, int W>
 struct PrepSums {
     static constexpr int VEC = (sizeof(T) == 4) ? (W >= 4 ? 4 : W) : (W >= 2 ? 2 : 1);
     double oper[VEC];
-    long long deg[VEC];  // the same sum while degrees are exact integers
+    long long deg[VEC];  // the same sum while degrees are integers (DevGraph::deg_int)
     int nodes[VEC];
     double vol;
     long long ivol;
@@ -800,7 +800,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
     float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
     const int64_t xld = x_ld(a);
     const bool f32 = !F64 && g.degf_exact;
-    const bool dint = g.degf_exact != 0;
+    const bool dint = g.deg_int != 0;
     // a push is (coef r) / div with div = the degree, InstantGNN's d^(1-beta)
     // or (Katz) 1; the solution takes gain r
     const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
@@ -848,7 +848,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
         const bool seed = tw > 0 && sh.level == 0;
         const long long di = u >= 0 ? (long long)((int)df) * m : 0;
         if (u >= 0) {
-            const double base64 = ign ? nf : (dint ? (double)df : g.degd[u]);
+            const double base64 = ign ? nf : (g.degf_exact ? (double)df : g.degd[u]);
             const float base_f = ign ? (float)base64 : df;
             const double thr64 = F64 && !all ? scale0 * base64 : 0.0;
 #pragma unroll
@@ -976,7 +976,7 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     PrepSums<T, W> sum = total;
     double thr_scale[VEC];
     bool live[VEC];
-    // FP32 tiles on integer degrees decide and push in FP32, as the W = 1
+    // FP32 tiles on exact degrees decide and push in FP32, as the W = 1
     // path does: each threshold test is exact through the FP64 band
     // (ge_band), and the push value is formed in FP32, the tile's precision.
     // FP64 is a small fraction of the FP32 rate on GB300, and a dense round
@@ -987,7 +987,7 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     // FP64 tiles: one threshold per node when the columns share theta, and
     // divisions by the node's divisor as products with its reciprocal
     const double* rdiv = (sizeof(T) == 8 && kind != KIND_KATZ) ? (kind == KIND_IGN ? g.rnf : g.rdeg) : nullptr;
-    const bool dint = g.degf_exact != 0;
+    const bool dint = g.deg_int != 0;
     bool same = true;
 #pragma unroll
     for (int k = 0; k < VEC; ++k) {
@@ -1083,7 +1083,10 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
                         r.v[k] = T(0);
                         wrote = true;
                         sum.nodes[k] += m;
-                        if (!absorb) sum.deg[k] += di;
+                        if (!absorb) {
+                            if (dint) sum.deg[k] += di;
+                            else sum.oper[k] += du * m;
+                        }
                         continue;
                     }
                     double pv;
@@ -1271,7 +1274,7 @@ __device__ __noinline__ void prep_cheby(const PushArgs& a, int t, const TileSh& 
     T* X = xslab_ptr<T>(a.X, a, t) + c0;
     float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
     const int64_t xld = x_ld(a);
-    const bool dint = g.degf_exact != 0;
+    const bool dint = g.deg_int != 0;
     const double* rdiv = katz ? nullptr : g.rdeg;
     // step = c1 r + c2 dx (ppr_solver.py:642-646 / katz_solver.py:407-411)
     const double c1 = sh.coef1, c2 = katz ? -sh.coef2 : sh.coef1 - 1.;
@@ -1308,7 +1311,7 @@ __device__ __noinline__ void prep_cheby(const PushArgs& a, int t, const TileSh& 
                 rp = g.row_ptr[u];
                 len = g.row_len[u];
             }
-            du = dint ? (double)df : g.degd[u];
+            du = g.degf_exact ? (double)df : g.degd[u];
             di = (int)df;
             const double thr = theta0 * du;
 #pragma unroll
@@ -1561,7 +1564,7 @@ __device__ __forceinline__ void push_edge(const DevGraph& g, T* tgt, int64_t ld,
                                           bool tgt_scale);
 
 // Did an addition take node v's residual from `old` to `s` across its
-// threshold theta * d_v?  Exact; FP32 residuals on integer degrees decide in
+// threshold theta * d_v?  Exact; FP32 residuals on exact degrees decide in
 // FP32 outside the band of ge_threshold.
 template <typename T>
 __device__ __forceinline__ bool crossed(const DevGraph& g, int v, T old, T s, double theta, float theta_f) {
