@@ -90,3 +90,22 @@ def test_operations_of_fractional_degrees(name, W, kind, method):
         assert res["oper"][i] == want
         # an FP32 rounding at a threshold moves a node's push by a round: a few nodes of the largest degree
         assert abs(r32["oper"][i] - want) <= 6 * deg.max()
+
+
+@pytest.mark.parametrize("kind, method", [(L.HK, L.HK_LOCAL), (L.PPR, L.LOCAL_GD), (L.KATZ, L.LOCAL_GD)])
+def test_fp32_tiles_of_degrees_that_fp32_does_not_hold(kind, method):
+    """Degrees of 1.1 times the row length, one eps for all columns: wide tiles push the nodes that one column pushes."""
+    g = _graph("dense")
+    deg = 1.1 * g.degree
+    G = api.Graph(g.indptr, g.indices, degree=deg)
+    seeds, eps = np.array([3, 60, 121, 182, 200, 261, 300, 332], np.int32), 1e-5
+    katz = 0.5 / deg.max()
+    args = dict(alpha=0.0 if kind == L.HK else katz if kind == L.KATZ else 0.1, tau=5.0 if kind == L.HK else 0.0)
+    want = api.solve(G, kind, method, seeds, eps, prec="fp64", tile_w=2, **args)["oper"]
+    if kind == L.HK:  # (the oracle's own count, to the rounding of a sum in another order)
+        for i, s in enumerate(seeds):
+            assert want[i] == pytest.approx(_operations(g, deg, kind, method, s, eps), rel=OPER_RTOL)
+    for W in (1, 2, 4, 8):
+        got = api.solve(G, kind, method, seeds, eps, prec="fp32", tile_w=W, **args)["oper"]
+        # an FP32 rounding at a threshold moves a node's push by a round: a few nodes of the largest degree
+        assert np.abs(got - want).max() <= 6 * deg.max()
