@@ -724,8 +724,13 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
     a.groups = std::max(1, std::min(std::min(p->groups > 0 ? p->groups : g_default, S), kMaxGroups));
     rc = alloc_large(ctx, G, S, tw);
     if (rc != GDE_OK) return rc;
+    // FP32 slots on a merged graph push in every round: a hub's FP64 residual
+    // takes a merged leaf's pushes whole (pack_item), which a gather of FP32
+    // push values by node could not
+    const bool whole_hubs = !prec64 && G->g.merged && G->g.hub_cut > 0;
     // the frontier bitmaps count against an HBM budget too
-    if (budget_bytes <= 0.0 || (double)S * ((double)served_slot_bytes(n, G->g.cap, prec64, any_hk, base, G->g.hub_cut) +
+    if (whole_hubs) a.pull_div = 0;
+    else if (budget_bytes <= 0.0 || (double)S * ((double)served_slot_bytes(n, G->g.cap, prec64, any_hk, base, G->g.hub_cut) +
                                             (double)(n / 4 + 16)) <= budget_bytes) {
         rc = enable_pull(ctx, G, a, 1, kPullDivServed);
         if (rc != GDE_OK) return rc;

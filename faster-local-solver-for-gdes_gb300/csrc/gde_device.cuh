@@ -89,18 +89,30 @@ __device__ __forceinline__ bool ge_abs64(double r, double thr) {
 // A work item of a one-column tile holds its push value instead of the
 // frontier index of a push row: the edges are one load away from the item.
 // Row starts take 40 bits and lengths 24 (the host caps the row classes).
+// FP32 items of a merged leaf hold its own push value and `times` it is pushed
+// (with its twins'); 0: once.
 template <typename T>
-__device__ __forceinline__ PushItem pack_item(long long rp, int len, T push) {
+__device__ __forceinline__ PushItem pack_item(long long rp, int len, T push, int times = 0) {
     PushItem it;
     it.rp = rp | ((long long)len << 40);
     if constexpr (sizeof(T) == 8) {
         it.len = __double2hiint(push);
         it.node = __double2loint(push);
     } else {
-        it.len = 0;
+        it.len = times;
         it.node = __float_as_int(push);
     }
     return it;
+}
+// The sum that an FP32 item of one edge pushes, whole: 24 bits times up to 23 fit
+// FP64's 53.  In integers: FP64 instructions issue at 1/16 rate.
+__device__ __forceinline__ double item_sum(const PushItem& it) {
+    const unsigned b = (unsigned)it.node, e = b >> 23 & 0xffu, times = it.len > 1 ? it.len : 1;
+    if (e == 0u || e == 0xffu) return (double)__int_as_float(it.node) * times;
+    const unsigned long long p = (unsigned long long)((b & 0x7fffffu) | 0x800000u) * times;
+    const int z = __clzll((long long)p);  // the product's first bit is 63 - z; 24 bits alone would be at 23
+    return __longlong_as_double((long long)((unsigned long long)(b >> 31) << 63 |
+                                            (unsigned long long)(e + 1023 - 127 + 40 - z) << 52 | p << (z + 1) >> 12));
 }
 template <typename T>
 __device__ __forceinline__ T unpack_item(const PushItem& it, long long& rp, int& len) {

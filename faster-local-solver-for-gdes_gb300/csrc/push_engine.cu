@@ -585,7 +585,7 @@ __device__ __forceinline__ void reserve_items(TileState& ts, int par, int small,
 // items, which carry the push value.
 template <typename T>
 __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, bool node_in, int len, long long rp,
-                                             T push) {
+                                             T push, int times) {
     const int lane = threadIdx.x & 31;
     const int64_t n = a.g.n;
     TileState& ts = a.ts[t];
@@ -612,7 +612,7 @@ __device__ __forceinline__ void emit_node_w1(const PushArgs& a, int t, int par, 
     const unsigned below = (1u << lane) - 1u;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;
     if (bucket == 0) {
-        bsmall[b1 + __popc(bs & below)] = pack_item<T>(rp, len, push);
+        bsmall[b1 + __popc(bs & below)] = pack_item<T>(rp, len, push, times);
     } else if (bucket == 1) {
         bsmall[(n - 1) - (b2 + __popc(bm & below))] = pack_item<T>(rp, len, push);
     } else {
@@ -699,6 +699,7 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
         for (int q = 0; q < kPrepILP; ++q) {
             bool act = false;
             T push = T(0);
+            int times = 0;  // FP32: pushes of u and its twins (pack_item)
             if (val[q]) {
                 const double du = g.degf_exact ? (double)df[q] : g.degd[u[q]];
                 if constexpr (sizeof(T) == 4) {
@@ -736,7 +737,8 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
                     }
                     if (tw[q] > 0 && sh.level > 0) {
                         m += tw[q];
-                        push = push * (T)m;
+                        if constexpr (sizeof(T) == 4) times = m;
+                        else push = push * (T)m;
                     }
                     my_nodes += m;
                     if (g.degf_exact) ideg += (long long)df[q] * m;
@@ -746,11 +748,11 @@ __device__ void prep_w1_cross(const PushArgs& a, int t, const TileSh& sh, long l
             }
             if (PULL && bits) {
                 if (act) {  // a pull round: the push value by node, and the node's frontier bit
-                    reinterpret_cast<T*>(a.P)[(int64_t)t * n + u[q]] = push;
+                    reinterpret_cast<T*>(a.P)[(int64_t)t * n + u[q]] = times ? push * (T)times : push;
                     atomicOr(bits + (u[q] >> 5), 1u << (u[q] & 31));
                 }
             } else {
-                emit_node_w1<T>(a, t, par, act, len[q], rp[q], push);
+                emit_node_w1<T>(a, t, par, act, len[q], rp[q], push, times);
             }
         }
     }
@@ -1867,7 +1869,11 @@ __device__ void scatter_short_w1(const PushArgs& a, const PushItem* items, const
     int len = 0;
     long long rp = 0;
     T pv = T(0);
-    if (lane < count) pv = unpack_item<T>(items[lane], rp, len);
+    if (lane < count) {
+        const PushItem it = items[lane];
+        pv = unpack_item<T>(it, rp, len);
+        if (sizeof(T) == 4 && it.len > 1) pv = pv * (T)it.len;
+    }
     int incl = len;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -1913,8 +1919,23 @@ __device__ void scatter_short_w1(const PushArgs& a, const PushItem* items, const
                     fagg[warp][lane] = T(0);
                     faggd[warp][lane] = 0.0;
                 }
+                double add = 0.0;
+                if (sizeof(T) == 4 && c.rh && g.merged) {
+                    // a merged leaf's pushes into an FP64 residual are added whole, not as an FP32 product
+                    // (the edge's row is looked up once more: kept from above it costs registers in every step)
+                    const int e = e0 + u * 32 + lane;
+                    int r = 0;
+#pragma unroll
+                    for (int b = 16; b > 0; b >>= 1) {
+                        const int ex = __shfl_sync(kFull, excl, (r + b) & 31);
+                        if (r + b < 32 && ex <= e) r += b;
+                    }
+                    if (hd) add = item_sum(items[r]);
+                } else if (hd) {
+                    add = (double)p[u];
+                }
                 __syncwarp();
-                if (hd) atomicAdd(&faggd[warp][leader], (double)p[u]);
+                if (hd) atomicAdd(&faggd[warp][leader], add);
                 else if (hub) atomicAdd(&fagg[warp][leader], p[u]);
                 __syncwarp();
                 if (hd && lane == leader) {

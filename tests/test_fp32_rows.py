@@ -72,3 +72,28 @@ def test_a_hub_of_many_leaves(W):
     x = api.solve(G, L.HK, L.HK_TAYLOR, seeds, eps, prec="fp32", tau=TAU, tile_w=W)["x"].astype(np.float64)
     centre, leaf = _taylor(levels)
     assert np.allclose(x[:, 0], centre, rtol=RTOL, atol=0) and np.allclose(x[:, 1:], leaf, rtol=RTOL, atol=0)
+
+
+def _served(eps):
+    """A served PPR query from the centre, whose residual is FP64: (residual of the centre, of a leaf, x of the centre)."""
+    rc, rl, xc = ALPHA, f32(0), _Kahan()
+    while True:
+        if rc >= eps * ALPHA * LEAVES:
+            xc.add(rc)
+            rc, rl = 0.0, rl + f32(((1.0 - ALPHA) * rc) / LEAVES)
+        elif float(rl) >= eps * ALPHA:
+            rc, rl = rc + LEAVES * float(f32(1.0 - ALPHA) * rl / f32(1)), f32(0)
+        else:
+            return rc, float(rl), xc.value()
+
+
+def test_a_served_hub_keeps_every_push_in_fp64():
+    indptr = np.concatenate([[0], LEAVES + np.arange(LEAVES + 1)])
+    indices = np.concatenate([np.arange(1, LEAVES + 1), np.zeros(LEAVES, np.int64)]).astype(np.int32)
+    G = api.Graph(indptr, indices)
+    eps = next(e for e in np.geomspace(1e-6, 2e-6, 50) if _served(e)[0] > 0)  # the last push is the leaves'
+    res = api.solve(G, L.PPR, L.LOCAL_GD, np.zeros(1, np.int32), eps, prec="fp32", out64=True, alpha=ALPHA)
+    rc, rl, xc = _served(eps)
+    # the sum of the pushes is exact in FP64 (24 bits times 20,000); rounded to FP32 it would be 2^-25 off
+    assert float(f32(rc)) != rc and abs(res["r"][0, 0] / rc - 1) < 2.0 ** -50
+    assert np.allclose(res["r"][0, 1:], rl, rtol=RTOL, atol=0) and res["x"][0, 0] == pytest.approx(xc, rel=RTOL)
