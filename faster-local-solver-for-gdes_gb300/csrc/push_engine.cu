@@ -441,7 +441,7 @@ extern __shared__ __align__(16) unsigned char dyn_smem[];
 __device__ __forceinline__ TileSlot* tile_slots() { return reinterpret_cast<TileSlot*>(dyn_smem); }
 
 enum : unsigned char {
-    SF_FINAL = 1, SF_TRACK = 2, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32
+    SF_FINAL = 1, SF_TRACK = 2, SF_PULLNEXT = 4, SF_TGTSCALE = 8, SF_HK = 16, SF_CROSS = 32
 };
 
 // Local GD for PPR and Katz only ever adds non-negative values to
@@ -2464,6 +2464,10 @@ __device__ __noinline__ void pull_phase(const PushArgs& a, int npull, const Grou
     const unsigned nw = (unsigned)gi.dim * kWarps;
     unsigned u = (unsigned)gi.blk * kWarps + (threadIdx.x >> 5);
     for (int p = 0; p < npull; ++p) {
+        if (u >= units) {  // (without the tile's state: few rows and many tiles leave a warp a unit or two in all)
+            u -= units;
+            continue;
+        }
         const TileSlot& s = tile_slots()[tile_slots()[p].pull];
         const int t = s.tile;
         const uint32_t* bits = tile_bits(a, t, s.level & 1);
@@ -3395,6 +3399,7 @@ __global__ void __launch_bounds__(kThreads, MB)
                         if (tp.kind == KIND_IGN) f |= SF_TGTSCALE;
                         if (tile_crosses(tp)) f |= SF_CROSS;
                         else if (!dense_next_round(a, tp, ts, par) && !fin && !last_taylor) f |= SF_TRACK;
+                        if (PULL && pull_next_round(a, ts, par)) f |= SF_PULLNEXT;
                         sl[k].flags = f;
                         pull = PULL && ts.pull[par] && ts.front_cnt[par] > 0 && !last_taylor;
                     }
@@ -3439,10 +3444,8 @@ __global__ void __launch_bounds__(kThreads, MB)
                 if (rs.npull > 0) pull_phase<T, W>(a, rs.npull, gi);
             // a clear bitmap for each tile whose next round pulls
             for (int k = 0; k < ntl; ++k) {
-                const int t = sl[k].tile;
-                const int par = sl[k].level & 1;
-                if (!pull_next_round(a, a.ts[t], par)) continue;
-                uint32_t* b = tile_bits(a, t, par ^ 1);
+                if (!(sl[k].flags & SF_PULLNEXT)) continue;
+                uint32_t* b = tile_bits(a, sl[k].tile, (sl[k].level & 1) ^ 1);
                 for (int64_t w = (int64_t)gi.blk * kThreads + threadIdx.x; w < a.bit_words;
                      w += (int64_t)gi.dim * kThreads)
                     b[w] = 0u;
