@@ -13,6 +13,8 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -57,8 +59,7 @@ void* wsget(gde_ctx* ctx, const std::string& name, size_t bytes, bool* fresh = n
     b.p = nullptr;
     b.bytes = 0;
     size_t want = std::max<size_t>(bytes, 256);
-    if (cudaMalloc(&b.p, want) != cudaSuccess) {
-        cudaGetLastError();
+    if (gde_internal_malloc(ctx, &b.p, want) != cudaSuccess) {
         b.p = nullptr;
         return nullptr;
     }
@@ -624,7 +625,7 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
         gde_graph_free(M);
         return GDE_OK;
     }
-    G->merged = M;  // (freed with G from here on)
+    std::shared_ptr<gde_graph> held(M, [](gde_graph* g) { gde_graph_free(g); });
     CK(cudaMemsetAsync(M->row_ptr, 0, (m + 3) * sizeof(int64_t), ctx->stream));
     CK(cudaMemcpyAsync(M->row_ptr, M->h_indptr.data(), (m + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     if (cap > 0) CK(cudaMemcpyAsync(M->col, mcol.data(), cap * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
@@ -642,9 +643,24 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     if (rc == GDE_OK) rc = build_static_records(ctx, M);
     if (rc == GDE_ENOMEM) {
         ctx->err.clear();
-        gde_graph_free(M);
-        G->merged = nullptr;
         return GDE_OK;
+    }
+    if (rc != GDE_OK) return rc;
+    G->merged = held;
+    std::lock_guard<std::mutex> lock(ctx->spare_mu);
+    ctx->spare.push_back(G);
+    return GDE_OK;
+}
+
+// Runs a solve of G, and once more if it ran out of memory with the merged
+// copy that it ran on given back meanwhile.
+template <typename F>
+int with_room(gde_ctx* ctx, gde_graph* G, F solve) {
+    const bool had = G && G->merged_copy();
+    int rc = solve();
+    if (rc == GDE_ENOMEM && had && !G->merged_copy()) {
+        ctx->err.clear();
+        rc = solve();
     }
     return rc;
 }
@@ -678,7 +694,8 @@ int solve_served(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, co
     // on the graph with merged leaves where there is one (hash-table queries
     // keep to single nodes); rows and seeds stay the caller's n_out nodes
     const int64_t n_out = G->g.n;
-    if (G->merged && p->sparse_blocks <= 0) G = G->merged;
+    const std::shared_ptr<gde_graph> merged = p->sparse_blocks > 0 ? nullptr : G->merged_copy();
+    if (merged) G = merged.get();
     const int64_t n = G->g.n;
     const int kind = p->kind;
     const int prec64 = (p->prec == GDE_FP64);
@@ -1209,7 +1226,7 @@ int gde_ctx_trace_read(gde_ctx* ctx, uint64_t* out, int64_t cap, int* iters, int
     return GDE_OK;
 }
 
-int gde_serve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
+static int serve_call(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
               const double* arrival_ms, void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out,
               double* oper_out, int32_t* rounds_out, float* lat_ms_out, gde_stats* stats) {
     if (!ctx || !G || !p || nq < 0 || (nq > 0 && (!seeds || !eps))) return fail(ctx, GDE_EINVAL, "bad serve arguments");
@@ -1237,7 +1254,16 @@ int gde_serve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
                         rounds_out, lat_ms_out, stats);
 }
 
-int gde_serve_mixed(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* kinds,
+int gde_serve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
+              const double* arrival_ms, void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out,
+              double* oper_out, int32_t* rounds_out, float* lat_ms_out, gde_stats* stats) {
+    return with_room(ctx, G, [&] {
+        return serve_call(ctx, G, p, nq, seeds, eps, arrival_ms, x_out, r_out, out64, out_mem, ld_out,
+                          oper_out, rounds_out, lat_ms_out, stats);
+    });
+}
+
+static int serve_mixed_call(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* kinds,
                     const int32_t* seeds, const double* eps, const double* alphas, const double* arrival_ms,
                     double hbm_budget_bytes, void* x_out, int out64, int out_mem, int64_t ld_out, double* oper_out,
                     int32_t* rounds_out, float* lat_ms_out, gde_stats* stats) {
@@ -1270,6 +1296,16 @@ int gde_serve_mixed(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq,
     pp.kind = kinds[0] == KIND_HK ? KIND_PPR : kinds[0];
     return solve_served(ctx, G, &pp, nq, seeds, eps, arrival_ms, x_out, nullptr, out64, out_mem, ld_out, oper_out,
                         rounds_out, lat_ms_out, stats, kinds, alphas, hbm_budget_bytes);
+}
+
+int gde_serve_mixed(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* kinds,
+                    const int32_t* seeds, const double* eps, const double* alphas, const double* arrival_ms,
+                    double hbm_budget_bytes, void* x_out, int out64, int out_mem, int64_t ld_out, double* oper_out,
+                    int32_t* rounds_out, float* lat_ms_out, gde_stats* stats) {
+    return with_room(ctx, G, [&] {
+        return serve_mixed_call(ctx, G, p, nq, kinds, seeds, eps, alphas, arrival_ms, hbm_budget_bytes,
+                                x_out, out64, out_mem, ld_out, oper_out, rounds_out, lat_ms_out, stats);
+    });
 }
 
 int gde_ctx_sync(gde_ctx* ctx) {
@@ -1352,11 +1388,12 @@ int gde_graph_upload(gde_ctx* ctx, int64_t n, int64_t cap, const int64_t* indptr
     G->g.n = n;
     G->g.cap = cap;
     // row_ptr gets two spare entries so aligned 16-byte windows stay in bounds
-    cudaError_t e = cudaMalloc(&G->row_ptr, (n + 3) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&G->col, std::max<int64_t>(cap, 1) * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&G->row_len, n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&G->degf, n * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&G->degd, n * sizeof(double));
+    auto room = [&](auto** p, size_t bytes) { return gde_internal_malloc(ctx, (void**)p, bytes); };
+    cudaError_t e = room(&G->row_ptr, (n + 3) * sizeof(int64_t));
+    if (e == cudaSuccess) e = room(&G->col, std::max<int64_t>(cap, 1) * sizeof(int32_t));
+    if (e == cudaSuccess) e = room(&G->row_len, n * sizeof(int32_t));
+    if (e == cudaSuccess) e = room(&G->degf, n * sizeof(float));
+    if (e == cudaSuccess) e = room(&G->degd, n * sizeof(double));
     if (e != cudaSuccess) {
         cudaFree(G->row_ptr); cudaFree(G->col); cudaFree(G->row_len); cudaFree(G->degf); cudaFree(G->degd);
         delete G;
@@ -1367,11 +1404,11 @@ int gde_graph_upload(gde_ctx* ctx, int64_t n, int64_t cap, const int64_t* indptr
                        ctx->stream));
     if (cap > 0) CK(cudaMemcpyAsync(G->col, col_src, cap * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     if (G->relabeled) {
-        CK(cudaMalloc(&G->perm_d, n * sizeof(int32_t)));
+        CK(room(&G->perm_d, n * sizeof(int32_t)));
         CK(cudaMemcpyAsync(G->perm_d, G->h_perm.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
         std::vector<int32_t> inv(n);
         for (int64_t u = 0; u < n; u++) inv[G->h_perm[u]] = (int32_t)u;
-        CK(cudaMalloc(&G->iperm_d, n * sizeof(int32_t)));
+        CK(room(&G->iperm_d, n * sizeof(int32_t)));
         CK(cudaMemcpyAsync(G->iperm_d, inv.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));  // inv is released on return
     }
@@ -1407,8 +1444,12 @@ int gde_graph_free(gde_graph* G) {
     cudaFree(G->pord); cudaFree(G->pchunk);
     cudaFree(G->rdeg); cudaFree(G->rnf); cudaFree(G->rtf);
     cudaFree(G->pw1); cudaFree(G->pwb);
-    if (G->merged) gde_graph_free(G->merged);
-    delete G;
+    {
+        std::lock_guard<std::mutex> lock(G->ctx->spare_mu);
+        std::vector<gde_graph*>& v = G->ctx->spare;
+        v.erase(std::remove(v.begin(), v.end(), G), v.end());
+    }
+    delete G;  // (and its merged copy, once no solve holds it)
     return GDE_OK;
 }
 
@@ -1420,7 +1461,7 @@ int gde_graph_info(gde_graph* G, int64_t* n, int64_t* cap, double* vol) {
     return GDE_OK;
 }
 
-int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
+static int solve_call(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
               void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out, double* oper_out, int32_t* rounds_out,
               float* lat_ms_out, gde_stats* stats) {
     if (!ctx || !G || !p || nq < 0 || (nq > 0 && (!seeds || !eps))) return fail(ctx, GDE_EINVAL, "bad solve arguments");
@@ -1469,7 +1510,9 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
     // gradient descent and the unrelaxed heat kernel run on the graph with
     // merged leaves where there is one (a Chebyshev seed differs from its twins
     // in every round); rows, seeds and volumes stay the caller's
-    if (G->merged && !method_is_cheby(method) && !relax && !one_by_one) G = G->merged;
+    const bool mergeable = !method_is_cheby(method) && !relax && !one_by_one;
+    const std::shared_ptr<gde_graph> merged = mergeable ? G->merged_copy() : nullptr;
+    if (merged) G = merged.get();
     int W = p->tile_w;
     if (W <= 0) W = (nq == 1) ? 1 : (prec64 ? 4 : 8);
     while (W > 1 && W > nq * 2) W >>= 1;
@@ -1745,6 +1788,15 @@ int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const
         stats->kernel_ms = kernel_ms;
     }
     return GDE_OK;
+}
+
+int gde_solve(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds, const double* eps,
+              void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out, double* oper_out, int32_t* rounds_out,
+              float* lat_ms_out, gde_stats* stats) {
+    return with_room(ctx, G, [&] {
+        return solve_call(ctx, G, p, nq, seeds, eps, x_out, r_out, out64, out_mem, ld_out, oper_out,
+                          rounds_out, lat_ms_out, stats);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -2063,6 +2115,29 @@ int gde_internal_graph_host(gde_graph* G, const int64_t** indptr, const int64_t*
     *len = G->h_len.data();
     *n = G->g.n;
     return GDE_OK;
+}
+
+cudaError_t gde_internal_malloc(gde_ctx* ctx, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return e;
+    cudaGetLastError();
+    *p = nullptr;
+    if (e != cudaErrorMemoryAllocation) return e;
+    std::vector<std::shared_ptr<gde_graph>> copies;  // freed here, or when the solve that runs on one returns
+    {
+        std::lock_guard<std::mutex> lock(ctx->spare_mu);
+        for (gde_graph* G : ctx->spare) {
+            std::lock_guard<std::mutex> own(G->mu);
+            copies.push_back(std::move(G->merged));
+            G->merged.reset();
+        }
+        ctx->spare.clear();
+    }
+    if (copies.empty()) return e;
+    copies.clear();
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
 }
 
 void* gde_internal_wsget(gde_ctx* ctx, const char* name, size_t bytes) { return wsget(ctx, name, bytes); }

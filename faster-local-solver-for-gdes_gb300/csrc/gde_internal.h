@@ -6,6 +6,8 @@
 
 #include <cmath>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -19,6 +21,8 @@ struct DevBuf {
 
 constexpr int kDefaultMaxRounds = 100000;
 
+struct gde_graph;
+
 struct gde_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -31,6 +35,8 @@ struct gde_ctx {
     gde::TileState* hts = nullptr;       // pinned scratch
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     std::map<std::string, DevBuf> ws;
+    std::mutex spare_mu;
+    std::vector<gde_graph*> spare;  // graphs of this context that hold a merged copy (gde_internal_malloc)
     std::vector<int> stamp;         // per-tile stamp bases (valid while "mark" is allocated)
     gde::PlainWork plain{};
     int64_t plain_n = -1;
@@ -84,8 +90,14 @@ struct gde_graph {
     gde::NodeRec* rec = nullptr;
     // the same graph with the leaves of each node merged into one (static graphs
     // where that drops a fifth of the nodes or more; nullptr: none).  Its h_perm /
-    // perm_d take caller ids to merged ids, many to one.
-    gde_graph* merged = nullptr;
+    // perm_d take caller ids to merged ids, many to one.  It is given back when
+    // device memory runs out (gde_internal_malloc): a solve holds a reference.
+    std::shared_ptr<gde_graph> merged;
+    std::mutex mu;                      // guards `merged`
+    std::shared_ptr<gde_graph> merged_copy() {
+        std::lock_guard<std::mutex> lock(mu);
+        return merged;
+    }
     // pull plan of the row capacities (DevGraph::pord, pchunk), built on first
     // use, and whether the live rows are symmetric (-1: not checked since the last edit)
     int32_t* pord = nullptr;
@@ -101,3 +113,7 @@ struct gde_graph {
     std::vector<int32_t> h_twins;  // merged graphs: twins of each node
     int32_t node_in(int64_t u) const { return relabeled ? h_perm[u] : (int32_t)u; }
 };
+
+// cudaMalloc that, before it fails, gives back the merged copies of the
+// context's graphs: they only make solves faster.  (gde_capi.cu)
+cudaError_t gde_internal_malloc(gde_ctx* ctx, void** p, size_t bytes);

@@ -1025,8 +1025,8 @@ extern "C" int gde_graph_repad(gde_ctx* ctx, gde_graph* G, int64_t min_slack, in
     cudaStream_t st = gde_internal_stream(ctx);
     int64_t* d_ptr = nullptr;
     int32_t* d_col = nullptr;
-    if (cudaMalloc(&d_ptr, (size_t)(n + 3) * sizeof(int64_t)) != cudaSuccess ||
-        cudaMalloc(&d_col, (size_t)std::max<int64_t>(cap, 1) * sizeof(int32_t)) != cudaSuccess) {
+    if (gde_internal_malloc(ctx, (void**)&d_ptr, (size_t)(n + 3) * sizeof(int64_t)) != cudaSuccess ||
+        gde_internal_malloc(ctx, (void**)&d_col, (size_t)std::max<int64_t>(cap, 1) * sizeof(int32_t)) != cudaSuccess) {
         cudaFree(d_ptr);
         cudaFree(d_col);
         cudaGetLastError();

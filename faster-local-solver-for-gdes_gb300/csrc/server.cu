@@ -129,7 +129,7 @@ struct gde_server {
     }
     void* dalloc(size_t bytes) {
         void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
+        if (gde_internal_malloc(ctx, &p, std::max<size_t>(bytes, 256)) != cudaSuccess) {
             cudaGetLastError();
             return nullptr;
         }

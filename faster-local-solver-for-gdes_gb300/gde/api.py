@@ -76,7 +76,8 @@ class Graph:
         vol = ctypes.c_double()
         lib.gde_graph_info(self.ptr, None, None, ctypes.byref(vol))
         self.vol = float(vol.value)
-        self._fin = weakref.finalize(self, lib.gde_graph_free, h.value)
+        # (the finalizer holds the context, which has to outlive its graphs)
+        self._fin = weakref.finalize(self, lambda free, ptr, ctx: free(ptr), lib.gde_graph_free, h.value, self.ctx)
 
     def free(self) -> None:
         self._fin()
