@@ -269,16 +269,14 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
         if (c <= kPullLong) break;
         for (int64_t b = 0; b < c; b += kPullChunk) chunks.push_back(make_int2(u, (int)b));
     }
-    G->g.pull_long = (int)i;
+    G->pull_long = (int)i;
     while (i < n && capacity(sorted ? i : ord[i]) > kPullMid) i++;
-    G->g.pull_mid = (int)i;
-    G->g.npchunk = (int)chunks.size();
+    G->pull_mid = (int)i;
+    G->npchunk = (int)chunks.size();
     cudaFree(G->pord);
     cudaFree(G->pchunk);
     G->pord = nullptr;
     G->pchunk = nullptr;
-    G->g.pord = nullptr;
-    G->g.pchunk = nullptr;
     if (cudaMalloc(&G->pchunk, std::max<size_t>(chunks.size(), 1) * sizeof(int2)) != cudaSuccess ||
         (!sorted && cudaMalloc(&G->pord, n * sizeof(int32_t)) != cudaSuccess)) {
         cudaGetLastError();
@@ -287,8 +285,6 @@ int build_pull_plan(gde_ctx* ctx, gde_graph* G) {
     CK(cudaMemcpyAsync(G->pchunk, chunks.data(), chunks.size() * sizeof(int2), cudaMemcpyHostToDevice, ctx->stream));
     if (G->pord) CK(cudaMemcpyAsync(G->pord, ord.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
-    G->g.pord = G->pord;
-    G->g.pchunk = G->pchunk;
     G->pull_plan = true;
     return GDE_OK;
 }
@@ -302,6 +298,7 @@ int enable_pull(gde_ctx* ctx, gde_graph* G, PushArgs& a, int W, int div) {
     a.pull_div = 0;
     const double row_cost = W == 1 ? kPullRowW1 * (double)G->g.n : 0.0;
     if (2.0 * (G->g.vol + row_cost) > div * G->g.vol) return GDE_OK;  // not even half the volume would pull
+    std::lock_guard<std::mutex> lock(G->tables_mu);
     if (!G->pull_plan) {
         const int rc = build_pull_plan(ctx, G);
         if (rc == GDE_ENOMEM) { ctx->err.clear(); return GDE_OK; }
@@ -314,20 +311,22 @@ int enable_pull(gde_ctx* ctx, gde_graph* G, PushArgs& a, int W, int div) {
     a.bits = (uint32_t*)wsget(ctx, "bits", (size_t)a.ntiles * 2 * words * 4);
     if (!a.bits) return GDE_OK;
     a.bit_words = words;
-    a.g.pord = G->g.pord;
-    a.g.pchunk = G->g.pchunk;
-    a.g.npchunk = G->g.npchunk;
-    a.g.pull_long = G->g.pull_long;
-    a.g.pull_mid = G->g.pull_mid;
+    a.g.pord = G->pord;
+    a.g.pchunk = G->pchunk;
+    a.g.npchunk = G->npchunk;
+    a.g.pull_long = G->pull_long;
+    a.g.pull_mid = G->pull_mid;
     a.pull_div = div;
     a.pull_vol = G->g.vol + row_cost;
     return GDE_OK;
 }
 
 // Reciprocal tables of an FP64 launch of `kind`, filled on the device when
-// they are stale; without memory for them the kernel divides.
+// they are stale; without memory for them the kernel divides.  They are marked
+// good only when they are filled: the next launch may be on another stream.
 int enable_reciprocals(gde_ctx* ctx, gde_graph* G, PushArgs& a, int kind) {
     const int64_t n = G->g.n;
+    std::lock_guard<std::mutex> lock(G->tables_mu);
     auto table = [&](double*& t) {
         if (!t && cudaMalloc(&t, n * 8) != cudaSuccess) {
             cudaGetLastError();
@@ -340,6 +339,7 @@ int enable_reciprocals(gde_ctx* ctx, gde_graph* G, PushArgs& a, int kind) {
         if (!G->rign_ok) {
             CK(reciprocals(G->nfac, G->rnf, n, ctx->stream));
             CK(reciprocals(G->tfac, G->rtf, n, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
             G->rign_ok = true;
         }
         a.g.rnf = G->rnf;
@@ -348,6 +348,7 @@ int enable_reciprocals(gde_ctx* ctx, gde_graph* G, PushArgs& a, int kind) {
         if (!table(G->rdeg)) return GDE_OK;
         if (!G->rdeg_ok) {
             CK(reciprocals(G->degd, G->rdeg, n, ctx->stream));
+            CK(cudaStreamSynchronize(ctx->stream));
             G->rdeg_ok = true;
         }
         a.g.rdeg = G->rdeg;

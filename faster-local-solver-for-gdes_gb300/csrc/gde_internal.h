@@ -94,6 +94,9 @@ struct gde_graph {
     // device memory runs out (gde_internal_malloc): a solve holds a reference.
     std::shared_ptr<gde_graph> merged;
     std::mutex mu;                      // guards `merged`
+    // guards what solves make on first use (pull plan, symmetry, reciprocals):
+    // contexts of other threads may solve on the graph meanwhile
+    std::mutex tables_mu;
     std::shared_ptr<gde_graph> merged_copy() {
         std::lock_guard<std::mutex> lock(mu);
         return merged;
@@ -102,6 +105,7 @@ struct gde_graph {
     // use, and whether the live rows are symmetric (-1: not checked since the last edit)
     int32_t* pord = nullptr;
     int2* pchunk = nullptr;
+    int npchunk = 0, pull_long = 0, pull_mid = 0;
     bool pull_plan = false;
     int symmetric = -1;
     // reciprocals of degd (rdeg) and of nfac, tfac (rnf, rtf); rebuilt on use after an edit
