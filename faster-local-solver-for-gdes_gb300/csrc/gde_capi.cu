@@ -382,6 +382,8 @@ int run_engine(gde_ctx* ctx, PushArgs& a, int prec64, int W, gde_stats* st, doub
     CK(cudaMemcpyAsync(&herr, ctx->derr, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(ctx->hstats, ctx->dstats, sizeof(LaunchStats), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    ctx->last_pull_rounds = (int64_t)ctx->hstats->pull_rounds;
+    ctx->last_nodes = a.g.n;
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     *kernel_ms += ms;
@@ -1211,6 +1213,13 @@ int gde_ctx_trace(gde_ctx* ctx, int iters) {
 int gde_ctx_set_wait_limit(gde_ctx* ctx, int64_t polls) {
     if (!ctx || polls < 0) return fail(ctx, GDE_EINVAL, "bad wait limit");
     ctx->wait_limit = polls;
+    return GDE_OK;
+}
+
+int gde_ctx_last_push(gde_ctx* ctx, int64_t* pull_rounds, int64_t* nodes) {
+    if (!ctx) return GDE_EINVAL;
+    if (pull_rounds) *pull_rounds = ctx->last_pull_rounds;
+    if (nodes) *nodes = ctx->last_nodes;
     return GDE_OK;
 }
 

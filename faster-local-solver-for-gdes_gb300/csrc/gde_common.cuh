@@ -302,6 +302,7 @@ struct LaunchStats {          // roofline counters summed over a launch
     unsigned long long iters;          // launch iterations run
     unsigned long long sp_done;        // served small queries finished in hash tables
     unsigned long long sp_ovf;         // ... handed to the dense slots
+    unsigned long long pull_rounds;    // rounds (of tiles) that pulled
 };
 
 // Arrivals so far, on a 128-byte line of its own.

@@ -47,6 +47,8 @@ struct gde_ctx {
     // bounded device waits: polls before a wait gives up (0: the defaults);
     // set by gde_ctx_set_wait_limit to exercise the GDE_EHANG paths
     int64_t wait_limit = 0;
+    // the last push launch (gde_ctx_last_push)
+    int64_t last_pull_rounds = 0, last_nodes = 0;
 };
 
 struct gde_graph {

@@ -2584,6 +2584,7 @@ __device__ void finish_round(const PushArgs& a, int t, int level, bool dense_nex
         }
         atomicAdd(&a.stats->rounds, 1ull);
         if (dense_next) atomicAdd(&a.stats->dense_rounds, 1ull);
+        if (ts.pull[par] && ts.front_cnt[par] > 0) atomicAdd(&a.stats->pull_rounds, 1ull);
     }
 }
 

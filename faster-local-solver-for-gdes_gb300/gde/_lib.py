@@ -79,6 +79,7 @@ SIGNATURES = {
     "gde_ctx_trace": (_int, [_p, _int]),
     "gde_ctx_trace_read": (_int, [_p, _p, _i64, _p, _p, _p]),
     "gde_ctx_set_wait_limit": (_int, [_p, _i64]),
+    "gde_ctx_last_push": (_int, [_p, ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "gde_server_start": (_int, [_p, _p, ctypes.POINTER(Params), _i64, _dbl, _dbl, ctypes.POINTER(_p)]),
     "gde_server_submit": (_int, [_p, _int, _i32, _dbl, _dbl, _p, _int, ctypes.POINTER(_i64)]),
     "gde_server_poll": (_int, [_p, _i64, ctypes.POINTER(_int), ctypes.POINTER(_dbl), ctypes.POINTER(_i32),

@@ -46,6 +46,12 @@ class Context:
             c = cls._by_device[device] = Context(device)
         return c
 
+    def last_push(self) -> dict:
+        """Rounds of the last push launch that pulled, and the nodes of the graph it ran on (fewer: merged leaves)."""
+        pulls, nodes = ctypes.c_int64(), ctypes.c_int64()
+        L.load().gde_ctx_last_push(self.ptr, ctypes.byref(pulls), ctypes.byref(nodes))
+        return {"pull_rounds": pulls.value, "nodes": nodes.value}
+
     def close(self) -> None:
         self._fin()
 

@@ -135,6 +135,13 @@ int gde_ctx_sync(gde_ctx *ctx);
 int gde_ctx_trace(gde_ctx *ctx, int iters);
 int gde_ctx_trace_read(gde_ctx *ctx, uint64_t *out, int64_t cap, int *iters, int *grid, int *points);
 
+/* ---- which way the last push launch of this context took (diagnostics) ----
+ * *pull_rounds: rounds, summed over tiles, in which rows gathered their
+ * neighbours' push values instead of pushing them; *nodes: nodes of the graph
+ * it ran on (fewer than uploaded: leaves were merged).  Both chosen by the
+ * library; either pointer may be NULL. */
+int gde_ctx_last_push(gde_ctx *ctx, int64_t *pull_rounds, int64_t *nodes);
+
 /* ---- bounded device waits (failure detection; no counterpart in the reference) ----
  * Every device-side wait of the library is bounded: the push kernel's grid
  * barrier and the edit dataflow's predecessor waits give up after a number of
