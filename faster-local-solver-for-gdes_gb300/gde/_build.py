@@ -45,6 +45,18 @@ def _digest(extra_flags: list[str]) -> str:
     return h.hexdigest()
 
 
+def identity() -> str:
+    """What the built library was made from (sources and flags); of a library without a stamp, its own bytes."""
+    stamp = os.path.join(BUILD, "libgde.stamp")
+    if os.path.exists(stamp):
+        with open(stamp) as fh:
+            return fh.read()
+    if os.path.exists(LIB):
+        with open(LIB, "rb") as fh:
+            return hashlib.sha256(fh.read()).hexdigest()
+    return ""
+
+
 def build(force: bool = False, verbose: bool = False, extra_flags: list[str] | None = None) -> str:
     # GDE_NVCC_EXTRA: extra nvcc flags (e.g. tuning macros) for experiments
     extra_flags = list(extra_flags or []) + os.environ.get("GDE_NVCC_EXTRA", "").split()

@@ -8,9 +8,9 @@ bound.  The search is staged: first the execution shape (served slots
 for single-column tiles, or node x column tiles of width 4..32), then the
 degree-bucket thresholds (rows per lane / per warp, long-row chunk) for the
 winning shape, and for served shapes the number of block groups the slots
-share.  Results are cached per graph, kind, precision, sample size
-and latency bound in a JSON file next to the graph cache, so a workload is
-tuned once.
+share.  Results are cached per graph, kind, precision, sample size, latency
+bound and build of the library in a JSON file next to the graph cache, so a
+workload is tuned once, and again after the kernels changed.
 """
 from __future__ import annotations
 
@@ -20,6 +20,7 @@ import os
 
 import numpy as np
 
+from gde import _build
 from gde import _lib as L
 from gde import api
 
@@ -53,7 +54,7 @@ def _cache_path(graph: api.Graph, key: str) -> str:
 
 
 def _graph_key(graph: api.Graph, kind: int, prec: str, n_sample: int, max_p99_ms) -> str:
-    h = hashlib.sha1(f"{graph.n}:{graph.cap}:{graph.vol}:{kind}:{prec}:{n_sample}:{max_p99_ms}".encode())
+    h = hashlib.sha1(f"{_build.identity()}:{graph.n}:{graph.cap}:{graph.vol}:{kind}:{prec}:{n_sample}:{max_p99_ms}".encode())
     return f"g{graph.n}_{h.hexdigest()[:16]}"
 
 
