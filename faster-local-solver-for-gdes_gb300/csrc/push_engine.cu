@@ -1758,41 +1758,7 @@ __device__ __forceinline__ void edge_step(const PushArgs& a, const ScatterCtx<T,
                                           int lane_g, int grp_w, const Vec<T, VEC>& p, const double (&theta)[VEC],
                                           const float (&theta_f)[VEC]) {
     bool cr = false;
-    bool combined = false;
-    if constexpr (VEC == 1 && L == 1) {
-        // Hubs (degree-sorted prefix) receive pushes from many frontier leaves
-        // in the same round; lanes of a warp that target the same hub add in
-        // shared memory first and one lane issues the global atomic.  The
-        // crossing test on the combined add is the same test on the stored
-        // value (all additions are non-negative).
-        if (!c.tgt_scale) {
-            const bool hub = ok && v < a.g.hub_cut;
-            if (__any_sync(kFull, hub)) {
-                const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-                const unsigned peers = __match_any_sync(kFull, hub ? v : -1 - lane);
-                const int leader = __ffs(peers) - 1;
-                __shared__ T agg[kWarps][32];
-                if (hub && lane == leader) agg[warp][lane] = T(0);
-                __syncwarp();
-                if (hub) atomicAdd(&agg[warp][leader], p.v[0]);
-                __syncwarp();
-                if (hub && lane == leader) {
-                    const T tot = agg[warp][lane];
-                    T* addr = c.tgt + (int64_t)v * c.tld;
-                    if (c.cross) {
-                        const T old = atomicAdd(addr, tot);
-                        const T s = old + tot;
-                        cr = crossed<T>(a.g, v, old, s, theta[0], theta_f[0]);
-                    } else {
-                        atomicAdd(addr, tot);
-                    }
-                }
-                __syncwarp();
-                combined = hub;
-            }
-        }
-    }
-    if (ok && !combined) {
+    if (ok) {
         if (c.cross) {
             Vec<T, VEC> old;
             vatomic_ret<T, VEC>(c.tgt + (int64_t)v * c.tld + c0, p, old);
