@@ -168,7 +168,9 @@ def committed_traffic():
 
 def algorithmic_bytes(stats: dict) -> float:
     """FP32: 4 B col_idx per union-frontier edge, 8 B residual RMW per (edge, column),
-    32 B per active (node, column): row_ptr pair, r read/zero, x RMW, degree, frontier index."""
+    32 B per active (node, column): row_ptr pair, r read/zero, x RMW, degree, frontier index.
+    Counted over the method's operations.  Fewer move where leaves are merged: their push counts for
+    every leaf that it stands for."""
     return 4.0 * stats["union_vol"] + 8.0 * stats["col_vol"] + 32.0 * stats["col_nodes"]
 
 
@@ -393,7 +395,9 @@ def run_ours(args):
             # launch's operations (traffic grows with the pushes)
             "traffic": (traffic["dram_bytes_per_oper"] * float(np.sum(opers)) / launches
                         if traffic and opers else None),
-            "algorithmic_bytes_per_launch": per_launch_bytes, "kernel": "push_kernel<float,%d>" % args.tile_w,
+            "algorithmic_bytes_per_launch": per_launch_bytes,
+            "bytes_of": "the method's operations (a merged leaf's push counts for each leaf it stands for)",
+            "kernel": "push_kernel<float,%d>" % args.tile_w,
             "kernel_ms_per_launch": kernel_ms_total / launches}
     lat_sorted = np.sort(np.asarray(lat))
     out = {
@@ -416,7 +420,7 @@ def run_ours(args):
     # the push's own ceiling: uniformly random FP32 atomics (with return) over
     # an array the size of the slots' residual slabs, against the SCATTER
     # phase's edge-push rate (its time includes the phase's barrier wait)
-    foot = int(res["stats"]["tiles"]) * args.tile_w * g.n
+    foot = int(res["stats"]["tiles"]) * args.tile_w * ctx.last_push()["nodes"]
     probe = api.probe_random_atomics(foot, True, ctx)
     scat_rate = agg["col_vol"] / (sum(ph["scatter"]) / 1e3) / 1e9
     out["random_access"] = {"scatter_atomics_gps": scat_rate, "probe_atomics_gps": probe,

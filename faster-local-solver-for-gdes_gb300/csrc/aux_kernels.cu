@@ -211,8 +211,10 @@ __global__ void node_tables_kernel(int64_t nn, const NodeTables* rec, int32_t* r
 }
 
 // A warp per row: sums over the row's live entries of h(u, v) - h(v, u) for
-// two mixing functions h.  Over a symmetric adjacency the terms cancel; over
-// another one both sums vanish with probability 2^-128.
+// two mixing functions h.  Over a symmetric adjacency the terms cancel.  The
+// check is a heuristic: another adjacency passes only if both 64-bit sums
+// vanish by chance (the mixers are fixed, so no bound holds against a graph
+// made to pass).
 __device__ __forceinline__ unsigned long long mix64(unsigned long long x, unsigned long long m) {
     x ^= x >> 31;
     x *= m;

@@ -143,7 +143,9 @@ int katz_compute_prec(gde_ctx* ctx, gde_graph* G, const gde_params* p) {
 // price of pushing along it in a W > 1 tile (1/2 to 1/32 measured: InstantGNN
 // push and update 272 / 85 ms at 1/2, 245 / 70 at 1/8, 245 / 70 at 1/32;
 // global GD and Chebyshev flat).  In a one-column tile each row costs about
-// as much as 16 entries, and 1/6 of that total measured best.
+// as much as 16 entries; served slots pull above 1/6 of that total, which
+// measured best for them.  Other one-column launches use 1/8 of it, which was
+// not measured apart.
 constexpr int kPullDiv = 8, kPullDivServed = 6;
 constexpr double kPullRowW1 = 16.0;
 
@@ -562,7 +564,9 @@ int check_symmetric(gde_ctx* ctx, gde_graph* G, int* yes) {
 // residual away) they hold equal residuals and push together.  On the
 // wiki-talk shape 2.36M nodes and 9.4M entries become 1.53M and 7.7M, a query's
 // frontier nodes 58% and its pushes 82%.  Symmetric graphs only (an equal row
-// then means equal senders), and only where it drops a fifth of the nodes.
+// then means equal senders), and only where it drops a fifth of the nodes: the
+// copy costs its upload and memory.  (Measured at 35% dropped; graphs near the
+// limit were not.)
 int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     const int64_t n = G->g.n;
     std::vector<int32_t> id(n, -1), rep, twins;  // internal id -> merged id; merged id -> its first node, its twins

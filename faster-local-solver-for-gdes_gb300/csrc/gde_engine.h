@@ -90,7 +90,8 @@ cudaError_t node_tables(int64_t nn, const NodeTables* rec, int32_t* row_len, dou
                         double* tfac, float* tfac_f, cudaStream_t st);
 
 // Is every live entry v of a row u matched by an entry u of row v (aux_kernels.cu)?  Adds two
-// hashes of every (u, v) minus those of (v, u) into out[0], out[1] (zeroed here): both end at zero.
+// hashes of every (u, v) minus those of (v, u) into out[0], out[1] (zeroed here): both end at zero
+// if so, and otherwise hardly ever.
 cudaError_t symmetry_sums(const DevGraph& g, unsigned long long* out, cudaStream_t st);
 
 // out[i] = 1 / in[i] (aux_kernels.cu).

@@ -70,9 +70,9 @@ typedef struct {
     double beta;       /* InstantGNN exponent */
     double omega;      /* relaxation of gde_sor and of the feature push / update (0 or 1 = synchronous push) */
     int max_rounds;    /* 0 = default (100000) */
-    int small_max;     /* degree buckets: <= small_max lane group per row, 0 = default */
-    int med_max;       /* <= med_max warp per row, else CTA chunks; 0 = default */
-    int chunk;         /* edges per CTA chunk; 0 = default */
+    int small_max;     /* degree buckets: rows of <= small_max entries share a warp, 0 = default */
+    int med_max;       /* <= med_max entries: a warp per row, else a warp per chunk; 0 = default */
+    int chunk;         /* entries per chunk of a long row; 0 = default */
     int dense_div;     /* next round scans all nodes when vol(frontier) > n/dense_div; 0 = default */
     int slots;         /* served PPR/Katz local GD: concurrent queries (one residual vector each); 0 = default */
     int groups;        /* served: the grid splits into this many block groups, each advancing its own slots
@@ -90,8 +90,10 @@ typedef struct {
     double total_ms;            /* device time of the whole call */
     int64_t rounds;             /* sum over tiles of rounds run */
     int64_t dense_rounds;
-    double union_vol;           /* sum_t vol(union frontier)   -> col_idx bytes */
-    double col_vol;             /* sum_t sum_c vol(S_t^c)      -> residual update bytes */
+    double union_vol;           /* sum_t vol(union frontier): the method's column reads */
+    double col_vol;             /* sum_t sum_c vol(S_t^c): its residual updates.  Operations of the method, not
+                                   bytes moved: a merged leaf's push counts for each leaf it stands for, and a
+                                   round that pulls reads every row */
     uint64_t union_nodes;       /* sum_t |union frontier| */
     uint64_t col_nodes;         /* sum_t sum_c |S_t^c| */
     int tiles;
