@@ -457,9 +457,9 @@ int upload_ign_tables(gde_ctx* ctx, gde_graph* G, double beta) {
         tff[u] = (float)tf[u];
     }
     if (!G->nfac) {
-        CK(cudaMalloc(&G->nfac, n * 8));
-        CK(cudaMalloc(&G->tfac, n * 8));
-        CK(cudaMalloc(&G->tfac_f, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&G->nfac, n * 8));
+        CK(gde_internal_malloc(ctx, (void**)&G->tfac, n * 8));
+        CK(gde_internal_malloc(ctx, (void**)&G->tfac_f, n * 4));
     }
     CK(cudaMemcpyAsync(G->nfac, nf.data(), n * 8, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(G->tfac, tf.data(), n * 8, cudaMemcpyHostToDevice, ctx->stream));
@@ -558,6 +558,17 @@ int check_symmetric(gde_ctx* ctx, gde_graph* G, int* yes) {
     return GDE_OK;
 }
 
+// Frees a graph that no launch uses any more.
+void release(gde_graph* G) {
+    cudaFree(G->row_ptr); cudaFree(G->col); cudaFree(G->row_len); cudaFree(G->degf); cudaFree(G->degd);
+    cudaFree(G->nfac); cudaFree(G->tfac); cudaFree(G->tfac_f); cudaFree(G->perm_d); cudaFree(G->iperm_d);
+    cudaFree(G->col_deg); cudaFree(G->rec);
+    cudaFree(G->pord); cudaFree(G->pchunk);
+    cudaFree(G->rdeg); cudaFree(G->rnf); cudaFree(G->rtf);
+    cudaFree(G->pw1); cudaFree(G->pwb);
+    delete G;
+}
+
 // The graph with the leaves of each node merged into one: nodes whose row is
 // the same single neighbour, with the same degree, receive the same additions
 // in every round, so from round 1 on (when a seed among them has pushed its own
@@ -629,10 +640,10 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
         cudaMalloc(&M->degd, m * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&M->perm_d, n * sizeof(int32_t)) != cudaSuccess) {
         cudaGetLastError();
-        gde_graph_free(M);
+        release(M);
         return GDE_OK;
     }
-    std::shared_ptr<gde_graph> held(M, [](gde_graph* g) { gde_graph_free(g); });
+    std::shared_ptr<gde_graph> held(M, release);  // (its context may be gone when another one's solve drops it)
     CK(cudaMemsetAsync(M->row_ptr, 0, (m + 3) * sizeof(int64_t), ctx->stream));
     CK(cudaMemcpyAsync(M->row_ptr, M->h_indptr.data(), (m + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
     if (cap > 0) CK(cudaMemcpyAsync(M->col, mcol.data(), cap * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream));
@@ -657,19 +668,6 @@ int build_merged(gde_ctx* ctx, gde_graph* G, const int32_t* col) {
     std::lock_guard<std::mutex> lock(ctx->spare_mu);
     ctx->spare.push_back(G);
     return GDE_OK;
-}
-
-// Runs a solve of G, and once more if it ran out of memory with the merged
-// copy that it ran on given back meanwhile.
-template <typename F>
-int with_room(gde_ctx* ctx, gde_graph* G, F solve) {
-    const bool had = G && G->merged_copy();
-    int rc = solve();
-    if (rc == GDE_ENOMEM && had && !G->merged_copy()) {
-        ctx->err.clear();
-        rc = solve();
-    }
-    return rc;
 }
 
 // Served solve of PPR / Katz local GD: `slots` single-column tiles cycle
@@ -1452,18 +1450,12 @@ int gde_graph_free(gde_graph* G) {
     if (!G) return GDE_EINVAL;
     cudaSetDevice(G->ctx->device);
     cudaStreamSynchronize(G->ctx->stream);
-    cudaFree(G->row_ptr); cudaFree(G->col); cudaFree(G->row_len); cudaFree(G->degf); cudaFree(G->degd);
-    cudaFree(G->nfac); cudaFree(G->tfac); cudaFree(G->tfac_f); cudaFree(G->perm_d); cudaFree(G->iperm_d);
-    cudaFree(G->col_deg); cudaFree(G->rec);
-    cudaFree(G->pord); cudaFree(G->pchunk);
-    cudaFree(G->rdeg); cudaFree(G->rnf); cudaFree(G->rtf);
-    cudaFree(G->pw1); cudaFree(G->pwb);
     {
         std::lock_guard<std::mutex> lock(G->ctx->spare_mu);
         std::vector<gde_graph*>& v = G->ctx->spare;
         v.erase(std::remove(v.begin(), v.end(), G), v.end());
     }
-    delete G;  // (and its merged copy, once no solve holds it)
+    release(G);  // (and its merged copy, once no solve holds it)
     return GDE_OK;
 }
 
@@ -2004,15 +1996,15 @@ int gde_plain_ppr_local(gde_ctx* ctx, gde_graph* G, int32_t seed, double alpha, 
         }
         PlainWork& w = ctx->plain;
         int64_t nb = (n + 255) / 256 + 1;
-        CK(cudaMalloc(&w.xt, n * 4));
-        CK(cudaMalloc(&w.rt, n * 4));
-        CK(cudaMalloc(&w.tmp, n * 4));
-        CK(cudaMalloc(&w.sp, n * 4));
-        CK(cudaMalloc(&w.eps_vec, n * 4));
-        CK(cudaMalloc(&w.queue, n * 4));
-        CK(cudaMalloc(&w.nz, nb * 4));
-        CK(cudaMalloc(&w.d_count, 4));
-        CK(cudaMalloc(&w.d_oper, 8));
+        CK(gde_internal_malloc(ctx, (void**)&w.xt, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.rt, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.tmp, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.sp, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.eps_vec, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.queue, n * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.nz, nb * 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.d_count, 4));
+        CK(gde_internal_malloc(ctx, (void**)&w.d_oper, 8));
         CK(cudaMallocHost(&w.h_count, 4));
         ctx->plain_n = n;
     }
@@ -2133,24 +2125,27 @@ int gde_internal_graph_host(gde_graph* G, const int64_t** indptr, const int64_t*
 
 cudaError_t gde_internal_malloc(gde_ctx* ctx, void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        std::vector<std::shared_ptr<gde_graph>> copies;  // freed here, or when the solve that runs on one returns
+        {
+            std::lock_guard<std::mutex> lock(ctx->spare_mu);
+            for (gde_graph* G : ctx->spare) {
+                std::lock_guard<std::mutex> own(G->mu);
+                copies.push_back(std::move(G->merged));
+                G->merged.reset();
+            }
+            ctx->spare.clear();
+        }
+        if (!copies.empty()) {
+            copies.clear();
+            e = cudaMalloc(p, bytes);
+        }
+    }
     if (e == cudaSuccess) return e;
     cudaGetLastError();
     *p = nullptr;
-    if (e != cudaErrorMemoryAllocation) return e;
-    std::vector<std::shared_ptr<gde_graph>> copies;  // freed here, or when the solve that runs on one returns
-    {
-        std::lock_guard<std::mutex> lock(ctx->spare_mu);
-        for (gde_graph* G : ctx->spare) {
-            std::lock_guard<std::mutex> own(G->mu);
-            copies.push_back(std::move(G->merged));
-            G->merged.reset();
-        }
-        ctx->spare.clear();
-    }
-    if (copies.empty()) return e;
-    copies.clear();
-    e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) cudaGetLastError();
+    ctx->malloc_failed |= e == cudaErrorMemoryAllocation;
     return e;
 }
 

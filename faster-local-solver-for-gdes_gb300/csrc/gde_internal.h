@@ -37,6 +37,7 @@ struct gde_ctx {
     std::map<std::string, DevBuf> ws;
     std::mutex spare_mu;
     std::vector<gde_graph*> spare;  // graphs of this context that hold a merged copy (gde_internal_malloc)
+    bool malloc_failed = false;     // ... has failed since with_room cleared this
     std::vector<int> stamp;         // per-tile stamp bases (valid while "mark" is allocated)
     gde::PlainWork plain{};
     int64_t plain_n = -1;
@@ -123,3 +124,22 @@ struct gde_graph {
 // cudaMalloc that, before it fails, gives back the merged copies of the
 // context's graphs: they only make solves faster.  (gde_capi.cu)
 cudaError_t gde_internal_malloc(gde_ctx* ctx, void** p, size_t bytes);
+
+// Runs a solve of G.  One for which device memory ran out (not a caller's
+// budget) runs once more without G's merged copy: allocations give back the
+// copies of their own context's graphs only, and G may be another's.
+template <typename F>
+int with_room(gde_ctx* ctx, gde_graph* G, F solve) {
+    const bool had = ctx && G && G->merged_copy();
+    if (ctx) ctx->malloc_failed = false;
+    const int rc = solve();
+    if (rc != GDE_ENOMEM || !had || !ctx->malloc_failed) return rc;
+    std::shared_ptr<gde_graph> copy;
+    {
+        std::lock_guard<std::mutex> lock(G->mu);
+        copy.swap(G->merged);
+    }
+    copy.reset();
+    ctx->err.clear();
+    return solve();
+}

@@ -239,8 +239,8 @@ struct gde_server {
 
 extern "C" {
 
-int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ring_capacity, double hbm_budget_bytes,
-                     double idle_ms, gde_server** out) {
+static int start_call(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ring_capacity, double hbm_budget_bytes,
+                      double idle_ms, gde_server** out) {
     if (!ctx || !G || !p || !out) return gde_internal_fail(ctx, GDE_EINVAL, "bad server arguments");
     if (p->prec != GDE_FP32 && p->prec != GDE_FP64) return gde_internal_fail(ctx, GDE_EINVAL, "bad precision");
     if (ring_capacity < 1 || ring_capacity > (1 << 24)) return gde_internal_fail(ctx, GDE_EINVAL, "ring capacity");
@@ -456,6 +456,11 @@ int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ri
     s->th = std::thread([s] { s->run(); });
     *out = s;
     return GDE_OK;
+}
+
+int gde_server_start(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t ring_capacity, double hbm_budget_bytes,
+                     double idle_ms, gde_server** out) {
+    return with_room(ctx, G, [&] { return start_call(ctx, G, p, ring_capacity, hbm_budget_bytes, idle_ms, out); });
 }
 
 int gde_server_submit(gde_server* s, int kind, int32_t seed, double eps, double alpha, void* x_out, int out64,

@@ -529,9 +529,9 @@ int sor_run(gde_ctx* ctx, SorArgs& a, int prec64, std::vector<double>& hop, std:
 
 }  // namespace
 
-extern "C" int gde_sor(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds,
-                       const double* eps, int local, void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out,
-                       double* oper_out, int32_t* sweeps_out, gde_stats* stats) {
+static int sor_call(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds,
+                    const double* eps, int local, void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out,
+                    double* oper_out, int32_t* sweeps_out, gde_stats* stats) {
     if (!ctx || !G || !p || nq < 0 || (nq > 0 && (!seeds || !eps))) return gde_internal_fail(ctx, GDE_EINVAL, "bad SOR arguments");
     if (p->kind != KIND_PPR && p->kind != KIND_KATZ) return gde_internal_fail(ctx, GDE_EINVAL, "SOR kinds are PPR and Katz");
     const int64_t n = G->g.n;
@@ -609,6 +609,15 @@ extern "C" int gde_sor(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t 
     }
     if (capped) return gde_internal_fail(ctx, GDE_EITERCAP, "max sweeps reached before nothing was pending");
     return GDE_OK;
+}
+
+extern "C" int gde_sor(gde_ctx* ctx, gde_graph* G, const gde_params* p, int64_t nq, const int32_t* seeds,
+                       const double* eps, int local, void* x_out, void* r_out, int out64, int out_mem, int64_t ld_out,
+                       double* oper_out, int32_t* sweeps_out, gde_stats* stats) {
+    return with_room(ctx, G, [&] {
+        return sor_call(ctx, G, p, nq, seeds, eps, local, x_out, r_out, out64, out_mem, ld_out, oper_out, sweeps_out,
+                        stats);
+    });
 }
 
 // InstantGNN push with relaxation omega != 1 (instantGNNSorPush,

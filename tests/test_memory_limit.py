@@ -50,3 +50,21 @@ def test_a_solve_that_would_fit_without_the_copy(arrays, solve, left):
         torch.cuda.empty_cache()
     assert np.array_equal(got["oper"], want["oper"])
     assert np.abs(got["x"] - want["x"]).sum() < 1e-12
+
+
+def test_a_solve_through_another_context(arrays):
+    """The graph's copy is not among those of the context that runs out."""
+    import torch
+    own, other = api.Context(0), api.Context(0)
+    G = api.Graph(*arrays, ctx=own)
+    want = np.array(_cheby(G)["x"])
+    view = object.__new__(api.Graph)
+    view.ctx, view.ptr, view.n, view.cap, view.vol = other, G.ptr, G.n, G.cap, G.vol
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (180 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        got = _cheby(view)
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+    assert np.abs(got["x"] - want).sum() < 1e-12
