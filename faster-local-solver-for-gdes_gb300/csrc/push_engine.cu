@@ -1244,19 +1244,22 @@ __device__ __noinline__ void prep_nodes(const PushArgs& a, int t, const TileSh& 
     total = sum;
 }
 
-// PREP of an FP32 tile of several columns whose round pushes, on exact degrees
-// and an unmerged graph, every method but Chebyshev.  Most scanned nodes are
-// below every threshold: only the residual and the degree are loaded before the
-// test.  prep_nodes gives the same results; its call, and the arguments and
-// sums that it reads and spills per node, cost FP32 tiles 8 to 13 us of every
-// round.  PREP of 154 rounds of global GD, 8 columns: 87k nodes 6.6 -> 3.5 ms,
-// 2.36M nodes 25.9 -> 14.2 ms.
-template <int W>
-__device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
-                                            PrepSums<float, W>& total) {
-    constexpr int VEC = PrepSums<float, W>::VEC;
+// PREP of a tile of several columns whose round pushes, on an unmerged graph (in
+// FP32 on exact degrees), every method but Chebyshev and the relaxed heat
+// kernel.  Most scanned nodes are below every threshold: only the residual and
+// the degree are loaded before the test.  prep_nodes gives the same results; its
+// call, and the arguments and sums that it reads and spills per node, cost FP32
+// tiles 8 to 13 us of every round.  PREP of 154 rounds of global GD, FP32, 8
+// columns: 87k nodes 6.6 -> 3.5 ms, 2.36M nodes 25.9 -> 14.2 ms.  FP64 solves of 61
+// columns, 4 a tile: global Katz on 87k nodes 0.79 -> 0.65 ms, local gradient
+// descent on the scale-17 R-MAT graph 2.65 -> 2.44 ms.
+template <typename T, int W>
+__device__ __forceinline__ void prep_push(const PushArgs& a, int t, const TileSh& sh, long long beg, long long end,
+                                          PrepSums<T, W>& total) {
+    constexpr int VEC = PrepSums<T, W>::VEC;
     constexpr int L = W / VEC;
     constexpr int GPW = 32 / L;
+    constexpr bool F64 = sizeof(T) == 8;
     const DevGraph& g = a.g;
     const int64_t n = g.n, ld = a.ld, xld = x_ld(a);
     const int kind = sh.tp.kind;
@@ -1268,27 +1271,29 @@ __device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const Tile
     const int32_t* cand = a.cand + ((int64_t)t * 2 + sh.parity) * n;
     PushItem* bsmall = a.bsmall + (int64_t)t * n;
     PushItem* blarge = a.blarge + (int64_t)t * a.large_cap;
-    float* Pw = reinterpret_cast<float*>(a.P) + (int64_t)t * n * W + c0;
-    float* R = slab_ptr<float>((hk && (sh.level & 1)) ? a.R2 : a.R, a, t) + c0;
-    float* X = xslab_ptr<float>(a.X, a, t) + c0;
-    float* XC = a.kahan ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
+    T* Pw = reinterpret_cast<T*>(a.P) + (int64_t)t * n * W + c0;
+    T* R = slab_ptr<T>((hk && (sh.level & 1)) ? a.R2 : a.R, a, t) + c0;
+    T* X = xslab_ptr<T>(a.X, a, t) + c0;
+    float* XC = (!F64 && a.kahan) ? xslab_ptr<float>(a.XC, a, t) + c0 : nullptr;
+    const double* rdiv = F64 && !katz ? (ign ? g.rnf : g.rdeg) : nullptr;
     const double hk_div = hk ? (double)sh.tp.n_levels * sh.psi : 1.0;
-    const float coef = (float)(hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.))
-                                  : katz ? sh.tp.alpha : 1. - sh.tp.alpha);
-    const float gain = (float)(ign ? sh.tp.x_gain : 1.0);
-    float thr[VEC];
+    const T coef = (T)(hk ? (sh.final_level ? 1.0 : sh.tp.tau / ((double)sh.level + 1.))
+                          : katz ? sh.tp.alpha : 1. - sh.tp.alpha);
+    const T gain = (T)(ign ? sh.tp.x_gain : 1.0);
+    T thr[VEC];
     unsigned live = 0;
 #pragma unroll
     for (int k = 0; k < VEC; ++k) {
         live |= sh.col_live[c0 + k] ? 1u << k : 0u;
-        thr[k] = (float)(hk ? sh.col_theta[c0 + k] / hk_div : sh.col_theta[c0 + k]);
+        thr[k] = (T)(hk ? sh.col_theta[c0 + k] / hk_div : sh.col_theta[c0 + k]);
     }
     int nodes[VEC], cnt = 0;
     long long oper[VEC], vol = 0;  // sums of degrees: integers, or the bits of FP64 sums
 #pragma unroll
     for (int k = 0; k < VEC; ++k) oper[k] = nodes[k] = 0;
-    auto add = [&](long long& sum, float d) {
-        sum = dint ? sum + (int)d : __double_as_longlong(__longlong_as_double(sum) + (double)d);
+    auto degree = [&](int u, float df) { return F64 && !g.degf_exact ? g.degd[u] : (double)df; };
+    auto add = [&](long long& sum, int u, float df) {
+        sum = dint ? sum + (int)df : __double_as_longlong(__longlong_as_double(sum) + degree(u, df));
     };
     for (long long base = beg + (long long)warp * GPW; base < end; base += (long long)kWarps * GPW) {
         const long long i = base + grp_w;
@@ -1296,19 +1301,23 @@ __device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const Tile
         unsigned act = 0;
         bool absorb = false;
         float df = 1.f;
-        Vec<float, VEC> r, push;
+        Vec<T, VEC> r, push;
 #pragma unroll
-        for (int k = 0; k < VEC; ++k) push.v[k] = 0.f;
+        for (int k = 0; k < VEC; ++k) push.v[k] = T(0);
         if (u >= 0) {
-            vload<float, VEC>(R + (int64_t)u * ld, r);
+            vload<T, VEC>(R + (int64_t)u * ld, r);
             df = g.degf[u];
-            const float b = ign ? (float)g.nfac[u] : df;
+            const T b = all ? T(0) : ign ? (T)g.nfac[u] : (T)degree(u, df);
 #pragma unroll
             for (int k = 0; k < VEC; ++k) {
-                const bool on = all ? r.v[k] != 0.f : ge_band(fabsf(r.v[k]), thr[k] * b, [&] {
-                    const double th = sh.col_theta[c0 + k] * (ign ? g.nfac[u] : (double)df);
+                auto exact = [&] {
+                    const double th = sh.col_theta[c0 + k] * (ign ? g.nfac[u] : degree(u, df));
                     return hk ? (th / (double)sh.tp.n_levels) / sh.psi : th;
-                });
+                };
+                bool on;
+                if (all) on = r.v[k] != T(0);
+                else if constexpr (F64) on = hk ? ge_band64(r.v[k], thr[k] * b, exact) : ge_abs64(r.v[k], thr[k] * b);
+                else on = ge_band(fabsf(r.v[k]), thr[k] * b, exact);
                 act |= on ? 1u << k : 0u;
             }
             act &= live;
@@ -1316,18 +1325,22 @@ __device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const Tile
                 absorb = true;  // (a zero residual has nothing to absorb)
 #pragma unroll
                 for (int k = 0; k < VEC; ++k)
-                    if (r.v[k] == 0.f) act &= ~(1u << k);
+                    if (r.v[k] == T(0)) act &= ~(1u << k);
             }
             if (act) {
-                const float div = katz ? 1.f : ign ? (float)g.npush[u] : df;
-                Vec<float, VEC> x, xc;
-                vload<float, VEC>(X + (int64_t)u * xld, x);
+                // a push is (coef r) / div; in FP64 r times the quotient, from the divisor's reciprocal
+                T div = T(1);
+                if (F64 && rdiv) div = coef * (T)rdiv[u];
+                else if (!katz) div = ign ? (T)g.npush[u] : (T)degree(u, df);
+                Vec<T, VEC> x;
+                Vec<float, VEC> xc;
+                vload<T, VEC>(X + (int64_t)u * xld, x);
                 if (XC) vload<float, VEC>(XC + (int64_t)u * xld, xc);
 #pragma unroll
                 for (int k = 0; k < VEC; ++k) {
                     if (!(act >> k & 1)) continue;
-                    const float rk = r.v[k];
-                    r.v[k] = 0.f;
+                    const T rk = r.v[k];
+                    r.v[k] = T(0);
                     nodes[k] += 1;
                     if (absorb) {
                         // p[u] = r[u]; r[u] = 0 for an absorbing node (InstantGNN.py:22-25)
@@ -1335,21 +1348,21 @@ __device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const Tile
                         if (XC) xc.v[k] = 0.f;
                         continue;
                     }
-                    add(oper[k], df);
-                    push.v[k] = (coef * rk) / div;
-                    const float xadd = gain * rk;
+                    add(oper[k], u, df);
+                    push.v[k] = F64 && rdiv ? div * rk : F64 && katz ? coef * rk : (coef * rk) / div;
+                    const T xadd = gain * rk;
                     if (XC) {
                         // Kahan-compensated FP32 accumulation of the solution
-                        const float y = xadd - xc.v[k];
-                        const float s = x.v[k] + y;
-                        xc.v[k] = (s - x.v[k]) - y;
-                        x.v[k] = s;
+                        const float y = (float)xadd - xc.v[k];
+                        const float s = (float)x.v[k] + y;
+                        xc.v[k] = (s - (float)x.v[k]) - y;
+                        x.v[k] = (T)s;
                     } else {
                         x.v[k] = x.v[k] + xadd;
                     }
                 }
-                vstore<float, VEC>(R + (int64_t)u * ld, r);
-                vstore<float, VEC>(X + (int64_t)u * xld, x);
+                vstore<T, VEC>(R + (int64_t)u * ld, r);
+                vstore<T, VEC>(X + (int64_t)u * xld, x);
                 if (XC) vstore<float, VEC>(XC + (int64_t)u * xld, xc);
             }
         }
@@ -1361,14 +1374,14 @@ __device__ __forceinline__ void prep_push32(const PushArgs& a, int t, const Tile
         const bool lead = in && c0 == 0;
         const unsigned bl = __ballot_sync(kFull, lead), below = (1u << lane) - 1u;
         if (bl == 0) continue;
-        if (in) vstore<float, VEC>(Pw + (int64_t)u * W, push);
+        if (in) vstore<T, VEC>(Pw + (int64_t)u * W, push);
         int len = 0, nch = 0;
         long long rp = 0;
         if (lead) {
             len = g.row_len[u];
             rp = g.row_ptr[u];
             if (len > a.med_max) nch = (len + a.chunk - 1) / a.chunk;
-            add(vol, df);
+            add(vol, u, df);
             cnt += 1;
         }
         const bool small = lead && len <= a.small_max, med = lead && !small && nch == 0;
@@ -1609,9 +1622,10 @@ __device__ void prep_range(const PushArgs& a, int t, const TileSh& sh, PrepSh& p
             a.g.merged ? prep_pull<T, W, true>(a, t, sh, beg, end, sum)
                        : prep_pull<T, W, false>(a, t, sh, beg, end, sum);
         else {
-            if constexpr (sizeof(T) == 4)
-                if (a.g.degf_exact && !a.g.merged) prep_push32<W>(a, t, sh, beg, end, sum);
-            if (sizeof(T) == 8 || !a.g.degf_exact || a.g.merged)
+            const bool relaxed = sizeof(T) == 8 && sh.tp.kind == KIND_HK && hk_relaxed(sh.tp);
+            if (!a.g.merged && !relaxed && (sizeof(T) == 8 || a.g.degf_exact))
+                prep_push<T, W>(a, t, sh, beg, end, sum);
+            else
                 a.g.merged ? prep_nodes<T, W, PULL, true>(a, t, sh, beg, end, sum)
                            : prep_nodes<T, W, PULL, false>(a, t, sh, beg, end, sum);
         }
