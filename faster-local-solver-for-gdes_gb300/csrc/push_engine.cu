@@ -853,7 +853,7 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
         if (u >= 0) {
             const double base64 = ign ? nf : (g.degf_exact ? (double)df : g.degd[u]);
             const float base_f = ign ? (float)base64 : df;
-            const double thr64 = !f32 && !all ? scale0 * base64 : 0.0;
+            const double thr64 = F64 && !all ? scale0 * base64 : 0.0;
 #pragma unroll
             for (int k = 0; k < VEC; ++k) {
                 auto exact = [&] {
@@ -864,8 +864,8 @@ __device__ __noinline__ void prep_pull(const PushArgs& a, int t, const TileSh& s
                 if (all) ge = r.v[k] != T(0);
                 else if (f32) ge = ge_band(fabsf((float)r.v[k]), thr_f[k] * base_f, exact);
                 else if (hk) ge = ge_band64((double)r.v[k],
-                                            same ? thr64 : (sh.col_theta[c0 + k] / hk_div) * base64, exact);
-                else ge = ge_abs64((double)r.v[k], same ? thr64 : sh.col_theta[c0 + k] * base64);
+                                            F64 && same ? thr64 : (sh.col_theta[c0 + k] / hk_div) * base64, exact);
+                else ge = ge_abs64((double)r.v[k], F64 && same ? thr64 : sh.col_theta[c0 + k] * base64);
                 act |= ge ? 1u << k : 0u;
             }
             act &= live;
